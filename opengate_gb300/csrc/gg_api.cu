@@ -123,6 +123,8 @@ struct gg_ctx {
   uint64_t singles_cap = 0;
   void *d_records = nullptr;
   size_t rec_cap = 0;
+  void *d_slot = nullptr;  // per-slot scratch of the pooled transport kernel
+  size_t slot_bytes = 0;
   // SPECT stage queues (head queue, return queue) and their lengths
   void *d_queue[3] = {nullptr, nullptr, nullptr};  // head, return, ARF fallback
   size_t q_cap = 0;
@@ -269,6 +271,8 @@ struct gg_ctx {
     q_cap = 0;
     dfree(d_cdf_z); dfree(d_cdf_y); dfree(d_cdf_x); dfree(d_proj); dfree(d_frames);
     rec_cap = 0;
+    dfree(d_slot);
+    slot_bytes = 0;
     for (auto e : ev) cudaEventDestroy(e);
     ev.clear();
     if (stream) cudaStreamDestroy(stream);
@@ -1260,26 +1264,12 @@ static int spect_stages(gg_ctx *c, gg::KernelArgs a, size_t smem, int minb) {
 static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool capturing = false) {
   size_t smem = c->precision == GG_PREC_F64 ? gg::transport_smem_bytes<double>(c->n_comp, c->n_e, c->n_mat)
                                             : gg::transport_smem_bytes<float>(c->n_comp, c->n_e, c->n_mat);
-  // kernel variant: register budget for `minb` resident 256-thread blocks
-  // batched simulations bind their geometry per history: more live registers, default 2 blocks / SM;
-  // the track-length estimator's voxel walks: 3 (80 registers: 34.3 ms per 1e7 pencil primaries
-  // against 36.5 at 4 blocks / SM)
+  // kernel variant (SPECT stages, track-length estimator): register budget for `minb` resident
+  // 256-thread blocks; the estimator's voxel walks: 3 (80 registers: 34.3 ms per 1e7 pencil
+  // primaries against 36.5 at 4 blocks / SM)
   const bool tle_run = c->tle && !c->have_spect && !c->have_batch;
   int minb = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, 4)
-                                  : ((c->precision == GG_PREC_F64 || c->have_batch) ? 2 : (tle_run ? 3 : 4));
-  int bps = 0;
-  {
-    // (occupancy_blocks counts one voxel list per thread; a dose grid scoring dose keeps two)
-    const bool two_lists = c->dgrid_on && c->ddose && !c->have_spect && !c->have_batch;
-    const size_t smem_occ = smem + (two_lists ? (c->precision == GG_PREC_F64 ? gg::hist_list_bytes<double>(1, c->block)
-                                                                             : gg::hist_list_bytes<float>(1, c->block))
-                                              : 0);
-    cudaError_t e = c->precision == GG_PREC_F64 ? gg::occupancy_blocks<double>(c->block, smem_occ, minb, &bps)
-                                                : gg::occupancy_blocks<float>(c->block, smem_occ, minb, &bps);
-    if (e != cudaSuccess) return c->cuda(e, "occupancy");
-    if (bps < 1) bps = 1;
-  }
-  int grid = c->n_sm * bps;
+                                  : (c->precision == GG_PREC_F64 ? 2 : (tle_run ? 3 : 4));
   // the compacted wavefront kernel: single dose simulations with analog scoring
   if (c->dgrid_on && c->tle && !c->have_spect && !c->have_batch)
     return c->fail(GG_ERR_STATE, "gg_run: the track-length estimator scores on the image grid (no dose grid)");
@@ -1314,6 +1304,7 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     const double lim = std::min(4294967296.0 / (em * em), 4294967296.0 / em);
     if ((double)batch > lim) batch = std::max<uint64_t>(1, (uint64_t)lim);
   }
+  batch = std::min<uint64_t>(batch, 0xffffffffull);  // (a history's record has a 32-bit number)
   c->last_batch = batch;
   uint64_t nb = (n + batch - 1) / batch;
   size_t cap = (size_t)std::min<uint64_t>(n, batch);
@@ -1324,6 +1315,30 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     int st = c->cuda(cudaMalloc(&c->d_records, bytes), "cudaMalloc primary records");
     if (st) return st;
     c->rec_cap = cap;
+  }
+  // launch shape of the dose transport: the pooled kernel, or the estimator's persistent grid
+  gg::PoolPlan plan{};
+  int tle_grid = 0;
+  if (tle_run) {
+    int bps = 0;
+    cudaError_t e = c->precision == GG_PREC_F64 ? gg::tle_occupancy<double>(c->block, smem, minb, &bps)
+                                                : gg::tle_occupancy<float>(c->block, smem, minb, &bps);
+    if (e != cudaSuccess) return c->cuda(e, "occupancy");
+    tle_grid = c->n_sm * std::max(bps, 1);
+  } else if (!c->have_spect && !wave) {
+    const bool two = c->dgrid_on && c->ddose && !c->have_batch;
+    const int pool_threads = c->block == gg::kBlock ? 0 : c->block;  // (the default: the kernel's own block size)
+    cudaError_t e = c->precision == GG_PREC_F64
+                        ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap, two, &plan)
+                        : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap, two, &plan);
+    if (e != cudaSuccess) return c->cuda(e, "transport launch shape");
+    if (plan.scratch > c->slot_bytes) {
+      dfree(c->d_slot);
+      c->slot_bytes = 0;
+      int st = c->cuda(cudaMalloc(&c->d_slot, plan.scratch), "cudaMalloc photon slots");
+      if (st) return st;
+      c->slot_bytes = plan.scratch;
+    }
   }
   // scatter splitting pushes several copies per history: a longer head queue
   // (the phantom passes adapt to it)
@@ -1368,7 +1383,8 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
   a.acc_d2 = dg && c->ddose && c->squared ? c->d_acc_d2 : nullptr;
   a.counters = c->d_counters;
   a.status = c->d_status;
-  a.chunk = c->chunk;
+  a.chunk = plan.grid ? gg::pool_chunk(plan, c->chunk, cap) : c->chunk;
+  a.slot_scratch = c->d_slot;
   a.records = c->d_records;
   a.rec_cap = c->rec_cap;
   a.refill_min = c->refill_min;
@@ -1398,9 +1414,13 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
               : gg::launch_wavefront<float>(c->scene<float>(), a, wgrid, wsmem, wminb, c->stream);
       if ((st = c->cuda(e, "wavefront transport launch"))) return st;
     } else {
-      e = c->precision == GG_PREC_F64
-              ? gg::launch_transport<double>(c->scene<double>(), a, grid, c->block, smem, minb, c->stream)
-              : gg::launch_transport<float>(c->scene<float>(), a, grid, c->block, smem, minb, c->stream);
+      if (tle_run)
+        e = c->precision == GG_PREC_F64
+                ? gg::launch_transport_tle<double>(c->scene<double>(), a, tle_grid, c->block, smem, minb, c->stream)
+                : gg::launch_transport_tle<float>(c->scene<float>(), a, tle_grid, c->block, smem, minb, c->stream);
+      else
+        e = c->precision == GG_PREC_F64 ? gg::launch_transport<double>(c->scene<double>(), a, plan, c->stream)
+                                        : gg::launch_transport<float>(c->scene<float>(), a, plan, c->stream);
       if ((st = c->cuda(e, "transport launch"))) return st;
     }
     if (!capturing && (st = c->cuda(cudaEventRecord(c->ev[3 * b + 2], c->stream), "event"))) return st;

@@ -89,6 +89,7 @@ struct Rng {
     h1 = (uint32_t)(history >> 32);
     idx = 4;
   }
+  __device__ __forceinline__ void reserve(int) {}  // (next() makes blocks on demand)
   __device__ __forceinline__ uint32_t next() {
     if (idx == 4) {
       uint4 b = philox_block(blk, stream, h0, h1, k0, k1);
@@ -690,18 +691,21 @@ __device__ __forceinline__ void set_energy(const Scene<real> &s, Photon<real> &p
   ph.inv_mumax = st.inv_mumax;
 }
 
+// A new photon at its position: in the image (its path there still to be
+// computed) or in the world.
 template <typename real>
-__device__ __forceinline__ void start_photon(const Scene<real> &s, Photon<real> &ph) {
+__device__ __forceinline__ void place_photon(const Scene<real> &s, Photon<real> &ph) {
   ph.steps = 0;
   ph.in_head = 0;
   ph.exclude = -1;
-  if (inside_box(ph.pos, s.bmin, s.bmax)) {
-    ph.in_image = 1;
-    ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-  } else {
-    ph.in_image = 0;
-    ph.can_enter = 1;
-  }
+  ph.in_image = inside_box(ph.pos, s.bmin, s.bmax) ? 1 : 0;
+  if (!ph.in_image) ph.can_enter = 1;
+}
+
+template <typename real>
+__device__ __forceinline__ void start_photon(const Scene<real> &s, Photon<real> &ph) {
+  place_photon(s, ph);
+  if (ph.in_image) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
 }
 
 }  // namespace gg

@@ -47,10 +47,11 @@ struct KernelArgs {
   void *records;                    // primary records of the batch (k_generate -> k_transport)
   size_t rec_cap;                   // records capacity (histories per batch)
   uint64_t rec_first;               // history of record 0 (<= h_begin; a SPECT pass can start later)
-  int refill_min;                   // lanes that must wait for a history before a refill phase
-  int interact_min;                 // pending collisions that trigger an interaction phase
+  int refill_min;                   // lanes that must wait for a history before a refill phase (phase kernels)
+  int interact_min;                 // pending collisions that trigger an interaction phase (phase kernels)
   unsigned long long *acc_d;        // dose grid: fixed-point sum(edep * rho_min / rho) (or null)
   unsigned long long *acc_d2;       // its history-by-history squares (or null)
+  void *slot_scratch;               // pooled kernels: PoolPlan::scratch bytes
 };
 
 // Bit of the kernel status word set when a stage queue overflowed (the low
@@ -160,7 +161,7 @@ __host__ __device__ inline size_t transport_smem_bytes(int n_comp, int n_e, int 
 }
 
 // Shared memory of `lists` per-history voxel lists of a block of `threads`
-// (one column per thread).
+// (one column per thread; the track-length estimator's kernel).
 template <typename real>
 __host__ __device__ constexpr size_t hist_list_bytes(int lists, int threads = kBlock) {
   return (size_t)lists * kHistList * (size_t)threads * (sizeof(uint32_t) + sizeof(real));
@@ -194,12 +195,45 @@ template <typename real>
 size_t record_bytes(size_t cap);
 template <typename real>
 cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStream_t st);
-// minb selects the kernel variant compiled for that many resident blocks per SM
+// Launch shape of a pooled transport kernel (gg_pool.cuh).
+struct PoolPlan {
+  int grid, block, gangs, slots;  // blocks, threads and gangs per block, photon slots per gang
+  size_t smem, scratch;           // dynamic shared memory; global scratch (KernelArgs::slot_scratch)
+};
+// Threads of a block (one block per SM), warps of a gang, entries of an event
+// queue's ring (more than a gang's slots).  Measured on the 256 x 256 x 160 CT,
+// 1e8 histories (transport ms): gangs of 2 / 3 / 4 / 6 / 12 warps of 24: 37.9 /
+// - / 33.5 / 32.5 / 34.6 (small gangs fetch more instructions, large ones wait
+// at their barrier); 16 / 18 / 20 / 24 warps in gangs of 4 / 3 / 4 / 4: 32.4 /
+// 30.4 / 30.4 / 33.5 (more warps leave fewer slots each).  FP64, 128 x 128 x 80
+// CT, 1e6 histories: 8 / 9 / 12 / 16 warps in gangs of 4 / 3 / 4 / 8: 4.64 /
+// 4.22 / 4.86 / 5.16 ms (FP64 units bound it: full rounds count, not warps).
 template <typename real>
-cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem,
-                             int minb, cudaStream_t st);
+struct PoolShape {
+  static constexpr int kBlock = 640, kGang = 4, kRing = 512;
+};
+template <>
+struct PoolShape<double> {
+  static constexpr int kBlock = 288, kGang = 3, kRing = 512;
+};
+// static shared memory of a pooled kernel, at most
 template <typename real>
-cudaError_t occupancy_blocks(int block, size_t smem, int minb, int *blocks_per_sm);
+__host__ __device__ constexpr int pool_static() {
+  using P = PoolShape<real>;
+  return 1024 + 16 * P::kBlock + (P::kBlock / (32 * P::kGang)) * (8 * P::kRing + 64);
+}
+template <typename real>
+cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, bool dose_list,
+                      PoolPlan *p);
+int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist);
+template <typename real>
+cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st);
+// track-length estimator; minb selects the kernel variant compiled for that many resident blocks per SM
+template <typename real>
+cudaError_t launch_transport_tle(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem, int minb,
+                                 cudaStream_t st);
+template <typename real>
+cudaError_t tle_occupancy(int block, size_t smem, int minb, int *blocks_per_sm);
 // Compacted wavefront dose transport (gg_wavefront.cu): 256-thread blocks,
 // dynamic shared memory = tables + photon slots.
 template <typename real>

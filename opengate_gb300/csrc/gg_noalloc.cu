@@ -40,6 +40,9 @@ namespace {
 
 constexpr size_t kScratchBytes = (size_t)GG_NOALLOC_SCRATCH_BYTES;
 constexpr int kMaxDevices = 64;
+// scratch of the transport's photon slots (24 bytes each): a slot for every
+// history of a batch on 152 SMs x 3 blocks, rounded up to 32 per block
+constexpr size_t kSlotBytes = (size_t)24 * 32 * 2500;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -51,7 +54,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // Offsets of the regions inside the scratch array for one call.
 struct Layout {
   size_t sig, cum, ray_amax, ray_x2, ray_cum, mat_rho, mat_comp, maj, spec_e, spec_cdf, acc_box;
-  size_t labels, acc_e, acc_e2, records, counters, next, status, end;
+  size_t labels, acc_e, acc_e2, records, slots, counters, next, status, end;
 };
 
 Layout make_layout(int n_comp, int n_e, int n_ray, int n_mat, size_t n_vox) {
@@ -77,6 +80,7 @@ Layout make_layout(int n_comp, int n_e, int n_ray, int n_mat, size_t n_vox) {
   L.acc_e = take(8 * n_vox);
   L.acc_e2 = take(16 * n_vox);  // 128-bit edep^2 accumulator per voxel
   L.records = take(gg::record_bytes<float>((size_t)GG_NOALLOC_BATCH));
+  L.slots = take(kSlotBytes);
   L.counters = take(8 * GG_N_COUNTERS);
   L.next = take(8);
   L.status = take(4);
@@ -271,13 +275,16 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
     s.spec_cdf = (const float *)(b + L.spec_cdf);
     s.acc_box = (const float *)(b + L.acc_box);
     // ---- kernels: source stage, transport, flush per batch -------------------
-    int n_sm = 0, bps = 0;
+    int n_sm = 0;
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
     size_t smem = gg::transport_smem_bytes<float>(t->n_comp, t->n_e, t->n_mat);
-    if ((e = gg::occupancy_blocks<float>(256, smem, 3, &bps)) != cudaSuccess) {
-      rc = fail(err, err_len, GG_ERR_CUDA, "occupancy: %s", cudaGetErrorString(e));
+    const uint64_t most = n_histories < (uint64_t)GG_NOALLOC_BATCH ? n_histories : (uint64_t)GG_NOALLOC_BATCH;
+    gg::PoolPlan plan{};
+    if ((e = gg::pool_plan<float>(device, smem, 0, 0, most, false, &plan)) != cudaSuccess) {
+      rc = fail(err, err_len, GG_ERR_CUDA, "launch shape: %s", cudaGetErrorString(e));
       break;
     }
+    if (plan.scratch > kSlotBytes) plan.grid = (int)((size_t)plan.grid * kSlotBytes / plan.scratch);
     gg::KernelArgs a;
     memset(&a, 0, sizeof(a));
     a.seed = seed;
@@ -286,7 +293,8 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
     a.acc_e2 = d_edep2 ? (unsigned long long *)(b + L.acc_e2) : nullptr;
     a.counters = (unsigned long long *)(b + L.counters);
     a.status = (unsigned int *)(b + L.status);
-    a.chunk = 256;
+    a.chunk = gg::pool_chunk(plan, 256, most);
+    a.slot_scratch = b + L.slots;
     a.records = b + L.records;
     a.rec_cap = (size_t)GG_NOALLOC_BATCH;
     a.refill_min = 8;
@@ -299,7 +307,7 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
                                                                             : first_history + n_histories;
       e = cudaMemsetAsync(a.next, 0, 8, st);
       if (e == cudaSuccess) e = gg::launch_generate<float>(s, a, st);
-      if (e == cudaSuccess) e = gg::launch_transport<float>(s, a, n_sm * (bps > 0 ? bps : 1), 256, smem, 3, st);
+      if (e == cudaSuccess) e = gg::launch_transport<float>(s, a, plan, st);
       if (e == cudaSuccess) e = gg::launch_flush(a.acc_e, a.acc_e2, d_edep, d_edep2, n_vox, n_sm * 8, st);
     }
     if (e != cudaSuccess) {

@@ -47,18 +47,20 @@ struct Tally {
 // do not depend on the order of the atomics, and a voxel hit by one history
 // has edep^2 == edep * edep exactly in these units.
 template <typename real>
-__device__ __forceinline__ void hlist_flush(HistList<real> &l, const Tally<real> &t, BlockCounters *bc) {
-  for (int k = 0; k < l.n; ++k) {
-    const unsigned long long q = (unsigned long long)to_fixed(l.acc[k * l.stride]);
-    const uint32_t v = l.vox[k * l.stride];
-    atomicAdd(&t.acc_e[v], q);
-    if (t.acc_e2) {
-      const unsigned long long lo = q * q;
-      const unsigned long long hi = __umul64hi(q, q);
-      atomicAdd(&t.acc_e2[2 * (size_t)v], lo & 0xffffffffull);
-      atomicAdd(&t.acc_e2[2 * (size_t)v + 1], (hi << 32) | (lo >> 32));
-    }
+__device__ __forceinline__ void tally_entry(const Tally<real> &t, uint32_t v, real x) {
+  const unsigned long long q = (unsigned long long)to_fixed(x);
+  atomicAdd(&t.acc_e[v], q);
+  if (t.acc_e2) {
+    const unsigned long long lo = q * q;
+    const unsigned long long hi = __umul64hi(q, q);
+    atomicAdd(&t.acc_e2[2 * (size_t)v], lo & 0xffffffffull);
+    atomicAdd(&t.acc_e2[2 * (size_t)v + 1], (hi << 32) | (lo >> 32));
   }
+}
+
+template <typename real>
+__device__ __forceinline__ void hlist_flush(HistList<real> &l, const Tally<real> &t, BlockCounters *bc) {
+  for (int k = 0; k < l.n; ++k) tally_entry(t, l.vox[k * l.stride], l.acc[k * l.stride]);
   if (l.n) atomicAdd(&bc->tally_entries, (unsigned int)l.n);
   l.n = 0;
 }
@@ -117,26 +119,30 @@ __device__ __forceinline__ void deposit(HistList<real> &l, const Tally<real> &t,
   l.n++;
 }
 
-// Klein-Nishina (G4KleinNishinaCompton sampling of the Physics Reference Manual)
-// The rejection loop of the Klein-Nishina sampling: eps = E'/E, 1 - cos(theta)
-// and sin^2(theta) of the scattering (3 draws per trial).
+// Klein-Nishina (G4KleinNishinaCompton sampling of the Physics Reference
+// Manual): the constants of a photon energy and one trial (3 draws) of the
+// rejection loop - eps = E'/E, 1 - cos(theta) and sin^2(theta); true when accepted.
 template <typename real>
-__device__ __forceinline__ void compton_kn(real e, Rng &g, BlockCounters *bc, real &eps, real &onecost,
-                                           real &sint2) {
-  real k = e * R<real>(1.0 / kMC2);
-  real twok = R<real>(2) * k;
-  real eps0 = R<real>(1) / (R<real>(1) + twok);
-  real eps0sq = eps0 * eps0;
-  real alpha1 = -gg_log(eps0);
-  real alpha2 = R<real>(1) - eps0sq;
-  alpha2 = R<real>(0.5) * alpha2;
-  alpha2 = alpha1 + alpha2;
-  real epssq;
-  int it = 0;
-  for (;;) {
-    real r0 = u01<real>(g);
-    real r1 = u01<real>(g);
-    real r2 = u01<real>(g);
+struct KleinNishina {
+  real k, eps0sq, alpha1, alpha2;
+
+  __device__ __forceinline__ explicit KleinNishina(real e) {
+    k = e * R<real>(1.0 / kMC2);
+    const real twok = R<real>(2) * k;
+    const real eps0 = R<real>(1) / (R<real>(1) + twok);
+    eps0sq = eps0 * eps0;
+    alpha1 = -gg_log(eps0);
+    alpha2 = R<real>(1) - eps0sq;
+    alpha2 = R<real>(0.5) * alpha2;
+    alpha2 = alpha1 + alpha2;
+  }
+  template <typename G>
+  __device__ __forceinline__ bool trial(G &g, real &eps, real &onecost, real &sint2) const {
+    g.reserve(3);
+    const real r0 = u01<real>(g);
+    const real r1 = u01<real>(g);
+    const real r2 = u01<real>(g);
+    real epssq;
     if (alpha1 > alpha2 * r0) {
       eps = gg_exp(-alpha1 * r1);
       epssq = eps * eps;
@@ -146,13 +152,23 @@ __device__ __forceinline__ void compton_kn(real e, Rng &g, BlockCounters *bc, re
       epssq = eps0sq + w;
       eps = gg_sqrt(epssq);
     }
-    real ek = eps * k;
+    const real ek = eps * k;
     onecost = (R<real>(1) - eps) / ek;
     sint2 = onecost * (R<real>(2) - onecost);
     real gr = eps * sint2;
     gr = gr / (R<real>(1) + epssq);
     gr = R<real>(1) - gr;
-    if (gr >= r2) break;
+    return gr >= r2;
+  }
+};
+
+// The whole rejection loop.
+template <typename real, typename G>
+__device__ __forceinline__ void compton_kn(real e, G &g, BlockCounters *bc, real &eps, real &onecost,
+                                           real &sint2) {
+  const KleinNishina<real> kn(e);
+  int it = 0;
+  while (!kn.trial(g, eps, onecost, sint2)) {
     if (++it >= kLoopCap) {
       atomicAdd(&bc->loop_capped, 1u);
       break;
@@ -160,19 +176,24 @@ __device__ __forceinline__ void compton_kn(real e, Rng &g, BlockCounters *bc, re
   }
 }
 
-// The rest of a Compton scattering sampled by compton_kn: azimuth (one draw),
-// new direction and energy; returns the energy given to the electron.
+// New direction after a scattering of cosine cost and squared sine st2: azimuth
+// (one draw) and rotation.
+template <typename real, typename G>
+__device__ __forceinline__ void scatter_dir(Photon<real> &ph, G &g, real cost, real st2) {
+  const real sint = gg_sqrt(st2 > R<real>(0) ? st2 : R<real>(0));
+  real sp, cp;
+  g.reserve(1);
+  gg_sincos_turn(u01<real>(g), sp, cp);
+  rotate_dir(ph.dir[0], ph.dir[1], ph.dir[2], cost, sint, cp, sp);
+}
+
+// The photon's energy after a Compton scattering to eps of it; returns the
+// energy given to the electron (all of it below the energy cut).
 template <typename real>
-__device__ __forceinline__ real compton_finish(const Scene<real> &s, Photon<real> &ph, Rng &g, real eps, real onecost,
-                                               real sint2) {
+__device__ __forceinline__ real compton_energy(const Scene<real> &s, Photon<real> &ph, real eps) {
   const real e = ph.e;
   real e1 = eps * e;
   real edep = e - e1;
-  real cost = R<real>(1) - onecost;
-  real sint = gg_sqrt(sint2 > R<real>(0) ? sint2 : R<real>(0));
-  real sp, cp;
-  gg_sincos_turn(u01<real>(g), sp, cp);
-  rotate_dir(ph.dir[0], ph.dir[1], ph.dir[2], cost, sint, cp, sp);
   if (e1 < s.e_min) {
     edep = edep + e1;
     ph.alive = 0;
@@ -182,8 +203,16 @@ __device__ __forceinline__ real compton_finish(const Scene<real> &s, Photon<real
   return edep;
 }
 
-template <typename real>
-__device__ __forceinline__ real compton(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc) {
+// The rest of a Compton scattering sampled by compton_kn.
+template <typename real, typename G>
+__device__ __forceinline__ real compton_finish(const Scene<real> &s, Photon<real> &ph, G &g, real eps, real onecost,
+                                               real sint2) {
+  scatter_dir(ph, g, R<real>(1) - onecost, sint2);
+  return compton_energy(s, ph, eps);
+}
+
+template <typename real, typename G>
+__device__ __forceinline__ real compton(const Scene<real> &s, Photon<real> &ph, G &g, BlockCounters *bc) {
   real eps, onecost, sint2;
   compton_kn(ph.e, g, bc, eps, onecost, sint2);
   return compton_finish(s, ph, g, eps, onecost, sint2);
@@ -191,8 +220,8 @@ __device__ __forceinline__ real compton(const Scene<real> &s, Photon<real> &ph, 
 
 // The rejection loop of the Rayleigh sampling (form-factor inversion, then
 // the 1 + cos^2 acceptance): cos(theta) of the scattering.
-template <typename real>
-__device__ __forceinline__ real rayleigh_cost(const Scene<real> &s, int comp, const Photon<real> &ph, Rng &g,
+template <typename real, typename G>
+__device__ __forceinline__ real rayleigh_cost(const Scene<real> &s, int comp, const Photon<real> &ph, G &g,
                                               BlockCounters *bc) {
   real k = ph.e * R<real>(1.0 / kHcMevAngstrom);
   real x2max = k * k;
@@ -206,11 +235,13 @@ __device__ __forceinline__ real rayleigh_cost(const Scene<real> &s, int comp, co
       atomicAdd(&bc->loop_capped, 1u);
       break;
     }
+    g.reserve(2);
     real r = u01<real>(g);
     real tt = r * amax;
     // exact inversion of the piecewise-linear cumulative: bisection for the
     // node interval, then linear in x^2 inside it
     int lo = 0, hi = s.n_ray - 1;
+#pragma unroll 1
     while (hi - lo > 1) {
       int mid = (lo + hi) >> 1;
       if (cu[mid] <= tt) lo = mid;
@@ -244,24 +275,21 @@ __device__ __forceinline__ real rayleigh_sint2(real cost) {
   return R<real>(1) - st2;
 }
 
-// The rest of a Rayleigh scattering of cosine cost: azimuth (one draw) and new direction.
-template <typename real>
-__device__ __forceinline__ void rayleigh_finish(Photon<real> &ph, Rng &g, real cost) {
-  const real st2 = rayleigh_sint2(cost);
-  real sint = gg_sqrt(st2 > R<real>(0) ? st2 : R<real>(0));
-  real sp, cp;
-  gg_sincos_turn(u01<real>(g), sp, cp);
-  rotate_dir(ph.dir[0], ph.dir[1], ph.dir[2], cost, sint, cp, sp);
+// The rest of a Rayleigh scattering of cosine cost.
+template <typename real, typename G>
+__device__ __forceinline__ void rayleigh_finish(Photon<real> &ph, G &g, real cost) {
+  scatter_dir(ph, g, cost, rayleigh_sint2(cost));
 }
 
-template <typename real>
-__device__ __forceinline__ void rayleigh(const Scene<real> &s, int comp, Photon<real> &ph, Rng &g,
+template <typename real, typename G>
+__device__ __forceinline__ void rayleigh(const Scene<real> &s, int comp, Photon<real> &ph, G &g,
                                          BlockCounters *bc) {
   rayleigh_finish(ph, g, rayleigh_cost(s, comp, ph, g, bc));
 }
 
-template <typename real>
-__device__ __forceinline__ void iso_dir(Rng &g, real d[3]) {
+template <typename real, typename G>
+__device__ __forceinline__ void iso_dir(G &g, real d[3]) {
+  g.reserve(2);
   real cost = R<real>(2) * u01<real>(g);
   cost = R<real>(1) - cost;
   real st2 = cost * cost;
@@ -291,8 +319,8 @@ struct Secondary {
 // Process of an interaction at energy index ph.ei in material `mat`: the
 // first draw of the interaction against the cumulative fractions (Compton,
 // + photoelectric, + Rayleigh; the rest is pair production).
-template <typename real>
-__device__ __forceinline__ int select_kind(const Scene<real> &s, const Photon<real> &ph, int mat, Rng &g) {
+template <typename real, typename G>
+__device__ __forceinline__ int select_kind(const Scene<real> &s, const Photon<real> &ph, int mat, G &g) {
   int c = s.mat_comp[mat];
   const real *cu = s.cum + (size_t)c * 3 * s.n_e;
   real r = u01<real>(g);
@@ -305,20 +333,11 @@ __device__ __forceinline__ int select_kind(const Scene<real> &s, const Photon<re
   return kPair;
 }
 
-// The interaction of process `kind` (after select_kind).  Returns the energy
-// deposited locally (scored by the caller when inside the image).
-template <typename real>
-__device__ __forceinline__ real apply_kind(const Scene<real> &s, Photon<real> &ph, int mat, int kind, Rng &g,
-                                           BlockCounters *bc, Secondary<real> &sec) {
-  if (kind == kCompton) return compton(s, ph, g, bc);
-  if (kind == kPhoto) {
-    ph.alive = 0;
-    return ph.e;
-  }
-  if (kind == kRayleigh) {
-    rayleigh(s, s.mat_comp[mat], ph, g, bc);
-    return R<real>(0);
-  }
+// Pair conversion: both leptons stop, the positron's annihilation photons
+// leave back to back; the photon goes on as one of them, the other waits in sec.
+template <typename real, typename G>
+__device__ __forceinline__ real pair_conversion(const Scene<real> &s, Photon<real> &ph, G &g, BlockCounters *bc,
+                                                Secondary<real> &sec) {
   real ekin = ph.e - R<real>(2.0 * kMC2);
   real d[3];
   iso_dir(g, d);
@@ -339,10 +358,27 @@ __device__ __forceinline__ real apply_kind(const Scene<real> &s, Photon<real> &p
   return ekin;
 }
 
+// The interaction of process `kind` (after select_kind).  Returns the energy
+// deposited locally (scored by the caller when inside the image).
+template <typename real, typename G>
+__device__ __forceinline__ real apply_kind(const Scene<real> &s, Photon<real> &ph, int mat, int kind, G &g,
+                                           BlockCounters *bc, Secondary<real> &sec) {
+  if (kind == kCompton) return compton(s, ph, g, bc);
+  if (kind == kPhoto) {
+    ph.alive = 0;
+    return ph.e;
+  }
+  if (kind == kRayleigh) {
+    rayleigh(s, s.mat_comp[mat], ph, g, bc);
+    return R<real>(0);
+  }
+  return pair_conversion(s, ph, g, bc, sec);
+}
+
 // Interaction at ph.pos in material `mat`.  Returns the energy deposited
 // locally (scored by the caller when inside the image).
-template <typename real>
-__device__ __forceinline__ real interact(const Scene<real> &s, Photon<real> &ph, int mat, Rng &g,
+template <typename real, typename G>
+__device__ __forceinline__ real interact(const Scene<real> &s, Photon<real> &ph, int mat, G &g,
                                          BlockCounters *bc, Secondary<real> &sec, int *kind = nullptr) {
   const int k = select_kind(s, ph, mat, g);
   if (kind) *kind = k;
@@ -1019,8 +1055,8 @@ struct TleScore {
 // photon at or below the estimator's threshold first stops (depositing its
 // energy in its voxel) when at or below the kill energy, else scores the
 // path of the step.
-template <typename real, bool TLE = false>
-__device__ __forceinline__ int image_flight(const Scene<real> &s, Photon<real> &ph, Rng &g, int &pmat, uint32_t &pv,
+template <typename real, bool TLE = false, typename G = Rng>
+__device__ __forceinline__ int image_flight(const Scene<real> &s, Photon<real> &ph, G &g, int &pmat, uint32_t &pv,
                                             int &pscored, unsigned int &n_wood, unsigned int &n_real,
                                             BlockCounters *bc = nullptr, TleScore<real> sc = {nullptr, nullptr, nullptr}) {
   {
@@ -1064,52 +1100,12 @@ __device__ __forceinline__ int image_flight(const Scene<real> &s, Photon<real> &
   }
 }
 
-template <typename real, bool SPECT, bool TLE = false>
-__device__ __forceinline__ int flight(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc, int &pmat,
-                                      uint32_t &pv, int &pscored, unsigned int &n_wood, unsigned int &n_real,
-                                      unsigned int &n_world, unsigned int &n_head,
-                                      TleScore<real> sc = {nullptr, nullptr, nullptr}) {
-  if (++ph.steps > kStepCap) {
-    atomicAdd(&bc->loop_capped, 1u);
-    ph.alive = 0;
-    return kRefill;
-  }
-  if (ph.in_image) {
-    const int r = image_flight<real, TLE>(s, ph, g, pmat, pv, pscored, n_wood, n_real, bc, sc);
-    if constexpr (SPECT) return r;
-    if (r != kFly || ph.in_image) return r;
-    // Left the image box: take the world step at once (the same flight
-    // count and draws as a separate phase, one block iteration fewer).
-    if (++ph.steps > kStepCap) {
-      atomicAdd(&bc->loop_capped, 1u);
-      ph.alive = 0;
-      return kRefill;
-    }
-  }
-  if constexpr (SPECT) {
-    if (ph.in_head) {
-      ++n_head;
-      int mat;
-      if (head_flight(s, ph, g, mat)) {
-        pmat = mat;
-        pscored = ph.hreg == s.hreg_cr ? 2 : 3;
-        return kInteract;
-      }
-      return ph.alive ? kFly : kRefill;  // (stopped by a shielded side)
-    }
-    ++n_world;
-    if (spect_world_flight(s, ph, g)) {
-      pmat = s.world_mat;
-      pscored = 0;
-      return kInteract;
-    }
-    if (!ph.alive) {
-      atomicAdd(&bc->escaped, 1u);
-      return kRefill;
-    }
-    return kFly;
-  }
-  ++n_world;
+// One free flight in the world (dose path): to a collision in the world
+// material, to the image box (kFly; the path inside it is the caller's), or
+// out of the world (kRefill).
+template <typename real, typename G>
+__device__ __forceinline__ int dose_world_flight(const Scene<real> &s, Photon<real> &ph, G &g, int &pmat,
+                                                 int &pscored) {
   real inf = gg_inf(real(0));
   real tin = ph.can_enter ? entry_distance(ph.pos, ph.dir, s.bmin, s.bmax) : inf;
   real wlo[3] = {-s.whalf[0], -s.whalf[1], -s.whalf[2]};
@@ -1131,12 +1127,37 @@ __device__ __forceinline__ int flight(const Scene<real> &s, Photon<real> &ph, Rn
 #pragma unroll
     for (int a = 0; a < 3; ++a) ph.pos[a] = ph.pos[a] + tin * ph.dir[a];
     ph.in_image = 1;
-    ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
     return kFly;
   }
   ph.alive = 0;
-  atomicAdd(&bc->escaped, 1u);
   return kRefill;
+}
+
+template <typename real, bool TLE = false>
+__device__ __forceinline__ int flight(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc, int &pmat,
+                                      uint32_t &pv, int &pscored, unsigned int &n_wood, unsigned int &n_real,
+                                      unsigned int &n_world, TleScore<real> sc = {nullptr, nullptr, nullptr}) {
+  if (++ph.steps > kStepCap) {
+    atomicAdd(&bc->loop_capped, 1u);
+    ph.alive = 0;
+    return kRefill;
+  }
+  if (ph.in_image) {
+    const int r = image_flight<real, TLE>(s, ph, g, pmat, pv, pscored, n_wood, n_real, bc, sc);
+    if (r != kFly || ph.in_image) return r;
+    // Left the image box: take the world step at once (the same flight
+    // count and draws as a separate phase, one block iteration fewer).
+    if (++ph.steps > kStepCap) {
+      atomicAdd(&bc->loop_capped, 1u);
+      ph.alive = 0;
+      return kRefill;
+    }
+  }
+  ++n_world;
+  const int r = dose_world_flight(s, ph, g, pmat, pscored);
+  if (r == kFly) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
+  if (r == kRefill) atomicAdd(&bc->escaped, 1u);
+  return r;
 }
 
 // A crystal hit of head H added to the event (GateDigiAdderInVolume::Update,
@@ -1201,37 +1222,10 @@ __device__ __forceinline__ bool dose_voxel(const Scene<real> &s, const real p[3]
   return true;
 }
 
-// do_interaction of the dose path with the tally on its own grid
-// (GateDoseActor::SteppingAction, GateDoseActor.cpp:180-243: the deposit is
-// scored in the dose-grid voxel of the interaction point, when there is one;
-// DG 2: also edep * rho_min / rho of the material there in the dose list ld).
-template <typename real, int DG>
-__device__ __forceinline__ int do_interaction_grid(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc,
-                                                   int pmat, int pscored, HistList<real> &l, HistList<real> &ld,
-                                                   const Tally<real> &t, const Tally<real> &td,
-                                                   Secondary<real> &sec, unsigned int &n_dep, BlockCounters *bcd) {
-  const real ed = interact(s, ph, pmat, g, bc, sec);
-  if (pscored == 1) {
-    uint32_t dv;
-    if (dose_voxel(s, ph.pos, dv)) {
-      deposit(l, t, bc, dv, ed, n_dep);
-      if constexpr (DG == 2) {
-        real dd = ed * s.drho_min;
-        dd = dd / s.mat_rho[pmat];
-        unsigned int nd = 0;
-        deposit(ld, td, bcd, dv, dd, nd);
-      }
-    }
-    if (ph.alive && ph.in_image) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-  } else if (pscored == 0) {
-    ph.can_enter = 1;
-    ph.exclude = -1;
-  }
-  return ph.alive ? kFly : kRefill;
-}
-
+// The waiting annihilation photon becomes the photon in flight (placed, its
+// path in the image still to be computed).
 template <typename real>
-__device__ __forceinline__ void pop_secondary(const Scene<real> &s, Photon<real> &ph, Secondary<real> &sec) {
+__device__ __forceinline__ void take_secondary(const Scene<real> &s, Photon<real> &ph, Secondary<real> &sec) {
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     ph.pos[a] = sec.at(a);
@@ -1240,7 +1234,13 @@ __device__ __forceinline__ void pop_secondary(const Scene<real> &s, Photon<real>
   sec.has = 0;
   ph.alive = 1;
   set_energy(s, ph, R<real>(kMC2));
-  start_photon(s, ph);
+  place_photon(s, ph);
+}
+
+template <typename real>
+__device__ __forceinline__ void pop_secondary(const Scene<real> &s, Photon<real> &ph, Secondary<real> &sec) {
+  take_secondary(s, ph, sec);
+  if (ph.in_image) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
 }
 
 // Batched launches: the lane's scene geometry, source and tally pointers

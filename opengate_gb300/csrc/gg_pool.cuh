@@ -1,0 +1,300 @@
+// gg_pool.cuh - photon slots and event queues of the pooled transport kernels.
+//
+// A gang of warps owns more photon slots than it has threads; their whole
+// state lives in shared memory, with one queue of slot numbers per kind of next
+// event.  Every round the gang picks its longest queue, each thread takes one
+// slot of it, runs that event, stores the photon back and appends the slot to
+// the queue of the photon's next event.  Nearly every lane of a round has a
+// photon: one photon per thread instead kept 8.6 of 32 lanes active, since a
+// lane could only wait for its own photon's kind of event to come up.
+//
+// The warps of a gang run one code region at a time because the kernels are
+// sensitive to instruction fetch; the gangs of a block share its tables and
+// run on their own, so one gang's barrier is covered by the others.
+//
+// One barrier per round: the pushes of round k are counted in push[(k + 1) % 3]
+// and read by every thread after the barrier that opens round k + 1; the set
+// of the round after is cleared meanwhile.  A round takes no more entries than
+// its ring has free, so its pushes never overwrite an entry that a slower warp
+// still has to read.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "gg_device.cuh"
+#include "gg_internal.h"
+#include "gg_physics.cuh"
+#include "gg_tc.cuh"
+
+namespace gg {
+
+enum : int { kQRefill = 0, kQFly = 1, kQWorld = 2, kQInteract = 3, kQueues = 4, kQNone = 4 };
+// A gang's event queues.  cnt / tail are the same in every thread: queue
+// lengths and ring positions, 16 bits each (queues 0, 1 in x, 2, 3 in y).
+template <int kPoolRing>
+struct EventQueues {
+  static_assert((kPoolRing & (kPoolRing - 1)) == 0 && kPoolRing <= 1024, "ring positions are masked, packed in 16 bits");
+  uint16_t *ring;     // [kQueues][kPoolRing]
+  unsigned *push;     // [3][kQueues]
+  uint2 cnt, tail;
+  unsigned rd;        // push set of this round's barrier, rotates through 0, 1, 2
+  unsigned tid, size; // the thread in its gang, the gang's threads
+  int bar;            // named barrier
+
+  // every slot waits for a history; the caller's next round() opens with the barrier
+  __device__ __forceinline__ void init(int gang, unsigned t, unsigned n, uint16_t *r, unsigned *p, unsigned slots) {
+    tid = t;
+    size = n;
+    bar = 1 + gang;
+    ring = r;
+    push = p;
+    for (unsigned i = tid; i < slots; i += size) ring[kQRefill * kPoolRing + i] = (uint16_t)i;
+    if (tid < 3 * kQueues) push[tid] = 0u;
+    cnt = make_uint2(slots, 0u);  // (kQRefill is queue 0)
+    tail = make_uint2(slots & (kPoolRing - 1u), 0u);
+    rd = 0u;
+  }
+  __device__ __forceinline__ void sync() const { named_bar(bar, (int)size); }
+
+  // The event of this round (kQNone: no slot is left) and the thread's slot
+  // (-1: none); n: threads that have one.
+  __device__ __forceinline__ int round(int &slot, unsigned &n) {
+    constexpr unsigned kMask = (kPoolRing - 1u) * 0x10001u;
+    sync();
+    const uint4 p = reinterpret_cast<const uint4 *>(push)[rd];
+    const unsigned clr = rd == 0u ? 2u : rd - 1u;  // (rd + 2) % 3: the set after next
+    if (tid == 0) reinterpret_cast<uint4 *>(push)[clr] = make_uint4(0u, 0u, 0u, 0u);
+    rd = rd == 2u ? 0u : rd + 1u;  // the set this round pushes to
+    const unsigned ax = p.x | (p.y << 16), ay = p.z | (p.w << 16);
+    cnt.x += ax;
+    cnt.y += ay;
+    tail.x = (tail.x + ax) & kMask;
+    tail.y = (tail.y + ay) & kMask;
+    // the longest queue: length * 4 + queue
+    const unsigned best = max(max((cnt.x & 0xffffu) << 2, ((cnt.x >> 14) & ~3u) | 1u),
+                              max(((cnt.y & 0xffffu) << 2) | 2u, ((cnt.y >> 14) & ~3u) | 3u));
+    const unsigned q = best & 3u, len = best >> 2, sh = (q & 1u) << 4;
+    n = min(min(len, size), (unsigned)kPoolRing - len);
+    slot = -1;
+    if (len == 0u) return kQNone;
+    const unsigned head = ((q & 2u ? tail.y : tail.x) >> sh) - len;
+    if (tid < n) slot = ring[q * kPoolRing + ((head + tid) & (kPoolRing - 1u))];
+    if (q & 2u) cnt.y -= n << sh;
+    else cnt.x -= n << sh;
+    return (int)q;
+  }
+
+  // Appends the lane's slot to queue `dest` (kQNone: nowhere); every lane of the warp calls it.
+  __device__ __forceinline__ void put(int dest, int slot, unsigned lane, unsigned lt_mask) {
+    const unsigned b0 = __ballot_sync(0xffffffffu, dest == 0), b1 = __ballot_sync(0xffffffffu, dest == 1),
+                   b2 = __ballot_sync(0xffffffffu, dest == 2), b3 = __ballot_sync(0xffffffffu, dest == 3);
+    const unsigned m = dest & 2 ? (dest & 1 ? b3 : b2) : (dest & 1 ? b1 : b0);
+    const unsigned rank = __popc(m & lt_mask);
+    unsigned off = 0u;
+    if (dest < kQueues && rank == 0u) off = atomicAdd(&push[rd * kQueues + (unsigned)dest], __popc(m));
+    off = __shfl_sync(0xffffffffu, off, __ffs(m) - 1);  // (the lane's own value is unused when m is 0)
+    const unsigned t = (dest & 2 ? tail.y : tail.x) >> ((dest & 1) << 4);
+    if (dest < kQueues) ring[(unsigned)dest * kPoolRing + ((t + off + rank) & (kPoolRing - 1u))] = (uint16_t)slot;
+  }
+};
+
+// Four reals that move as 16-byte words.
+template <typename real>
+struct alignas(16) Real4 {
+  real x, y, z, w;
+};
+__device__ __forceinline__ float bits_real(float, uint32_t u) { return __uint_as_float(u); }
+__device__ __forceinline__ double bits_real(double, uint32_t u) { return __longlong_as_double((long long)u); }
+__device__ __forceinline__ uint32_t real_bits(float v) { return __float_as_uint(v); }
+__device__ __forceinline__ uint32_t real_bits(double v) { return (uint32_t)__double_as_longlong(v); }
+
+// meta word of a slot: steps (20 bits) | words of the Philox buffer used (3) |
+// exclude + 1 (2) | pending interaction in the image (1) | waiting secondary
+// (1) | list length (4) | Compton sampling not finished (1)
+constexpr uint32_t kSlSteps = (1u << 20) - 1u;
+constexpr int kSlIdx = 20, kSlExcl = 23, kSlImage = 25, kSlSec = 26, kSlList = 27, kSlRetry = 31;
+static_assert(kStepCap < (1 << 20), "the step count has 20 bits in the slot's meta word");
+static_assert(kHistList < 16, "the list length has 4 bits in the slot's meta word");
+
+// A photon slot in shared memory.  a: position, path to the image boundary (a
+// pending interaction: its voxel); b: direction, energy; c: majorant (Compton
+// sampling not finished: rejected trials), its inverse, energy-grid fraction,
+// energy index | material << 16; rng: the Philox block being drawn from; e:
+// next block, record of the history, meta, a word of the kernel's own; vox,
+// acc: the history's voxel list.  The stride is an odd number of 16-byte
+// words, so slots spread over the banks.
+template <typename real>
+struct PhotonSlot {
+  Real4<real> a, b, c;
+  uint4 rng, e;
+  uint32_t vox[kHistList];
+  alignas(16) real acc[kHistList];
+};
+template <>
+struct PhotonSlot<double> {
+  Real4<double> a, b, c;
+  uint4 rng, e;
+  uint32_t vox[kHistList];
+  alignas(16) double acc[kHistList];
+  uint4 pad;
+};
+static_assert(sizeof(PhotonSlot<float>) % 32 == 16 && sizeof(PhotonSlot<double>) % 32 == 16, "odd 16-byte stride");
+static_assert(kHistList == 8, "list_deposit reads the voxels as two 16-byte words");
+
+// The stream of one event: the slot's block (words idx .. 3 left) and the one
+// after it, made when the event begins while the warp is converged, so the
+// draws inside divergent code seldom call the generator.  The words live in
+// shared memory (a register window would be selected word by word); reserve(n)
+// comes before n draws.
+struct EventRng {
+  uint32_t *buf, *nxt;  // the slot's block, the thread's own block
+  uint32_t k0, k1, stream, h0, h1;
+  uint32_t blk;         // number of nxt's block
+  int idx;              // 0 .. 8: words used of buf, nxt
+
+  __device__ __forceinline__ void begin() {
+    *reinterpret_cast<uint4 *>(nxt) = philox_block(blk, stream, h0, h1, k0, k1);
+  }
+  // nxt becomes the slot's block
+  __device__ __forceinline__ void shift() {
+    *reinterpret_cast<uint4 *>(buf) = *reinterpret_cast<const uint4 *>(nxt);
+    blk += 1u;
+    idx -= 4;
+  }
+  __device__ __forceinline__ void reserve(int n) {
+    if (idx + n > 8) {
+      shift();
+      begin();
+    }
+  }
+  __device__ __forceinline__ uint32_t next() {
+    const uint32_t v = idx < 4 ? buf[idx] : nxt[idx - 4];
+    ++idx;
+    return v;
+  }
+  // the slot's state after the event: nxt becomes its block when words of it are drawn
+  __device__ __forceinline__ void end() {
+    if (idx > 4) shift();
+  }
+};
+
+// The one or two words of a flight, drawn while the warp is converged: at most
+// one block is made, by the lanes whose buffer runs out.
+struct TwoWords {
+  uint32_t w[2];
+  uint4 nb;
+  int used;
+
+  __device__ __forceinline__ void draw(const uint32_t *buf, uint32_t blk, int idx, uint32_t stream, uint32_t h0,
+                                       uint32_t h1, uint32_t k0, uint32_t k1) {
+    if (idx > 2) nb = philox_block(blk, stream, h0, h1, k0, k1);
+    w[0] = idx < 4 ? buf[idx & 3] : nb.x;
+    w[1] = idx < 3 ? buf[(idx + 1) & 3] : (idx == 3 ? nb.x : nb.y);
+    used = 0;
+  }
+  __device__ __forceinline__ uint32_t next() {
+    const uint32_t v = used == 0 ? w[0] : w[1];
+    ++used;
+    return v;
+  }
+  // the slot's state after `used` draws
+  __device__ __forceinline__ void end(uint32_t *buf, uint32_t &blk, int &idx) const {
+    idx += used;
+    if (idx > 4) {
+      *reinterpret_cast<uint4 *>(buf) = nb;
+      blk += 1u;
+      idx -= 4;
+    }
+  }
+};
+
+// A history's voxel list in its slot (the entries of HistList, in their order).
+// deposit(): all voxels are compared at once - a loop over the entries makes
+// the warp wait for its longest list.
+template <typename real>
+__device__ __forceinline__ void list_deposit(PhotonSlot<real> &S, int &n, const Tally<real> &t, uint32_t v, real e,
+                                             unsigned int &n_dep, unsigned int &n_entries, unsigned int &n_over) {
+  if (!(e > R<real>(0))) return;
+  ++n_dep;
+  const uint4 a = *reinterpret_cast<const uint4 *>(S.vox), b = *reinterpret_cast<const uint4 *>(S.vox + 4);
+  const uint32_t u[kHistList] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  int at = n;
+#pragma unroll
+  for (int k = kHistList - 1; k >= 0; --k)
+    if (k < n && u[k] == v) at = k;
+  if (at < n) {
+    S.acc[at] = S.acc[at] + e;
+    return;
+  }
+  if (n == kHistList) {
+    ++n_over;
+    n_entries += kHistList;
+#pragma unroll 1
+    for (int k = 0; k < kHistList; ++k) tally_entry(t, S.vox[k], S.acc[k]);
+    n = at = 0;
+  }
+  S.vox[at] = v;
+  S.acc[at] = e;
+  n = at + 1;
+}
+
+// The lists of the warp's ended histories (`n` entries of the lane's slot
+// `slot`) into the tallies: the entries are dealt over the lanes, one each -
+// about 1.5 per history, but the longest of 32 lists has 4 or 5.  ids: 32 *
+// kHistList numbers of the warp's own.  tally_of(slot): the slot's tally.
+template <typename real, typename TallyOf>
+__device__ __forceinline__ void lists_flush(const PhotonSlot<real> *slots, int slot, int n, uint16_t *ids, unsigned lane,
+                                            TallyOf &&tally_of, unsigned int &n_entries) {
+  unsigned end = (unsigned)n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned x = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= (unsigned)o) end += x;
+  }
+  const unsigned total = __shfl_sync(0xffffffffu, end, 31);
+  uint16_t *p = ids + (end - (unsigned)n);
+#pragma unroll
+  for (int k = 0; k < kHistList; ++k)
+    if (k < n) p[k] = (uint16_t)(slot * kHistList + k);
+  __syncwarp();
+#pragma unroll 1
+  for (unsigned i = lane; i < total; i += 32u) {
+    const unsigned id = ids[i];
+    const PhotonSlot<real> &S = slots[id / kHistList];
+    tally_entry(tally_of(S), S.vox[id % kHistList], S.acc[id % kHistList]);
+  }
+  n_entries += (unsigned)n;
+  __syncwarp();
+}
+
+// The second list of a dose grid that scores dose too, in global memory:
+// [kHistList][slots] sums and voxels.
+template <typename real>
+struct GlobalList {
+  real *ga;
+  uint32_t *gv;
+  size_t slots, at;
+  int n;
+
+  __device__ __forceinline__ void flush(const Tally<real> &t) {
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) tally_entry(t, gv[(size_t)k * slots + at], ga[(size_t)k * slots + at]);
+    n = 0;
+  }
+  __device__ __forceinline__ void deposit(const Tally<real> &t, uint32_t v, real e) {
+    if (!(e > R<real>(0))) return;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k)
+      if (gv[(size_t)k * slots + at] == v) {
+        ga[(size_t)k * slots + at] += e;
+        return;
+      }
+    if (n == kHistList) flush(t);
+    gv[(size_t)n * slots + at] = v;
+    ga[(size_t)n * slots + at] = e;
+    ++n;
+  }
+};
+
+}  // namespace gg

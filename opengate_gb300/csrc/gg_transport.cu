@@ -7,29 +7,32 @@
 // FlushSquaredValues (core/opengate_core/opengate_lib/GateDoseActor.cpp:180-243, 359-397).
 //
 // Kernel design (one GB300, one process):
-//   * persistent grid, one photon history per thread at a time; a warp claims
-//     histories from a global counter in chunks (one atomic per chunk) and
-//     hands them to its lanes as they finish (ballot + popc), so no lane idles
-//     while work remains;
+//   * a source stage samples the primaries into coalesced records;
+//   * the transport stage keeps more photons than threads in shared memory and
+//     runs one kind of event at a time on full warps (gg_pool.cuh); only the
+//     track-length estimator still carries one photon per thread;
 //   * Woodcock (delta) tracking against a per-energy majorant inside the image
 //     box; analytic free flight in the world material outside it;
 //   * the majorant, total attenuation rows and the label->(composition,
 //     density) table are staged in shared memory; labels are read through the
 //     read-only path (the image is L2-resident up to ~60 M voxels);
-//   * every history keeps its deposits in a register list of (voxel, sum);
-//     when the history ends each entry adds q = round(sum * 2^32) to the edep
-//     tally (64-bit integer atomic) and q^2 to a 128-bit edep-squared tally:
-//     the history-by-history squared sum of GateDoseActor, order independent
-//     and therefore bit-reproducible;
-//   * a second kernel flushes the per-batch fixed-point tallies into the
+//   * every history keeps its deposits in a list of (voxel, sum); when the
+//     history ends each entry adds q = round(sum * 2^32) to the edep tally
+//     (64-bit integer atomic) and q^2 to a 128-bit edep-squared tally: the
+//     history-by-history squared sum of GateDoseActor, order independent and
+//     therefore bit-reproducible;
+//   * a third kernel flushes the per-batch fixed-point tallies into the
 //     float64 images (and clears them), one voxel per thread, coalesced.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "gg_device.cuh"
 #include "gg_internal.h"
 #include "gg_physics.cuh"
+#include "gg_pool.cuh"
+#include "gg_queue.cuh"
 #include "gg_spect.cuh"
 
 namespace gg {
@@ -172,7 +175,337 @@ __global__ void __launch_bounds__(256) k_generate(Scene<real> s, KernelArgs a) {
   }
 }
 
-// Transport stage.  Persistent grid; each lane carries one history at a time
+// Adds the lanes' counts to a counter (out of line: one copy of the exchange).
+static __device__ __noinline__ void warp_count(unsigned long long *counter, unsigned int v) {
+  unsigned long long x = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  if ((threadIdx.x & 31u) == 0u && x) atomicAdd(counter, x);
+}
+
+// The dose tally from voxel `off` on (batched simulations: the simulation's part).
+template <typename real>
+__device__ __forceinline__ Tally<real> tally_at(const KernelArgs &a, size_t off, real) {
+  return Tally<real>{a.acc_e + off, a.acc_e2 ? a.acc_e2 + 2 * off : nullptr};
+}
+
+// Compton trials of one interaction event; a photon that is rejected as often
+// waits for the next event with the photons it meets there, instead of keeping
+// its warp in the loop (a third of the trials fail; the worst of 32 lanes takes
+// five or six).
+constexpr int kKnTrials = 2;
+
+// Transport stage: the pooled event loop of gg_pool.cuh.  Events: a new history
+// (the ended one's voxel list goes to the tallies first), a Woodcock step in
+// the image, a free flight in the world, an interaction; a photon that starts
+// or scatters in the image takes its next Woodcock step in the same round.
+// The order of operations inside each history, hence its result, does not
+// depend on which lane or round executes them.
+// Bound by instruction issue and by the gangs' barrier: 256 x 256 x 160 CT, 1e8
+// histories to 6 MeV, 47.9 -> 30.4 ms against one photon per thread with block-wide phases
+// (203 warp instructions per history at 21.5 active lanes; 379 at 8.6); 24
+// batched simulations 22.8 -> 14.1 ms, FP64 9.2 -> 4.2 ms per 1e6.
+// MULTI: batched simulations; DG: dose tally on a grid of its own (1: edep,
+// 2: edep and dose), Scene::dgrid.
+template <typename real, bool MULTI, int DG>
+__global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(Scene<real> sg, KernelArgs args, int n_slots) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ BlockCounters bc;
+  using Shape = PoolShape<real>;
+  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
+  __shared__ __align__(16) unsigned push[kGangs][3 * kQueues];
+  __shared__ __align__(16) uint32_t ahead[Shape::kBlock][4];  // EventRng's second block of each thread
+  __shared__ uint16_t ring[kGangs][kQueues * Shape::kRing];
+  __shared__ unsigned long long s_claim[kGangs];
+  Scene<real> s = sg;
+  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
+  const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
+  const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
+  // dynamic shared memory: slots of the gangs, tables
+  PhotonSlot<real> *const slots = reinterpret_cast<PhotonSlot<real> *>(smem_raw) + gang * n_slots;
+  EventQueues<Shape::kRing> Q;
+  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
+         (unsigned)n_slots);
+  for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) slots[i].e = make_uint4(0u, 0u, 0u, 0u);
+  stage_tables(sg, s, smem_raw + sizeof(PhotonSlot<real>) * (size_t)(gangs * n_slots), bc);
+
+  const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
+  Tally<real> t{args.acc_e, args.acc_e2};
+  const Tally<real> td{args.acc_d, args.acc_d2};
+  const uint32_t n_hist = (uint32_t)(args.h_end - args.h_begin);
+  const uint32_t slot0 = (blockIdx.x * (uint32_t)gangs + (uint32_t)gang) * (uint32_t)n_slots;
+  const uint32_t all_slots = gridDim.x * (uint32_t)(gangs * n_slots);  // global scratch: one column per slot
+  Secondary<real> sec;
+  sec.base = reinterpret_cast<real *>(args.slot_scratch);
+  sec.stride = (int)all_slots;
+  GlobalList<real> ld;
+  ld.ga = sec.base + 6 * (size_t)all_slots;
+  ld.gv = reinterpret_cast<uint32_t *>(ld.ga + kHistList * (size_t)all_slots);
+  ld.slots = all_slots;
+  unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0, n_ent = 0, n_over = 0, n_esc = 0;
+  uint32_t pool_next = 0, pool_end = 0;  // claimed records not yet handed out (the same in the whole gang)
+  bool exhausted = false;
+
+  for (;;) {
+    int k;
+    unsigned n;
+    const int event = Q.round(k, n);
+    if (event == kQNone) break;
+    int dest = kQNone;
+    uint32_t base = 0, got = 0;
+    const uint32_t avail = pool_end - pool_next;
+    if (event == kQRefill) {
+      // the n slots take the next n records in thread order (coalesced loads)
+      if (avail < n && !exhausted) {
+        if (Q.tid == 0) s_claim[gang] = atomicAdd(args.next, (unsigned long long)args.chunk);
+        Q.sync();
+        const unsigned long long c = s_claim[gang];
+        if (c < n_hist) {
+          base = (uint32_t)c;
+          got = min((uint32_t)args.chunk, n_hist - base);
+        }
+        exhausted = c + (unsigned long long)args.chunk >= n_hist;
+      }
+      // the ended histories' voxel lists
+      lists_flush(slots, max(k, 0), k >= 0 ? (int)((slots[k].e.z >> kSlList) & 15u) : 0,
+                  reinterpret_cast<uint16_t *>(ahead[threadIdx.x & ~31u]), lane,
+                  [&](const PhotonSlot<real> &S) {
+                    if constexpr (MULTI) return tally_at(args, sg.sims[S.e.w].vox_off, real(0));
+                    else return t;
+                  },
+                  n_ent);
+    }
+    if (k >= 0) {
+      PhotonSlot<real> &S = slots[k];
+      uint4 e = S.e;
+      int n_list = (int)((e.z >> kSlList) & 15u);
+      if constexpr (DG == 2) {
+        ld.at = slot0 + (uint32_t)k;
+        ld.n = (int)e.w;
+      }
+      auto bind = [&](uint32_t sim) {  // batched simulations: the history's geometry, majorant and tally
+        const SimDesc<real> &d = sg.sims[sim];
+        bind_geometry(s, d, sg.labels, sg.sim_maj + (size_t)sim * sg.n_e);
+        t = tally_at(args, d.vox_off, real(0));
+      };
+      if constexpr (MULTI) bind(e.w);
+      Photon<real> ph;
+      ph.alive = 1;
+      uint32_t cw = 0, pv = 0, trials = 0;
+      int pmat = 0, pscored = 0, idx = 0;
+      bool fresh = event != kQFly && event != kQWorld;  // direction and energy change
+      bool live = true;                                 // the slot holds a photon
+      bool aim = false;                                 // its path to the image boundary is not known (in a slot: negative)
+      sec.has = 0;
+      uint32_t *const buf = &S.rng.x;
+      if (event == kQRefill) {
+        n_list = 0;
+        if constexpr (DG == 2) ld.flush(td);
+        const uint32_t r = Q.tid;
+        const bool have = r < avail || r - avail < got;
+        const uint32_t h = r < avail ? pool_next + r : base + (r - avail);
+        uint32_t f = kRecDead;
+        if (have) f = rec.flags[h];
+        dest = have || !exhausted ? kQRefill : kQNone;
+        live = (f & 3u) != kRecDead;
+        e = make_uint4(0u, h, 0u, 0u);
+        if (live) {
+          if constexpr (MULTI) {
+            e.w = rec.sim[h];
+            bind(e.w);
+          }
+          ph.pos[0] = rec.px[h];
+          ph.pos[1] = rec.py[h];
+          ph.pos[2] = rec.pz[h];
+          ph.dir[0] = rec.dx[h];
+          ph.dir[1] = rec.dy[h];
+          ph.dir[2] = rec.dz[h];
+          set_energy(s, ph, rec.e[h]);
+          const uint32_t rp = rec.rng_pos[h];
+          S.rng = rec.rng_buf[h];
+          e.x = rp >> 3;
+          idx = (int)(rp & 7u);
+          ph.steps = (int)((f >> 2) & 1u);
+          ph.can_enter = 1;
+          ph.t_exit = R<real>(0);
+          if ((f & 3u) == kRecInImage) {
+            aim = true;
+            dest = kQFly;
+          } else if ((f & 3u) == kRecWorld) {
+            dest = kQWorld;
+          } else {
+            pmat = s.world_mat;
+            dest = kQInteract;
+          }
+        }
+      } else {
+        const Real4<real> a = S.a, b = S.b, c = S.c;
+        cw = real_bits(c.w);
+        ph.pos[0] = a.x;
+        ph.pos[1] = a.y;
+        ph.pos[2] = a.z;
+        ph.dir[0] = b.x;
+        ph.dir[1] = b.y;
+        ph.dir[2] = b.z;
+        ph.e = b.w;
+        ph.t_exit = a.w;
+        ph.mumax = c.x;
+        ph.inv_mumax = c.y;
+        ph.ei.fe = c.z;
+        ph.ei.ie = (int)(cw & 0xffffu);
+        ph.steps = (int)(e.z & kSlSteps);
+        ph.can_enter = (int)((e.z >> kSlExcl) & 1u);
+        sec.has = (int)((e.z >> kSlSec) & 1u);
+        idx = (int)((e.z >> kSlIdx) & 7u);
+        dest = kQFly;
+        aim = event == kQFly && ph.t_exit < R<real>(0);
+      }
+      sec.tid = (int)(slot0 + (uint32_t)k);
+      uint64_t key = args.seed, hid = args.h_begin + e.y;
+      if constexpr (MULTI) {
+        key = sg.sims[e.w].seed;
+        hid = hid - sg.sims[e.w].h_begin;
+      }
+      const uint32_t h0 = (uint32_t)hid, h1 = (uint32_t)(hid >> 32), k0 = (uint32_t)key, k1 = (uint32_t)(key >> 32);
+      if (event == kQInteract) {
+        pmat = (int)(cw >> 16);
+        pscored = (int)((e.z >> kSlImage) & 1u);
+        pv = real_bits(ph.t_exit);
+        EventRng g{buf, ahead[threadIdx.x], k0, k1, 0u, h0, h1, e.x, idx};
+        g.begin();
+        const bool retry = (e.z >> kSlRetry) != 0u;
+        const int kind = retry ? kCompton : select_kind(s, ph, pmat, g);
+        real ed = R<real>(0);
+        bool done = true;
+        real cost = R<real>(1), st2 = R<real>(0), eps = R<real>(1);
+        if (kind == kCompton) {
+          const KleinNishina<real> kn(ph.e);
+          trials = retry ? real_bits(ph.mumax) : 0u;
+          real onecost;
+          int left = kKnTrials;
+#pragma unroll 1
+          do {
+            done = kn.trial(g, eps, onecost, st2);
+            if (!done && ++trials >= (uint32_t)kLoopCap) {
+              atomicAdd(&bc.loop_capped, 1u);
+              done = true;
+            }
+          } while (!done && --left > 0);
+          cost = R<real>(1) - onecost;
+        } else if (kind == kPhoto) {
+          ph.alive = 0;
+          ed = ph.e;
+        } else if (kind == kRayleigh) {
+          cost = rayleigh_cost(s, s.mat_comp[pmat], ph, g, &bc);
+          st2 = rayleigh_sint2(cost);
+        } else {
+          ed = pair_conversion(s, ph, g, &bc, sec);
+        }
+        if (done && (kind == kCompton || kind == kRayleigh)) scatter_dir(ph, g, cost, st2);
+        if (done && kind == kCompton) ed = compton_energy(s, ph, eps);
+        g.end();
+        e.x = g.blk;
+        idx = g.idx;
+        if (done) trials = 0;
+        if (!done) {
+          dest = kQInteract;
+        } else if (pscored) {
+          uint32_t v = pv;
+          bool in = true;
+          if constexpr (DG > 0) in = dose_voxel(s, ph.pos, v);
+          if (in) {
+            list_deposit(S, n_list, t, v, ed, n_dep, n_ent, n_over);
+            if constexpr (DG == 2) {
+              real dd = ed * s.drho_min;
+              dd = dd / s.mat_rho[pmat];
+              ld.deposit(td, v, dd);
+            }
+          }
+          aim = ph.alive;
+          if (!ph.alive) dest = kQRefill;
+        } else {
+          dest = ph.alive ? kQWorld : kQRefill;
+          ph.can_enter = 1;
+        }
+      }
+      if (aim) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
+      if (event == kQWorld || dest == kQFly) {
+        // ---- a flight
+        if (++ph.steps > kStepCap) {
+          atomicAdd(&bc.loop_capped, 1u);
+          dest = kQRefill;
+        } else {
+          TwoWords g;
+          g.draw(buf, e.x, idx, 0u, h0, h1, k0, k1);
+          if (event == kQWorld) {
+            ++n_world;
+            const int r = dose_world_flight(s, ph, g, pmat, pscored);
+            if (r == kRefill) ++n_esc;
+            ph.t_exit = R<real>(-1);
+            dest = r == kInteract ? kQInteract : (r == kFly ? kQFly : kQRefill);
+          } else {
+            ph.in_image = 1;
+            const int r = image_flight(s, ph, g, pmat, pv, pscored, n_wood, n_real);
+            dest = r == kInteract ? kQInteract : (ph.in_image ? kQFly : kQWorld);
+          }
+          g.end(buf, e.x, idx);
+        }
+      }
+      if (dest == kQRefill && sec.has) {
+        take_secondary(s, ph, sec);
+        ph.t_exit = R<real>(-1);
+        dest = ph.in_image ? kQFly : kQWorld;
+        fresh = true;
+      }
+      // ---- the photon back into its slot
+      const bool pend = dest == kQInteract;
+      if (live) {
+        S.a = Real4<real>{ph.pos[0], ph.pos[1], ph.pos[2], pend ? bits_real(real(0), pv) : ph.t_exit};
+        cw = (uint32_t)ph.ei.ie | ((uint32_t)pmat << 16);
+        if (fresh) {
+          S.b = Real4<real>{ph.dir[0], ph.dir[1], ph.dir[2], ph.e};
+          S.c = Real4<real>{trials ? bits_real(real(0), trials) : ph.mumax, ph.inv_mumax, ph.ei.fe,
+                            bits_real(real(0), cw)};
+        } else if (pend) {
+          S.c.w = bits_real(real(0), cw);
+        }
+        e.z = (uint32_t)ph.steps | ((uint32_t)idx << kSlIdx) | ((uint32_t)ph.can_enter << kSlExcl) |
+              ((uint32_t)sec.has << kSlSec) | ((uint32_t)n_list << kSlList);
+        if (pend) e.z |= (pscored ? 1u << kSlImage : 0u) | (trials ? 1u << kSlRetry : 0u);
+      }
+      if constexpr (DG == 2) e.w = (uint32_t)ld.n;
+      S.e = e;
+    }
+    if (event == kQRefill) {
+      if (n <= avail) {
+        pool_next += n;
+      } else {
+        pool_next = base + min(n - avail, got);
+        pool_end = base + got;
+      }
+    }
+    Q.put(dest, k, lane, lt_mask);
+  }
+  // ---- counters -------------------------------------------------------------
+  unsigned long long *cnt = args.counters;
+  warp_count(cnt + GG_CNT_WOODCOCK_STEPS, n_wood);
+  warp_count(cnt + GG_CNT_REAL_INTERACTIONS, n_real);
+  warp_count(cnt + GG_CNT_DEPOSITS, n_dep);
+  warp_count(cnt + GG_CNT_WORLD_STEPS, n_world);
+  warp_count(cnt + GG_CNT_TALLY_ENTRIES, n_ent);
+  warp_count(cnt + GG_CNT_LIST_OVERFLOWS, n_over);
+  warp_count(cnt + GG_CNT_ESCAPED, n_esc);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (bc.loop_capped) atomicAdd(&cnt[GG_CNT_LOOP_CAPPED], (unsigned long long)bc.loop_capped);
+    if (bc.stack_overflow) atomicAdd(&cnt[GG_CNT_STACK_OVERFLOW], (unsigned long long)bc.stack_overflow);
+    if (bc.secondaries) atomicAdd(&cnt[GG_CNT_SECONDARIES], (unsigned long long)bc.secondaries);
+  }
+}
+
+// Transport stage with the track-length estimator (a history scores every voxel
+// it crosses: its list fills and empties many times, so it stays with its
+// thread).  Persistent grid; each lane carries one history at a time
 // and is in one of the states kRefill (needs a history), kFly (next event is
 // a flight) or kInteract (a collision is pending).  Every iteration the block
 // picks ONE phase from counts of its lanes' states - refill when at least
@@ -185,13 +518,10 @@ __global__ void __launch_bounds__(256) k_generate(Scene<real> s, KernelArgs a) {
 // and the order of operations inside each history, hence its result, is
 // unchanged.
 // MINB = resident blocks per SM the register budget is sized for.
-// SPECT selects the head transport and projection scoring instead of the dose tally.
-// DG: dose tally on a grid of its own (1: edep, 2: edep and dose), Scene::dgrid.
-template <typename real, int MINB, bool SPECT, bool MULTI, bool TLE, int DG = 0>
-__global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelArgs args) {
+template <typename real, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_transport_tle(Scene<real> sg, KernelArgs args) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
-  __shared__ BlockCounters bcd;  // counts of the dose list (DG 2), not reported
   __shared__ real sec_store[6 * 256];
   // ---- stage tables in shared memory --------------------------------------
   Scene<real> s = sg;
@@ -217,10 +547,6 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
   }
   const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
   Tally<real> t{args.acc_e, args.acc_e2};
-  const Tally<real> td{args.acc_d, args.acc_d2};
-  if constexpr (DG == 2) {
-    if (threadIdx.x == 0) bcd = BlockCounters{0, 0, 0, 0, 0, 0, 0, 0};
-  }
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
   const uint64_t n_hist = args.h_end - args.h_begin;
@@ -237,7 +563,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
   sec.tid = threadIdx.x;
   sec.has = 0;
   // history lists after the tables: [list][vox | acc][kHistList][blockDim.x]
-  HistList<real> l, ld;  // ld: dose list of the history (DG 2), same voxels as l
+  HistList<real> l;
   {
     const int nt = (int)blockDim.x;
     unsigned char *lists = smem_raw + transport_smem_bytes<real>(sg.n_comp, sg.n_e, sg.n_mat);
@@ -245,12 +571,6 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
     l.acc = reinterpret_cast<real *>(lists + (size_t)kHistList * nt * sizeof(uint32_t)) + threadIdx.x;
     l.stride = nt;
     l.n = 0;
-    ld = l;
-    if constexpr (DG == 2) {
-      lists += hist_list_bytes<real>(1, nt);
-      ld.vox = reinterpret_cast<uint32_t *>(lists) + threadIdx.x;
-      ld.acc = reinterpret_cast<real *>(lists + (size_t)kHistList * nt * sizeof(uint32_t)) + threadIdx.x;
-    }
   }
   Event<real> ev;
   ev.clear();
@@ -259,7 +579,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
   bool in_hist = false;
   int pmat = 0, pscored = 0;
   uint32_t pv = 0;
-  unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0, n_head = 0, n_singles = 0;
+  unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0;
 
   for (;;) {
     // phase chosen per block: all warps run the same code region at the same
@@ -277,17 +597,10 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
 
     if (phase == kRefill) {
       const bool need = state == kRefill;
-      if constexpr (SPECT) {
-        if (need && in_hist) n_singles += score_singles(s, ev, ph.run, g);
-      } else {
-        // per-lane atomics: a warp-aggregated flush (same-voxel entries of the warp summed
-        // first, __match_any_sync + shuffles) issued as many atomic instructions here and
-        // made the transport 28 % slower, so it is not used
-        if (need && in_hist) {
-          hlist_flush(l, t, &bc);
-          if constexpr (DG == 2) hlist_flush(ld, td, &bcd);
-        }
-      }
+      // per-lane atomics: a warp-aggregated flush (same-voxel entries of the warp summed
+      // first, __match_any_sync + shuffles) issued as many atomic instructions here and
+      // made the transport 28 % slower, so it is not used
+      if (need && in_hist) hlist_flush(l, t, &bc);
       if (need) in_hist = false;
       const uint64_t h = warp_pool_claim(pool, m_ref, lane, lt_mask, args.next, args.chunk);
       if (need) {
@@ -297,18 +610,8 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
           const uint32_t f = rec.flags[h];
           const uint32_t rs = f & 3u;
           if (rs != kRecDead) {
-            uint64_t hid = args.h_begin + h;
-            uint64_t key = args.seed;
-            if constexpr (MULTI) {
-              // batched simulations: this history's geometry, majorant, tally and Philox stream
-              const uint32_t k = rec.sim[h];
-              const SimDesc<real> &d = sg.sims[k];
-              bind_geometry(s, d, sg.labels, sg.sim_maj + (size_t)k * sg.n_e);
-              t.acc_e = args.acc_e + d.vox_off;
-              t.acc_e2 = args.acc_e2 ? args.acc_e2 + 2 * d.vox_off : nullptr;
-              key = d.seed;
-              hid = hid - d.h_begin;
-            }
+            const uint64_t hid = args.h_begin + h;
+            const uint64_t key = args.seed;
             ph.pos[0] = rec.px[h];
             ph.pos[1] = rec.py[h];
             ph.pos[2] = rec.pz[h];
@@ -322,10 +625,6 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
             ph.in_head = 0;
             ph.exclude = -1;
             ph.w = s.s_fd_w;  // 1, or the forced direction's cone weight
-            if constexpr (SPECT) {
-              ev.clear();
-              ph.run = s.run_base + (int)((hid - s.run_first) / s.run_len);
-            }
             const uint32_t rp = rec.rng_pos[h];
             const uint4 b = rec.rng_buf[h];
             g.k0 = (uint32_t)key;
@@ -358,10 +657,7 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
       }
     } else if (phase == kInteract) {
       if (state == kInteract) {
-        if constexpr (DG > 0)
-          state = do_interaction_grid<real, DG>(s, ph, g, &bc, pmat, pscored, l, ld, t, td, sec, n_dep, &bcd);
-        else
-          state = do_interaction<real, SPECT, TLE>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev);
+        state = do_interaction<real, false, true>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev);
         if (state == kRefill && sec.has) {
           pop_secondary(s, ph, sec);
           state = kFly;
@@ -369,8 +665,8 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
       }
     } else {
       if (state == kFly) {
-        state = flight<real, SPECT, TLE>(s, ph, g, &bc, pmat, pv, pscored, n_wood, n_real, n_world, n_head,
-                                         TleScore<real>{&l, &t, &n_dep});
+        state = flight<real, true>(s, ph, g, &bc, pmat, pv, pscored, n_wood, n_real, n_world,
+                                   TleScore<real>{&l, &t, &n_dep});
         if (state == kRefill && sec.has) {
           pop_secondary(s, ph, sec);
           state = kFly;
@@ -390,8 +686,6 @@ __global__ void __launch_bounds__(256, MINB) k_transport(Scene<real> sg, KernelA
   warp_add(n_real, GG_CNT_REAL_INTERACTIONS);
   warp_add(n_dep, GG_CNT_DEPOSITS);
   warp_add(n_world, GG_CNT_WORLD_STEPS);
-  warp_add(n_head, GG_CNT_HEAD_STEPS);
-  warp_add(n_singles, GG_CNT_SINGLES);
   __syncthreads();
   if (threadIdx.x == 0) {
     atomicAdd(&cnt[GG_CNT_TALLY_ENTRIES], (unsigned long long)bc.tally_entries);
@@ -448,51 +742,47 @@ cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStrea
   return cudaGetLastError();
 }
 
-template <typename real, int MINB, bool MULTI, bool TLE = false, int DG = 0>
-static cudaError_t launch_transport_v(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem,
-                                      cudaStream_t st) {
+template <typename real, bool MULTI, int DG>
+static cudaError_t launch_pool_v(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st) {
   static unsigned long long configured = 0;
-  if (block <= 0 || block > kBlock) return cudaErrorInvalidValue;
-  cudaError_t e = configure_smem(k_transport<real, MINB, false, MULTI, TLE, DG>, kTransportSmemMax, configured);
+  cudaError_t e = configure_smem(k_transport_pool<real, MULTI, DG>, 227 * 1024, configured);
   if (e != cudaSuccess) return e;
-  smem += hist_list_bytes<real>(DG == 2 ? 2 : 1, block);
+  k_transport_pool<real, MULTI, DG><<<p.grid, p.block, p.smem, st>>>(s, a, p.slots);
+  return cudaGetLastError();
+}
+
+template <typename real, int MINB>
+static cudaError_t launch_tle_v(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem,
+                                cudaStream_t st) {
+  static unsigned long long configured = 0;
+  cudaError_t e = configure_smem(k_transport_tle<real, MINB>, kTransportSmemMax, configured);
+  if (e != cudaSuccess) return e;
+  smem += hist_list_bytes<real>(1, block);
   if (smem > (size_t)kTransportSmemMax) return cudaErrorInvalidValue;
-  k_transport<real, MINB, false, MULTI, TLE, DG><<<grid, block, smem, st>>>(s, a);
+  k_transport_tle<real, MINB><<<grid, block, smem, st>>>(s, a);
   return cudaGetLastError();
 }
 
 template <typename real>
-cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem,
-                             int minb, cudaStream_t st) {
-  // SPECT runs use the two-stage kernels of gg_spect.cu
-  if (s.spect) return cudaErrorInvalidValue;
+cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st) {
+  // SPECT runs use the stage kernels of gg_spect.cu, the track-length estimator launch_transport_tle
+  if (s.spect || s.muen || p.block <= 0 || p.block > PoolShape<real>::kBlock || p.slots < 8 || p.slots > PoolShape<real>::kRing) return cudaErrorInvalidValue;
   if (s.dgrid) {
     // dose grid of its own (single simulations, analog scoring)
-    if (s.muen || s.n_sims > 0) return cudaErrorInvalidValue;
-    if (s.ddose) {
-      if (minb <= 2) return launch_transport_v<real, 2, false, false, 2>(s, a, grid, block, smem, st);
-      if (minb == 3) return launch_transport_v<real, 3, false, false, 2>(s, a, grid, block, smem, st);
-      return launch_transport_v<real, 4, false, false, 2>(s, a, grid, block, smem, st);
-    }
-    if (minb <= 2) return launch_transport_v<real, 2, false, false, 1>(s, a, grid, block, smem, st);
-    if (minb == 3) return launch_transport_v<real, 3, false, false, 1>(s, a, grid, block, smem, st);
-    return launch_transport_v<real, 4, false, false, 1>(s, a, grid, block, smem, st);
-  }
-  if (s.muen) {
-    // track-length estimator (single simulations only)
     if (s.n_sims > 0) return cudaErrorInvalidValue;
-    if (minb <= 2) return launch_transport_v<real, 2, false, true>(s, a, grid, block, smem, st);
-    if (minb == 3) return launch_transport_v<real, 3, false, true>(s, a, grid, block, smem, st);
-    return launch_transport_v<real, 4, false, true>(s, a, grid, block, smem, st);
+    return s.ddose ? launch_pool_v<real, false, 2>(s, a, p, st) : launch_pool_v<real, false, 1>(s, a, p, st);
   }
-  if (s.n_sims > 0) {
-    if (minb <= 2) return launch_transport_v<real, 2, true>(s, a, grid, block, smem, st);
-    if (minb == 3) return launch_transport_v<real, 3, true>(s, a, grid, block, smem, st);
-    return launch_transport_v<real, 4, true>(s, a, grid, block, smem, st);
-  }
-  if (minb <= 2) return launch_transport_v<real, 2, false>(s, a, grid, block, smem, st);
-  if (minb == 3) return launch_transport_v<real, 3, false>(s, a, grid, block, smem, st);
-  return launch_transport_v<real, 4, false>(s, a, grid, block, smem, st);
+  return s.n_sims > 0 ? launch_pool_v<real, true, 0>(s, a, p, st) : launch_pool_v<real, false, 0>(s, a, p, st);
+}
+
+template <typename real>
+cudaError_t launch_transport_tle(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem, int minb,
+                                 cudaStream_t st) {
+  // single simulations on the image grid only
+  if (s.spect || !s.muen || s.dgrid || s.n_sims > 0 || block <= 0 || block > kBlock) return cudaErrorInvalidValue;
+  if (minb <= 2) return launch_tle_v<real, 2>(s, a, grid, block, smem, st);
+  if (minb == 3) return launch_tle_v<real, 3>(s, a, grid, block, smem, st);
+  return launch_tle_v<real, 4>(s, a, grid, block, smem, st);
 }
 
 cudaError_t launch_flush(unsigned long long *acc_e, unsigned long long *acc_e2, double *edep, double *edep2,
@@ -502,22 +792,71 @@ cudaError_t launch_flush(unsigned long long *acc_e, unsigned long long *acc_e2, 
 }
 
 template <typename real>
-cudaError_t occupancy_blocks(int block, size_t smem, int minb, int *bps) {
+cudaError_t tle_occupancy(int block, size_t smem, int minb, int *bps) {
   smem += hist_list_bytes<real>(1, block);
-  if (minb <= 2) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport<real, 2, false, false, false>, block, smem);
-  if (minb == 3) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport<real, 3, false, false, false>, block, smem);
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport<real, 4, false, false, false>, block, smem);
+  if (minb <= 2) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 2>, block, smem);
+  if (minb == 3) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 3>, block, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 4>, block, smem);
+}
+
+// Launch shape of a pooled run: one block per SM.  More slots per thread keep
+// the rounds full, so they take all shared memory beside the tables, but no
+// more than the run has histories for.  block, blocks: most threads per block
+// and resident blocks per SM (of 256 threads) of the options, 0 for the
+// kernel's register budget; dose_list: the second list of a dose grid.
+template <typename real>
+cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, bool dose_list,
+                      PoolPlan *p) {
+  int n_sm = 0, optin = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e != cudaSuccess) return e;
+  using Shape = PoolShape<real>;
+  constexpr int kGang = 32 * Shape::kGang;
+  const uint64_t per_sm = (n_hist + n_sm - 1) / n_sm;
+  int threads = Shape::kBlock;
+  if (blocks > 0) threads = std::min(threads, 256 * blocks);
+  if (block > 0) threads = std::min(threads, block);
+  threads = (int)std::min<uint64_t>(threads, (per_sm + 31) / 32 * 32);
+  const size_t slot = sizeof(PhotonSlot<real>), fixed = pool_static<real>() + table_bytes;
+  const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
+  while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
+  const int gangs = (threads + kGang - 1) / kGang;
+  const int most = std::min(room / gangs, Shape::kRing - 32) / 8 * 8;
+  if (most < 8) return cudaErrorInvalidValue;
+  const uint64_t share = std::max<uint64_t>((per_sm + gangs - 1) / gangs, 32);
+  p->grid = n_sm;
+  p->block = threads;
+  p->gangs = gangs;
+  p->slots = (int)std::min<uint64_t>(most, (share + 7) / 8 * 8);
+  p->smem = slot * p->slots * gangs + table_bytes;
+  p->scratch = (size_t)p->grid * gangs * p->slots *
+               (6 * sizeof(real) + (dose_list ? kHistList * (sizeof(real) + sizeof(uint32_t)) : 0));
+  return cudaSuccess;
+}
+
+// Histories a gang claims at a time: an even share of a small run, else the
+// per-warp chunk of the options for each of its warps.
+int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist) {
+  const uint64_t gangs = (uint64_t)p.grid * p.gangs, share = (n_hist + gangs - 1) / gangs;
+  const uint64_t warps = (uint64_t)std::max(p.block / 32 / p.gangs, 1);
+  return (int)std::max<uint64_t>(32, std::min<uint64_t>(share, warps * std::min(chunk, 1 << 20)));
 }
 
 template size_t record_bytes<float>(size_t);
 template size_t record_bytes<double>(size_t);
 template cudaError_t launch_generate<float>(const Scene<float> &, const KernelArgs &, cudaStream_t);
 template cudaError_t launch_generate<double>(const Scene<double> &, const KernelArgs &, cudaStream_t);
-template cudaError_t launch_transport<float>(const Scene<float> &, const KernelArgs &, int, int, size_t, int,
-                                             cudaStream_t);
-template cudaError_t launch_transport<double>(const Scene<double> &, const KernelArgs &, int, int, size_t, int,
+template cudaError_t launch_transport<float>(const Scene<float> &, const KernelArgs &, const PoolPlan &, cudaStream_t);
+template cudaError_t launch_transport<double>(const Scene<double> &, const KernelArgs &, const PoolPlan &,
                                               cudaStream_t);
-template cudaError_t occupancy_blocks<float>(int, size_t, int, int *);
-template cudaError_t occupancy_blocks<double>(int, size_t, int, int *);
+template cudaError_t launch_transport_tle<float>(const Scene<float> &, const KernelArgs &, int, int, size_t, int,
+                                                 cudaStream_t);
+template cudaError_t launch_transport_tle<double>(const Scene<double> &, const KernelArgs &, int, int, size_t, int,
+                                                  cudaStream_t);
+template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, bool, PoolPlan *);
+template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, bool, PoolPlan *);
+template cudaError_t tle_occupancy<float>(int, size_t, int, int *);
+template cudaError_t tle_occupancy<double>(int, size_t, int, int *);
 
 }  // namespace gg

@@ -166,7 +166,6 @@ __device__ __forceinline__ int wf_process(int code, int slot, uint64_t h, const 
                                           const Records<real> &rec, const Tally<real> &tally, uint64_t key,
                                           uint64_t h_begin, uint64_t n_hist, BlockCounters *bc, unsigned int &n_wood,
                                           unsigned int &n_real, unsigned int &n_dep, unsigned int &n_world) {
-  unsigned int n_head = 0;
   if (code == kWFly) {
     // ---- one flight step (Woodcock in the image, or the world step) ----------
     Photon<real> ph;
@@ -176,7 +175,7 @@ __device__ __forceinline__ int wf_process(int code, int slot, uint64_t h, const 
     int pmat = 0, pscored = 0;
     uint32_t pv = 0;
     int nc;
-    const int r = flight<real, false, false>(s, ph, g, bc, pmat, pv, pscored, n_wood, n_real, n_world, n_head);
+    const int r = flight<real>(s, ph, g, bc, pmat, pv, pscored, n_wood, n_real, n_world);
     const uint32_t f = S.flags[slot];
     if (r == kInteract) {
       const int kind = select_kind(s, ph, pmat, g);
