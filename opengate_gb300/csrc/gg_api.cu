@@ -99,6 +99,8 @@ struct gg_ctx {
   int run_base = 0;
   unsigned long long *d_proj = nullptr;
   size_t n_proj = 0;
+  double *d_fetch = nullptr;  // FP64 pixels of a projection being fetched
+  size_t fetch_cap = 0;
 
   // tally
   unsigned long long *d_acc_e = nullptr, *d_acc_e2 = nullptr;
@@ -273,6 +275,8 @@ struct gg_ctx {
     rec_cap = 0;
     dfree(d_slot);
     slot_bytes = 0;
+    dfree(d_fetch);
+    fetch_cap = 0;
     for (auto e : ev) cudaEventDestroy(e);
     ev.clear();
     if (stream) cudaStreamDestroy(stream);
@@ -709,6 +713,21 @@ static int tally_alloc(gg_ctx *c) {
     if ((st = c->cuda(cudaMalloc(&c->d_dose2, n * 8), "cudaMalloc dose2"))) return st;
   }
   return GG_OK;
+}
+
+// A projection tally of n pixels as FP64 into the caller's buffer, through a
+// device buffer that the context keeps.
+static int fetch_projection(gg_ctx *c, int kind, const unsigned long long *src, double *out, size_t n) {
+  int st;
+  if (n > c->fetch_cap) {
+    dfree(c->d_fetch);
+    c->fetch_cap = 0;
+    if ((st = c->cuda(cudaMalloc(&c->d_fetch, n * sizeof(double)), "cudaMalloc projection"))) return st;
+    c->fetch_cap = n;
+  }
+  if ((st = c->cuda(gg::launch_projection_f64(kind, src, c->d_fetch, n, c->n_sm, c->stream), "projection to FP64")))
+    return st;
+  return c->d2h(out, c->d_fetch, n * sizeof(double), "download projection");
 }
 
 extern "C" {
@@ -2035,22 +2054,9 @@ int gg_get_arf_projection(gg_ctx *c, double *counts, double *squared, size_t n) 
   if ((!c->arf_on && !c->ff_on) || !c->d_arf_proj)
     return c->fail(GG_ERR_STATE, "gg_get_arf_projection: neither the ARF stage nor free flight is on");
   if (n != c->arf_proj_n) return c->fail(GG_ERR_ARG, "gg_get_arf_projection: buffer has %zu values, need %zu", n, c->arf_proj_n);
-  std::vector<unsigned long long> tmp(n);
-  int st = c->d2h(tmp.data(), c->d_arf_proj, n * 8, "download ARF projection");
-  if (st) return st;
-  for (size_t i = 0; i < n; ++i) counts[i] = (double)tmp[i] * 2.3283064365386963e-10;
-  if (squared) {
-    std::vector<unsigned long long> t2(2 * n);
-    if ((st = c->d2h(t2.data(), c->d_arf_proj2, n * 16, "download ARF projection squared"))) return st;
-    for (size_t i = 0; i < n; ++i) {
-      double lo = (double)t2[2 * i];
-      lo = lo * 5.421010862427522e-20;
-      double hi = (double)t2[2 * i + 1];
-      hi = hi * 2.3283064365386963e-10;
-      squared[i] = hi + lo;
-    }
-  }
-  return GG_OK;
+  int st = fetch_projection(c, gg::kProjWeights, c->d_arf_proj, counts, n);
+  if (!st && squared) st = fetch_projection(c, gg::kProjSquares, c->d_arf_proj2, squared, n);
+  return st;
 }
 
 int gg_batch_setup(gg_ctx *c, const gg_sim_desc *sims, int32_t n) {
@@ -2306,11 +2312,7 @@ int gg_get_projection(gg_ctx *c, double *out, size_t n) {
   cudaSetDevice(c->device);
   if (!c->have_spect) return c->fail(GG_ERR_STATE, "gg_get_projection: no SPECT heads");
   if (n != c->n_proj) return c->fail(GG_ERR_ARG, "gg_get_projection: buffer has %zu values, need %zu", n, c->n_proj);
-  std::vector<unsigned long long> tmp(n);
-  int st = c->d2h(tmp.data(), c->d_proj, n * 8, "download projections");
-  if (st) return st;
-  for (size_t i = 0; i < n; ++i) out[i] = (double)tmp[i];
-  return GG_OK;
+  return fetch_projection(c, gg::kProjCounts, c->d_proj, out, n);
 }
 
 }  // extern "C"

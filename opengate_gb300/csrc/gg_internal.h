@@ -191,6 +191,10 @@ size_t split_bytes(size_t cap);
 template <typename real>
 cudaError_t launch_spect_walk(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
                               int n_sm, cudaStream_t st);
+// A projection tally (counts; fixed-point weights; their squares, two words per pixel) as FP64.
+enum : int { kProjCounts = 0, kProjWeights = 1, kProjSquares = 2 };
+cudaError_t launch_projection_f64(int kind, const unsigned long long *src, double *dst, size_t n, int n_sm,
+                                  cudaStream_t st);
 template <typename real>
 size_t record_bytes(size_t cap);
 template <typename real>
