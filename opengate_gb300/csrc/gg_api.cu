@@ -1093,15 +1093,16 @@ static constexpr size_t kSsQueueMax = (size_t)1 << 26;
 // SPECT transport of one batch: phantom stage on the primary records, head
 // stage on the head queue, then phantom / head passes on the photons that
 // flew back into the image until the return queue stays empty.
-static int spect_stages(gg_ctx *c, gg::KernelArgs a, size_t smem, int minb) {
-  int bps[2] = {0, 0};
-  for (int stage = 0; stage < 2; ++stage) {
-    cudaError_t e = c->precision == GG_PREC_F64
-                        ? gg::spect_stage_occupancy<double>(stage, c->block, smem, minb, &bps[stage])
-                        : gg::spect_stage_occupancy<float>(stage, c->block, smem, minb, &bps[stage]);
+static int spect_stages(gg_ctx *c, gg::KernelArgs a, const gg::PoolPlan &plan, size_t smem, int minb) {
+  int bps = 0;  // of the head stage
+  {
+    cudaError_t e = c->precision == GG_PREC_F64 ? gg::spect_head_occupancy<double>(c->block, smem, minb, &bps)
+                                                : gg::spect_head_occupancy<float>(c->block, smem, minb, &bps);
     if (e != cudaSuccess) return c->cuda(e, "occupancy");
-    if (bps[stage] < 1) bps[stage] = 1;
+    if (bps < 1) bps = 1;
   }
+  gg::KernelArgs ha = a;  // the head stage's warps claim the chunk of the options
+  ha.chunk = std::max(c->chunk, 32);
   unsigned long long *nh = c->d_qn, *nr = c->d_qn + 1, *nf = c->d_qn + 2;
   auto stage_run = [&](int stage, void *in_q, const unsigned long long *in_n, void *out_q,
                        unsigned long long *out_n) -> int {
@@ -1109,13 +1110,16 @@ static int spect_stages(gg_ctx *c, gg::KernelArgs a, size_t smem, int minb) {
     int st;
     if ((st = c->cuda(cudaMemsetAsync(out_n, 0, sizeof(unsigned long long), c->stream), "memset"))) return st;
     if ((st = c->cuda(cudaMemsetAsync(c->d_next, 0, 8, c->stream), "memset"))) return st;
-    int grid = c->n_sm * bps[stage];
     if ((st = stage_event(c, stage, true))) return st;
-    cudaError_t e = c->precision == GG_PREC_F64
-                        ? gg::launch_spect_stage<double>(stage, c->scene<double>(), a, q, grid, c->block, smem, minb,
-                                                         c->stream)
-                        : gg::launch_spect_stage<float>(stage, c->scene<float>(), a, q, grid, c->block, smem, minb,
-                                                        c->stream);
+    const int grid = c->n_sm * bps;
+    const bool f64 = c->precision == GG_PREC_F64;
+    cudaError_t e;
+    if (stage == 0)
+      e = f64 ? gg::launch_spect_phantom<double>(c->scene<double>(), a, q, plan, c->n_sm, c->stream)
+              : gg::launch_spect_phantom<float>(c->scene<float>(), a, q, plan, c->n_sm, c->stream);
+    else
+      e = f64 ? gg::launch_spect_head<double>(c->scene<double>(), ha, q, grid, c->block, smem, minb, c->stream)
+              : gg::launch_spect_head<float>(c->scene<float>(), ha, q, grid, c->block, smem, minb, c->stream);
     if ((st = c->cuda(e, "SPECT stage launch"))) return st;
     return stage_event(c, stage, false);
   };
@@ -1344,12 +1348,17 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
                                                 : gg::tle_occupancy<float>(c->block, smem, minb, &bps);
     if (e != cudaSuccess) return c->cuda(e, "occupancy");
     tle_grid = c->n_sm * std::max(bps, 1);
-  } else if (!c->have_spect && !wave) {
-    const bool two = c->dgrid_on && c->ddose && !c->have_batch;
+  } else if (!wave) {
+    const bool f64 = c->precision == GG_PREC_F64, sp = c->have_spect;
+    const bool two = c->dgrid_on && c->ddose && !c->have_batch && !sp;
     const int pool_threads = c->block == gg::kBlock ? 0 : c->block;  // (the default: the kernel's own block size)
-    cudaError_t e = c->precision == GG_PREC_F64
-                        ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap, two, &plan)
-                        : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap, two, &plan);
+    cudaError_t e =
+        f64 ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
+                                    sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(),
+                                    gg::slot_scratch_bytes<double>(two), &plan)
+            : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
+                                   sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(),
+                                   gg::slot_scratch_bytes<float>(two), &plan);
     if (e != cudaSuccess) return c->cuda(e, "transport launch shape");
     if (plan.scratch > c->slot_bytes) {
       dfree(c->d_slot);
@@ -1402,7 +1411,8 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
   a.acc_d2 = dg && c->ddose && c->squared ? c->d_acc_d2 : nullptr;
   a.counters = c->d_counters;
   a.status = c->d_status;
-  a.chunk = plan.grid ? gg::pool_chunk(plan, c->chunk, cap) : c->chunk;
+  // (a warp that claims for its lanes needs one history each)
+  a.chunk = plan.grid ? gg::pool_chunk(plan, c->chunk, cap) : std::max(c->chunk, 32);
   a.slot_scratch = c->d_slot;
   a.records = c->d_records;
   a.rec_cap = c->rec_cap;
@@ -1425,7 +1435,7 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     if ((st = c->cuda(e, "generate launch"))) return st;
     if (!capturing && (st = c->cuda(cudaEventRecord(c->ev[3 * b + 1], c->stream), "event"))) return st;
     if (c->have_spect) {
-      if ((st = spect_stages(c, a, smem, minb))) return st;
+      if ((st = spect_stages(c, a, plan, smem, minb))) return st;
       c->run_stage_launches += c->last_stage_launches;
     } else if (wave) {
       e = c->precision == GG_PREC_F64

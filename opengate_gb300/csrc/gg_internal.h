@@ -166,39 +166,6 @@ template <typename real>
 __host__ __device__ constexpr size_t hist_list_bytes(int lists, int threads = kBlock) {
   return (size_t)lists * kHistList * (size_t)threads * (sizeof(uint32_t) + sizeof(real));
 }
-// Rows of p.n samples appended to rows[*total ...] (capacity rows); *total advances on the device.
-template <typename real>
-cudaError_t launch_arf_dataset(const Scene<real> &s, const ArfArgs &p, float4 *rows, uint64_t capacity,
-                               unsigned long long *total, cudaStream_t st);
-template <typename real>
-size_t queue_bytes(size_t cap);
-// stage 0: phantom stage, 1: head stage
-template <typename real>
-cudaError_t launch_spect_stage(int stage, const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid,
-                               int block, size_t smem, int minb, cudaStream_t st);
-template <typename real>
-cudaError_t spect_stage_occupancy(int stage, int block, size_t smem, int minb, int *blocks_per_sm);
-// Copies of scatter splitting (gg_spect.cu): the split requests of q.split_q
-// into the walk queue (q.out_q / q.out_n); does nothing when the requests
-// overflowed the buffer.
-template <typename real>
-cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
-                               int n_sm, cudaStream_t st);
-template <typename real>
-size_t split_bytes(size_t cap);
-// Free flights of the copies the split kernel queued (q.in_q / q.in_n) into
-// the head queue (q.out_q / q.out_n).
-template <typename real>
-cudaError_t launch_spect_walk(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
-                              int n_sm, cudaStream_t st);
-// A projection tally (counts; fixed-point weights; their squares, two words per pixel) as FP64.
-enum : int { kProjCounts = 0, kProjWeights = 1, kProjSquares = 2 };
-cudaError_t launch_projection_f64(int kind, const unsigned long long *src, double *dst, size_t n, int n_sm,
-                                  cudaStream_t st);
-template <typename real>
-size_t record_bytes(size_t cap);
-template <typename real>
-cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStream_t st);
 // Launch shape of a pooled transport kernel (gg_pool.cuh).
 struct PoolPlan {
   int grid, block, gangs, slots;  // blocks, threads and gangs per block, photon slots per gang
@@ -227,9 +194,52 @@ __host__ __device__ constexpr int pool_static() {
   return 1024 + 16 * P::kBlock + (P::kBlock / (32 * P::kGang)) * (8 * P::kRing + 64);
 }
 template <typename real>
-cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, bool dose_list,
-                      PoolPlan *p);
+cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
+                      size_t scratch_bytes, PoolPlan *p);
 int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist);
+// Shared memory of a dose slot; its global scratch (two: the second list of a dose grid).
+template <typename real>
+size_t dose_slot_bytes();
+template <typename real>
+size_t slot_scratch_bytes(bool two);
+// Rows of p.n samples appended to rows[*total ...] (capacity rows); *total advances on the device.
+template <typename real>
+cudaError_t launch_arf_dataset(const Scene<real> &s, const ArfArgs &p, float4 *rows, uint64_t capacity,
+                               unsigned long long *total, cudaStream_t st);
+template <typename real>
+size_t queue_bytes(size_t cap);
+// Phantom and head stages of the SPECT wavefront (gg_spect.cu)
+template <typename real>
+cudaError_t launch_spect_phantom(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, const PoolPlan &p,
+                                 int n_sm, cudaStream_t st);
+template <typename real>
+size_t phantom_slot_bytes();
+template <typename real>
+cudaError_t launch_spect_head(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid, int block,
+                              size_t smem, int minb, cudaStream_t st);
+template <typename real>
+cudaError_t spect_head_occupancy(int block, size_t smem, int minb, int *blocks_per_sm);
+// Copies of scatter splitting (gg_spect.cu): the split requests of q.split_q
+// into the walk queue (q.out_q / q.out_n); does nothing when the requests
+// overflowed the buffer.
+template <typename real>
+cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
+                               int n_sm, cudaStream_t st);
+template <typename real>
+size_t split_bytes(size_t cap);
+// Free flights of the copies the split kernel queued (q.in_q / q.in_n) into
+// the head queue (q.out_q / q.out_n).
+template <typename real>
+cudaError_t launch_spect_walk(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
+                              int n_sm, cudaStream_t st);
+// A projection tally (counts; fixed-point weights; their squares, two words per pixel) as FP64.
+enum : int { kProjCounts = 0, kProjWeights = 1, kProjSquares = 2 };
+cudaError_t launch_projection_f64(int kind, const unsigned long long *src, double *dst, size_t n, int n_sm,
+                                  cudaStream_t st);
+template <typename real>
+size_t record_bytes(size_t cap);
+template <typename real>
+cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStream_t st);
 template <typename real>
 cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st);
 // track-length estimator; minb selects the kernel variant compiled for that many resident blocks per SM

@@ -117,30 +117,98 @@ constexpr int kSlIdx = 20, kSlExcl = 23, kSlImage = 25, kSlSec = 26, kSlList = 2
 static_assert(kStepCap < (1 << 20), "the step count has 20 bits in the slot's meta word");
 static_assert(kHistList < 16, "the list length has 4 bits in the slot's meta word");
 
-// A photon slot in shared memory.  a: position, path to the image boundary (a
-// pending interaction: its voxel); b: direction, energy; c: majorant (Compton
-// sampling not finished: rejected trials), its inverse, energy-grid fraction,
-// energy index | material << 16; rng: the Philox block being drawn from; e:
-// next block, record of the history, meta, a word of the kernel's own; vox,
-// acc: the history's voxel list.  The stride is an odd number of 16-byte
+// A photon slot in shared memory.  a: position, path to the image boundary
+// (negative: not known; a pending interaction: its voxel); b: direction,
+// energy; c: majorant (Compton sampling not finished: rejected trials), its
+// inverse, energy-grid fraction, energy index | material << 16; rng: the Philox
+// block being drawn from; e: next block, history (record), meta, a word of the
+// kernel's own; X: more of its own.  The stride is an odd number of 16-byte
 // words, so slots spread over the banks.
-template <typename real>
+template <typename real, typename X>
 struct PhotonSlot {
   Real4<real> a, b, c;
   uint4 rng, e;
-  uint32_t vox[kHistList];
-  alignas(16) real acc[kHistList];
+  X x;
 };
-template <>
-struct PhotonSlot<double> {
-  Real4<double> a, b, c;
-  uint4 rng, e;
-  uint32_t vox[kHistList];
-  alignas(16) double acc[kHistList];
-  uint4 pad;
+
+// A slot's photon into registers.
+template <typename real, typename Slot>
+__device__ __forceinline__ void slot_load(const Slot &S, const uint4 &e, Photon<real> &ph, uint32_t &cw, int &idx) {
+  const Real4<real> a = S.a, b = S.b, c = S.c;
+  cw = real_bits(c.w);
+  ph.pos[0] = a.x;
+  ph.pos[1] = a.y;
+  ph.pos[2] = a.z;
+  ph.dir[0] = b.x;
+  ph.dir[1] = b.y;
+  ph.dir[2] = b.z;
+  ph.e = b.w;
+  ph.t_exit = a.w;
+  ph.mumax = c.x;
+  ph.inv_mumax = c.y;
+  ph.ei.fe = c.z;
+  ph.ei.ie = (int)(cw & 0xffffu);
+  ph.steps = (int)(e.z & kSlSteps);
+  idx = (int)((e.z >> kSlIdx) & 7u);
+}
+
+// ... and back: pend: an interaction in pmat (voxel pv) is pending; fresh:
+// direction and energy changed; trials: of a Compton sampling not finished.
+template <typename real, typename Slot>
+__device__ __forceinline__ void slot_store(Slot &S, const Photon<real> &ph, bool pend, bool fresh, int pmat,
+                                           uint32_t pv, uint32_t trials) {
+  S.a = Real4<real>{ph.pos[0], ph.pos[1], ph.pos[2], pend ? bits_real(real(0), pv) : ph.t_exit};
+  const uint32_t cw = (uint32_t)ph.ei.ie | ((uint32_t)pmat << 16);
+  if (fresh) {
+    S.b = Real4<real>{ph.dir[0], ph.dir[1], ph.dir[2], ph.e};
+    S.c = Real4<real>{trials ? bits_real(real(0), trials) : ph.mumax, ph.inv_mumax, ph.ei.fe,
+                      bits_real(real(0), cw)};
+  } else if (pend) {
+    S.c.w = bits_real(real(0), cw);
+  }
+}
+
+// Items (records, queue entries) claimed from the launch's work counter and not
+// yet handed out; the same in every thread of a gang.
+struct ItemClaims {
+  uint32_t next, end, avail, base, got;
+  bool exhausted;
+
+  __device__ __forceinline__ void init() {
+    next = end = 0u;
+    exhausted = false;
+  }
+  // the next n items, one per thread in order (coalesced loads), claiming `chunk` more when short
+  template <typename Queues>
+  __device__ __forceinline__ void take(const Queues &q, unsigned n, unsigned long long *counter, int chunk,
+                                       uint32_t n_items, unsigned long long *s_claim) {
+    avail = end - next;
+    base = got = 0u;
+    if (avail < n && !exhausted) {
+      if (q.tid == 0) *s_claim = atomicAdd(counter, (unsigned long long)chunk);
+      q.sync();
+      const unsigned long long c = *s_claim;
+      if (c < n_items) {
+        base = (uint32_t)c;
+        got = min((uint32_t)chunk, n_items - base);
+      }
+      exhausted = c + (unsigned long long)chunk >= n_items;
+    }
+  }
+  // thread r's item; false: none is left now
+  __device__ __forceinline__ bool item(uint32_t r, uint32_t &h) const {
+    h = r < avail ? next + r : base + (r - avail);
+    return r < avail || r - avail < got;
+  }
+  __device__ __forceinline__ void advance(unsigned n) {
+    if (n <= avail) {
+      next += n;
+    } else {
+      next = base + min(n - avail, got);
+      end = base + got;
+    }
+  }
 };
-static_assert(sizeof(PhotonSlot<float>) % 32 == 16 && sizeof(PhotonSlot<double>) % 32 == 16, "odd 16-byte stride");
-static_assert(kHistList == 8, "list_deposit reads the voxels as two 16-byte words");
 
 // The stream of one event: the slot's block (words idx .. 3 left) and the one
 // after it, made when the event begins while the warp is converged, so the
@@ -209,11 +277,74 @@ struct TwoWords {
   }
 };
 
+// Compton trials of one interaction event; a photon that is rejected as often
+// waits for the next event with the photons it meets there, instead of keeping
+// its warp in the loop (a third of the trials fail; the worst of 32 lanes takes
+// five or six).
+constexpr int kKnTrials = 2;
+
+// The interaction of a photon in material pmat (interact(): select_kind, then
+// the process).  False: its Compton sampling is not finished, `trials` rejected
+// so far; retry: it is such a photon.  ed: energy deposited locally.
+template <typename real>
+__device__ __forceinline__ bool pool_interact(const Scene<real> &s, Photon<real> &ph, EventRng &g, BlockCounters *bc,
+                                              Secondary<real> &sec, int pmat, bool retry, uint32_t &trials, int &kind,
+                                              real &ed) {
+  kind = retry ? kCompton : select_kind(s, ph, pmat, g);
+  ed = R<real>(0);
+  bool done = true;
+  real cost = R<real>(1), st2 = R<real>(0), eps = R<real>(1);
+  if (kind == kCompton) {
+    const KleinNishina<real> kn(ph.e);
+    trials = retry ? real_bits(ph.mumax) : 0u;
+    real onecost;
+    int left = kKnTrials;
+#pragma unroll 1
+    do {
+      done = kn.trial(g, eps, onecost, st2);
+      if (!done && ++trials >= (uint32_t)kLoopCap) {
+        atomicAdd(&bc->loop_capped, 1u);
+        done = true;
+      }
+    } while (!done && --left > 0);
+    cost = R<real>(1) - onecost;
+  } else if (kind == kPhoto) {
+    ph.alive = 0;
+    ed = ph.e;
+  } else if (kind == kRayleigh) {
+    cost = rayleigh_cost(s, s.mat_comp[pmat], ph, g, bc);
+    st2 = rayleigh_sint2(cost);
+  } else {
+    ed = pair_conversion(s, ph, g, bc, sec);
+  }
+  if (done && (kind == kCompton || kind == kRayleigh)) scatter_dir(ph, g, cost, st2);
+  if (done && kind == kCompton) ed = compton_energy(s, ph, eps);
+  if (done) trials = 0u;
+  return done;
+}
+
+// The dose kernel's part of a slot: the history's voxel list.
+template <typename real>
+struct VoxelList {
+  uint32_t vox[kHistList];
+  alignas(16) real acc[kHistList];
+};
+template <>
+struct VoxelList<double> {
+  uint32_t vox[kHistList];
+  alignas(16) double acc[kHistList];
+  uint4 pad;
+};
+template <typename real>
+using DoseSlot = PhotonSlot<real, VoxelList<real>>;
+static_assert(sizeof(DoseSlot<float>) % 32 == 16 && sizeof(DoseSlot<double>) % 32 == 16, "odd 16-byte stride");
+static_assert(kHistList == 8, "list_deposit reads the voxels as two 16-byte words");
+
 // A history's voxel list in its slot (the entries of HistList, in their order).
 // deposit(): all voxels are compared at once - a loop over the entries makes
 // the warp wait for its longest list.
 template <typename real>
-__device__ __forceinline__ void list_deposit(PhotonSlot<real> &S, int &n, const Tally<real> &t, uint32_t v, real e,
+__device__ __forceinline__ void list_deposit(VoxelList<real> &S, int &n, const Tally<real> &t, uint32_t v, real e,
                                              unsigned int &n_dep, unsigned int &n_entries, unsigned int &n_over) {
   if (!(e > R<real>(0))) return;
   ++n_dep;
@@ -244,7 +375,7 @@ __device__ __forceinline__ void list_deposit(PhotonSlot<real> &S, int &n, const 
 // about 1.5 per history, but the longest of 32 lists has 4 or 5.  ids: 32 *
 // kHistList numbers of the warp's own.  tally_of(slot): the slot's tally.
 template <typename real, typename TallyOf>
-__device__ __forceinline__ void lists_flush(const PhotonSlot<real> *slots, int slot, int n, uint16_t *ids, unsigned lane,
+__device__ __forceinline__ void lists_flush(const DoseSlot<real> *slots, int slot, int n, uint16_t *ids, unsigned lane,
                                             TallyOf &&tally_of, unsigned int &n_entries) {
   unsigned end = (unsigned)n;
 #pragma unroll
@@ -261,8 +392,8 @@ __device__ __forceinline__ void lists_flush(const PhotonSlot<real> *slots, int s
 #pragma unroll 1
   for (unsigned i = lane; i < total; i += 32u) {
     const unsigned id = ids[i];
-    const PhotonSlot<real> &S = slots[id / kHistList];
-    tally_entry(tally_of(S), S.vox[id % kHistList], S.acc[id % kHistList]);
+    const DoseSlot<real> &S = slots[id / kHistList];
+    tally_entry(tally_of(S), S.x.vox[id % kHistList], S.x.acc[id % kHistList]);
   }
   n_entries += (unsigned)n;
   __syncwarp();

@@ -149,7 +149,10 @@ __device__ __forceinline__ uint64_t rng_history(const Rng &g) { return ((uint64_
 
 template <typename real>
 __device__ __forceinline__ int run_of(const Scene<real> &s, uint64_t hid) {
-  return s.run_base + (int)((hid - s.run_first) / s.run_len);
+  const uint64_t d = hid - s.run_first;
+  // (a 64-bit division is some hundred instructions)
+  const uint64_t r = (d | s.run_len) >> 32 ? d / s.run_len : (uint64_t)((uint32_t)d / (uint32_t)s.run_len);
+  return s.run_base + (int)r;
 }
 
 // Writes the lane's photon (and event) to slot k of the output queue; the

@@ -26,69 +26,14 @@
 #include "gg_device.cuh"
 #include "gg_internal.h"
 #include "gg_physics.cuh"
+#include "gg_pool.cuh"
 #include "gg_queue.cuh"
 #include "gg_spect.cuh"
 
 namespace gg {
 
 // Free-flight modes of the stages (Scene::ff).
-constexpr int kFfOff = 0, kFfPrimary = 1, kFfScatter = 2;
-
-// Phantom-stage flight: Woodcock step in the image (followed, when it leaves
-// the image box, by the world step) or one world step; a photon whose world
-// step ends at a head-box entry leaves the stage (kPush).  Primary free
-// flight (FFM 1): one free flight to a head instead.  Scatter splitting
-// (FFM 2): analog flights, and an analog photon that reaches a head is killed
-// there (the heads are its kill volumes; only its split copies are detected).
-template <typename real, int FFM>
-__device__ __forceinline__ int phantom_flight(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc,
-                                              int &pmat, uint32_t &pv, int &pscored, unsigned int &n_wood,
-                                              unsigned int &n_real, unsigned int &n_world) {
-  if (++ph.steps > kStepCap) {
-    atomicAdd(&bc->loop_capped, 1u);
-    ph.alive = 0;
-    return kRefill;
-  }
-  if constexpr (FFM == kFfPrimary) {  // free flight to a head: no interaction outside the heads
-    // the checks here (cutoffs, angle, the head the line enters); the optical
-    // depth of the photons that pass is walked by k_spect_walk, with full warps
-    ++n_world;
-    real tb;
-    if (ff_target(s, ph, s.ss_cos, tb)) return kPush;
-    atomicAdd(&bc->escaped, 1u);
-    return kRefill;
-  }
-  if (ph.in_image) {
-    const int r = image_flight(s, ph, g, pmat, pv, pscored, n_wood, n_real);
-    if (r != kFly || ph.in_image) return r;
-    // left the image box: the world step follows in the same iteration (same
-    // flight count and draws as a separate phase)
-    if (++ph.steps > kStepCap) {
-      atomicAdd(&bc->loop_capped, 1u);
-      ph.alive = 0;
-      return kRefill;
-    }
-  }
-  ++n_world;
-  if (spect_world_flight(s, ph, g)) {
-    pmat = s.world_mat;
-    pscored = 0;
-    return kInteract;
-  }
-  if (!ph.alive) {
-    atomicAdd(&bc->escaped, 1u);
-    return kRefill;
-  }
-  if constexpr (FFM == kFfScatter) {
-    if (ph.in_head) {
-      ph.alive = 0;
-      atomicAdd(&bc->escaped, 1u);
-      return kRefill;
-    }
-    return kFly;
-  }
-  return ph.in_head ? kPush : kFly;
-}
+constexpr int kFfPrimary = 1, kFfScatter = 2;
 
 // Head-stage flight: one step in a head, or one world step; a photon whose
 // world step ends at the image-box entry leaves the stage (kPush).
@@ -391,220 +336,367 @@ __global__ void __launch_bounds__(256) k_spect_walk(Scene<real> sg, KernelArgs a
   stage_counters(args.counters, bc, lane, 0u, 0u, 0u, 0u, 0u);
 }
 
-// Phantom stage.  Input: the batch's primary records (q.in_q == null) or the
-// return queue; output: the head queue.  Persistent grid with the
-// phase-batched lane loop of the dose transport kernel (refill / fly /
-// interact, one phase per warp iteration).  FFM: free-flight mode (kFf*).
-template <typename real, int MINB, int FFM>
-__global__ void __launch_bounds__(256, MINB) k_spect_phantom(Scene<real> sg, KernelArgs args, StageArgs q) {
+// The phantom stage's part of a slot: x the input-queue flag (1: the photon
+// came back from a head and carries an event), y its queue entry, z split
+// copies of the history so far, w Compton interactions of the analog track.
+template <typename real>
+struct PhantomPart {
+  uint4 v;
+};
+template <>
+struct PhantomPart<float> {
+  uint4 v, pad;
+};
+template <typename real>
+using PhantomSlot = PhotonSlot<real, PhantomPart<real>>;
+static_assert(sizeof(PhantomSlot<float>) % 32 == 16 && sizeof(PhantomSlot<double>) % 32 == 16, "odd 16-byte stride");
+
+// The event of a photon that came back from a head and died in the phantom
+// (out of line: less than 1 % of the photons).
+template <typename real>
+static __device__ __noinline__ unsigned score_returned(const Scene<real> &s, void *in_q, size_t q_cap, uint32_t entry,
+                                                       int run, Rng g) {
+  const PQueue<real> in = PQueue<real>::carve(in_q, q_cap);
+  Event<real> ev;
+  real v[kEvSlots];
+  load_event(in, entry, v);
+  event_from(v, ev);
+  return score_singles(s, ev, run, g);
+}
+
+// Phantom stage: the pooled event loop of gg_pool.cuh (as the dose transport).
+// Input: the batch's primary records (q.in_q == null) or the return queue;
+// output: the head queue.  Events: a new photon, a Woodcock step in the image,
+// a flight in the world (to a head box: the photon leaves the stage), an
+// interaction.  SPLIT (scatter splitting): photons that reach a head die
+// there, and every Compton up to the maximum level and every Rayleigh
+// scattering asks for split copies (GateScatterSplittingFreeFlightOptrActor.cpp:
+// 291-360), made by the split kernel.
+template <typename real, bool SPLIT>
+__global__ void __launch_bounds__(PoolShape<real>::kBlock, 1)
+    k_spect_phantom(const __grid_constant__ Scene<real> sg, KernelArgs args, StageArgs q, int n_slots) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
-  __shared__ real sec_store[6 * 256];
+  using Shape = PoolShape<real>;
+  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
+  __shared__ __align__(16) unsigned push[kGangs][3 * kQueues];
+  __shared__ __align__(16) uint32_t ahead[Shape::kBlock][4];  // EventRng's second block of each thread
+  __shared__ uint16_t ring[kGangs][kQueues * Shape::kRing];
+  __shared__ unsigned long long s_claim[kGangs];
   Scene<real> s = sg;
-  stage_tables(sg, s, smem_raw, bc);
-  const bool from_queue = q.in_q != nullptr;
+  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
+  const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
+  const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
+  // dynamic shared memory: slots of the gangs, tables
+  PhantomSlot<real> *const slots = reinterpret_cast<PhantomSlot<real> *>(smem_raw) + gang * n_slots;
+  EventQueues<Shape::kRing> Q;
+  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
+         (unsigned)n_slots);
+  for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) {
+    slots[i].e = make_uint4(0u, 0u, 0u, 0u);
+    slots[i].x.v = make_uint4(0u, 0u, 0u, 0u);
+  }
+  stage_tables(sg, s, smem_raw + sizeof(PhantomSlot<real>) * (size_t)(gangs * n_slots), bc);
+
+  const bool from_queue = !SPLIT && q.in_q != nullptr;
   const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
   PQueue<real> in{};
   if (from_queue) in = PQueue<real>::carve(q.in_q, q.q_cap);
-  const PQueue<real> out = PQueue<real>::carve(q.out_q, q.q_cap);
   // a queue length above the capacity means entries were dropped (status
   // GG_ERR_QUEUE_OVERFLOW): never read past the capacity
-  const uint64_t n_items = from_queue ? min((uint64_t)*q.in_n, (uint64_t)q.q_cap) : args.h_end - args.h_begin;
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  __shared__ uint64_t wpool[kBlock / 32][2];  // per warp: claimed histories not yet handed out
-  uint64_t *pool = wpool[threadIdx.x >> 5];
-  if (lane == 0) pool[0] = pool[1] = 0;
-  __syncwarp();
-
-  Photon<real> ph;
-  ph.alive = 0;
-  ph.in_head = 0;
-  ph.head = 0;
-  ph.hreg = 0;
+  const uint32_t n_items =
+      (uint32_t)(from_queue ? min((uint64_t)*q.in_n, (uint64_t)q.q_cap) : args.h_end - args.h_begin);
+  const PQueue<real> out = PQueue<real>::carve(q.out_q, q.q_cap);
+  const uint32_t slot0 = (blockIdx.x * (uint32_t)gangs + (uint32_t)gang) * (uint32_t)n_slots;
   Secondary<real> sec;
-  sec.base = sec_store;
-  sec.stride = blockDim.x;
-  sec.tid = threadIdx.x;
-  sec.has = 0;
-  HistList<real> l{nullptr, nullptr, 0, 0};  // never scored here
-  Tally<real> t{nullptr, nullptr};
-  Event<real> ev_unused;
-  Rng g;
-  int state = kRefill;
-  bool in_hist = false;
-  // input-queue slot of the lane's photon | kHasEv when it carries an event
-  // (read when the photon dies or leaves)
-  __shared__ uint64_t sslot[kBlock];
-  constexpr uint64_t kHasEv = 1ull << 63;
-  sslot[threadIdx.x] = 0;
-  int pmat = 0, pscored = 0;
-  uint32_t pv = 0;
-  unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0, n_singles = 0;
-  uint32_t nsplit = 0;  // split copies of the history so far
-  int ncompt = 0;       // Compton interactions of the analog track
+  sec.base = reinterpret_cast<real *>(args.slot_scratch);
+  sec.stride = (int)(gridDim.x * (uint32_t)(gangs * n_slots));
+  const uint32_t k0 = (uint32_t)args.seed, k1 = (uint32_t)(args.seed >> 32);
+  unsigned int n_wood = 0, n_real = 0, n_world = 0, n_singles = 0, n_esc = 0;
+  ItemClaims claims;
+  claims.init();
 
   for (;;) {
-    // phase chosen per block: all warps run the same code region at the same
-    // time (instruction-cache locality); thresholds are per warp
-    const unsigned m_ref = __ballot_sync(0xffffffffu, state == kRefill);
-    const int c_ref = __syncthreads_count(state == kRefill);
-    const int c_fly = __syncthreads_count(state == kFly);
-    const int c_int = __syncthreads_count(state == kInteract);
-    if (c_ref + c_fly + c_int == 0) break;
-    const int n_warps = (int)(blockDim.x >> 5);
-    int phase;
-    if (c_ref >= args.refill_min * n_warps || (c_fly + c_int) == 0) phase = kRefill;
-    else if (c_int >= args.interact_min * n_warps || c_fly == 0) phase = kInteract;
-    else phase = kFly;
-
-    if (phase == kRefill) {
-      const bool need = state == kRefill;
-      if (need && in_hist && (sslot[threadIdx.x] & kHasEv)) {
-        // a photon that came back from a head died here: score its event
-        Event<real> ev;
-        real v[kEvSlots];
-        load_event(in, sslot[threadIdx.x] & ~kHasEv, v);
-        event_from(v, ev);
-        n_singles += score_singles(s, ev, ph.run, g);
-      }
-      if (need) in_hist = false;
-      const uint64_t h = warp_pool_claim(pool, m_ref, lane, lt_mask, args.next, args.chunk);
-      if (need) {
-        if (h >= n_items) {
-          state = kDone;
-        } else if (from_queue) {
-          bool has_ev;
-          queue_get<real, FFM != kFfOff>(s, in, h, ph, g, args.seed, has_ev);
-          sslot[threadIdx.x] = h | (has_ev ? kHasEv : 0ull);
-          ph.in_head = 0;
-          ph.in_image = 1;
-          ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-          state = kFly;
-          in_hist = true;
-        } else {
-          const uint64_t r = h + (args.h_begin - args.rec_first);  // record of the history
-          const uint32_t f = rec.flags[r];
-          const uint32_t rs = f & 3u;
-          if (rs != kRecDead) {
-            ph.pos[0] = rec.px[r];
-            ph.pos[1] = rec.py[r];
-            ph.pos[2] = rec.pz[r];
-            ph.dir[0] = rec.dx[r];
-            ph.dir[1] = rec.dy[r];
-            ph.dir[2] = rec.dz[r];
-            set_energy(s, ph, rec.e[r]);
+    int k;
+    unsigned n;
+    const int event = Q.round(k, n);
+    if (event == kQNone) break;
+    if (event == kQRefill) claims.take(Q, n, args.next, args.chunk, n_items, &s_claim[gang]);
+    int dest = kQNone, idx = 0, kind = 0, copies = 0, pmat = 0;
+    int smat = 0, pscored = 0;
+    uint32_t pv = 0, trials = 0;
+    bool leave = false;                               // to the head queue
+    bool fresh = event != kQFly && event != kQWorld;  // direction and energy change
+    bool live = k >= 0;                               // the slot holds a photon
+    Photon<real> ph;
+    sec.has = 0;
+    uint4 e = make_uint4(0u, 0u, 0u, 0u), x = make_uint4(0u, 0u, 0u, 0u);
+    uint64_t hid = 0;
+    if (k >= 0) {
+      PhantomSlot<real> &S = slots[k];
+      e = S.e;
+      x = S.x.v;
+      ph.alive = 1;
+      uint32_t cw = 0;
+      bool aim = false;  // its path to the image boundary is not known (in a slot: negative)
+      uint32_t *const buf = &S.rng.x;
+      if (event == kQRefill) {
+        if (!SPLIT && x.x) {
+          hid = args.h_begin + e.y;
+          Rng g;
+          rng_resume(g, args.seed, hid, (e.x << 3) | ((e.z >> kSlIdx) & 7u), S.rng);
+          n_singles += score_returned(sg, q.in_q, q.q_cap, x.y, (int)e.w, g);
+        }
+        uint32_t h;
+        const bool have = claims.item(Q.tid, h);
+        uint32_t f = kRecDead;
+        size_t r = h;
+        if (!from_queue) r += args.h_begin - args.rec_first;  // record of the history
+        if (have) f = from_queue ? kRecInImage : rec.flags[r];
+        dest = have || !claims.exhausted ? kQRefill : kQNone;
+        live = (f & 3u) != kRecDead;
+        e = x = make_uint4(0u, 0u, 0u, 0u);
+        if (live) {
+          const real *const src[7] = {from_queue ? in.px : rec.px, from_queue ? in.py : rec.py,
+                                      from_queue ? in.pz : rec.pz, from_queue ? in.dx : rec.dx,
+                                      from_queue ? in.dy : rec.dy, from_queue ? in.dz : rec.dz,
+                                      from_queue ? in.e : rec.e};
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            ph.pos[a] = src[a][r];
+            ph.dir[a] = src[3 + a][r];
+          }
+          set_energy(s, ph, src[6][r]);
+          const uint32_t rp = (from_queue ? in.rng_pos : rec.rng_pos)[r];
+          S.rng = (from_queue ? in.rng_buf : rec.rng_buf)[r];
+          e.x = rp >> 3;
+          idx = (int)(rp & 7u);
+          e.y = h;
+          ph.exclude = -1;
+          if (from_queue) {
+            const uint32_t m = in.meta[h];
+            e.y = (uint32_t)(in.hid[h] - args.h_begin);
+            ph.steps = (int)(m & kMetaSteps);
+            ph.exclude = (int)((m >> kMetaExcl) & 7u) - 1;
+            x.x = (m >> kMetaEv) & 1u;
+            x.y = h;
+          } else {
             ph.steps = (int)((f >> 2) & 1u);
-            ph.alive = 1;
-            ph.can_enter = 1;
-            ph.in_head = 0;
-            ph.exclude = -1;
-            ph.w = s.s_fd_w;  // 1, or the forced direction's cone weight
-            const uint64_t hid = args.h_begin + h;
-            ph.run = run_of(s, hid);
-            sslot[threadIdx.x] = 0;
-            nsplit = 0;
-            ncompt = 0;
-            rng_resume(g, args.seed, hid, rec.rng_pos[r], rec.rng_buf[r]);
-            if (rs == kRecInImage) {
-              ph.in_image = 1;
-              ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-              state = kFly;
-            } else if (rs == kRecWorld) {
-              ph.in_image = 0;
-              state = kFly;
-            } else {
-              ph.in_image = 0;
-              pmat = s.world_mat;
-              pscored = 0;
-              state = kInteract;
-            }
-            in_hist = true;
           }
+          e.w = (uint32_t)run_of(s, args.h_begin + e.y);
+          ph.t_exit = R<real>(0);
+          aim = (f & 3u) == kRecInImage;
+          dest = aim ? kQFly : kQWorld;
+          if ((f & 3u) == kRecPendingWorld) {
+            smat = s.world_mat;
+            dest = kQInteract;
+          }
+        }
+      } else {
+        slot_load(S, e, ph, cw, idx);
+        ph.exclude = (int)((e.z >> kSlExcl) & 3u) - 1;
+        sec.has = (int)((e.z >> kSlSec) & 1u);
+        dest = kQFly;
+        aim = event == kQFly && ph.t_exit < R<real>(0);
+      }
+      ph.run = (int)e.w;
+      ph.in_head = 0;
+      sec.tid = (int)(slot0 + (uint32_t)k);
+      hid = args.h_begin + e.y;
+      const uint32_t h0 = (uint32_t)hid, h1 = (uint32_t)(hid >> 32);
+      if (event == kQInteract) {
+        pmat = (int)(cw >> 16);
+        pscored = (int)((e.z >> kSlImage) & 1u);
+        pv = real_bits(ph.t_exit);
+        EventRng g{buf, ahead[threadIdx.x], k0, k1, 0u, h0, h1, e.x, idx};
+        g.begin();
+        real ed;
+        const bool done = pool_interact(s, ph, g, &bc, sec, pmat, (e.z >> kSlRetry) != 0u, trials, kind, ed);
+        g.end();
+        e.x = g.blk;
+        idx = g.idx;
+        if (!done) {
+          dest = kQInteract;
+          smat = pmat;
+        } else {
+          aim = pscored && ph.alive;
+          if (!pscored) {
+            dest = kQWorld;
+            ph.exclude = -1;
+          }
+          if constexpr (SPLIT) {
+            if (kind == kCompton && s.ss_nc > 0) {
+              if ((int)++x.w > s.ss_max) ph.alive = 0;
+              else copies = s.ss_nc;
+            } else if (kind == kRayleigh) {
+              copies = s.ss_nr;
+            }
+            aim = aim && ph.alive;
+          }
+          if (!ph.alive) dest = kQRefill;
         }
       }
-    } else if (phase == kInteract) {
-      if constexpr (FFM == kFfScatter) {
-        // GateScatterSplittingFreeFlightOptrActor.cpp:291-360: every Compton
-        // up to the maximum level and every Rayleigh is split; the analog
-        // photon goes on, and is killed after a Compton beyond the level
-        const Photon<real> pre = ph;
-        int kind = 0, n = 0;
-        if (state == kInteract) {
-          state = do_interaction<real, true>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev_unused, &kind);
-          if (kind == kCompton && s.ss_nc > 0) {
-            if (++ncompt > s.ss_max) {
-              ph.alive = 0;
-              state = kRefill;
+      if (aim) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
+      if (event == kQWorld || dest == kQFly) {
+        // ---- a flight
+        if (++ph.steps > kStepCap) {
+          atomicAdd(&bc.loop_capped, 1u);
+          dest = kQRefill;
+        } else {
+          TwoWords g;
+          g.draw(buf, e.x, idx, 0u, h0, h1, k0, k1);
+          if (event == kQWorld) {
+            ++n_world;
+            ph.in_image = 0;
+            if (spect_world_flight(s, ph, g)) {
+              smat = s.world_mat;
+              pscored = 0;
+              dest = kQInteract;
+            } else if (ph.alive && ph.in_image) {
+              ph.t_exit = R<real>(-1);
+              dest = kQFly;
             } else {
-              n = s.ss_nc;
+              // stopped by a shield, out of the world, or at a head (split copies only are detected there)
+              leave = !SPLIT && ph.alive;
+              dest = kQRefill;
+              if (!leave) ++n_esc;
             }
-          } else if (kind == kRayleigh) {
-            n = s.ss_nr;
+          } else {
+            ph.in_image = 1;
+            const int r = image_flight(s, ph, g, smat, pv, pscored, n_wood, n_real);
+            dest = r == kInteract ? kQInteract : (ph.in_image ? kQFly : kQWorld);
           }
+          g.end(buf, e.x, idx);
         }
-        // the copies are made by the split kernel: one request per split interaction
-        const bool req_c = n > 0 && kind == kCompton, req_r = n > 0 && kind == kRayleigh;
+      }
+    }
+    // ---- collective claims: split requests, head-queue entries
+    if constexpr (SPLIT) {
+      if (event == kQInteract) {
+        const bool req_c = copies > 0 && kind == kCompton, req_r = copies > 0 && kind == kRayleigh;
         const size_t kc = queue_claim(q.split_n, req_c, lane, lt_mask);
         const size_t kr = queue_claim(q.split_n + 1, req_r, lane, lt_mask);
-        if (req_c || req_r) {
+        if (copies > 0) {
           // past the capacity the split kernel skips the whole buffer and the pass is repeated
           if (req_c ? kc < q.split_cap : kr < q.split_cap) {
-            const size_t k = req_c ? kc : q.split_cap - 1 - kr;
+            const size_t j = req_c ? kc : q.split_cap - 1 - kr;
             const SplitQueue<real> sq = SplitQueue<real>::carve(q.split_q, q.split_cap);
-            sq.hid[k] = rng_history(g);
-            sq.px[k] = pre.pos[0];
-            sq.py[k] = pre.pos[1];
-            sq.pz[k] = pre.pos[2];
-            sq.dx[k] = pre.dir[0];
-            sq.dy[k] = pre.dir[1];
-            sq.dz[k] = pre.dir[2];
-            sq.e[k] = pre.e;
-            sq.w[k] = pre.w;
-            sq.base[k] = nsplit;
-            sq.comp[k] = s.mat_comp[pmat];
-            sq.run[k] = ph.run;
+            const Real4<real> a = slots[k].a, b = slots[k].b;  // the photon before the interaction
+            sq.hid[j] = hid;
+            sq.px[j] = a.x;
+            sq.py[j] = a.y;
+            sq.pz[j] = a.z;
+            sq.dx[j] = b.x;
+            sq.dy[j] = b.y;
+            sq.dz[j] = b.z;
+            sq.e[j] = b.w;
+            sq.w[j] = s.s_fd_w;
+            sq.base[j] = x.z;
+            sq.comp[j] = s.mat_comp[pmat];
+            sq.run[j] = ph.run;
           }
-          nsplit += (uint32_t)n;
-        }
-        if (state == kRefill && sec.has) {
-          pop_secondary(s, ph, sec);
-          ncompt = 0;
-          state = kFly;
-        }
-      } else if (state == kInteract) {
-        state = do_interaction<real, true>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev_unused);
-        if (state == kRefill && sec.has) {
-          pop_secondary(s, ph, sec);
-          state = kFly;
+          x.z += (uint32_t)copies;
         }
       }
     } else {
-      if (state == kFly) {
-        state = phantom_flight<real, FFM>(s, ph, g, &bc, pmat, pv, pscored, n_wood, n_real, n_world);
-        if (state == kRefill && sec.has) {
-          pop_secondary(s, ph, sec);
-          state = kFly;
+      if (event == kQWorld) {
+        const size_t j = queue_claim(q.out_n, leave, lane, lt_mask);
+        if (leave) {
+          if (j < q.q_cap) {
+            Rng g;
+            rng_resume(g, args.seed, hid, (e.x << 3) | (uint32_t)idx, slots[k].rng);
+            real v[kEvSlots];
+            if (x.x) load_event(in, x.y, v);
+            queue_put<real, false>(out, j, ph, g, hid, v, x.x != 0u);
+          } else {
+            atomicOr(args.status, kStatusQueueOverflow);
+          }
+          x.x = 0u;  // nothing to score here
         }
       }
-      const bool push = state == kPush;
-      const size_t k = queue_claim(q.out_n, push, lane, lt_mask);
-      if (push) {
-        if (k < q.q_cap) {
-          real v[kEvSlots];
-          const uint64_t sl = sslot[threadIdx.x];
-          const bool has_ev = (sl & kHasEv) != 0;
-          if (has_ev) load_event(in, sl & ~kHasEv, v);
-          queue_put<real, FFM != kFfOff>(out, k, ph, g, rng_history(g), v, has_ev);
-        } else {
-          atomicOr(args.status, kStatusQueueOverflow);
-        }
-        in_hist = false;
-        state = kRefill;
+    }
+    if (k >= 0) {
+      PhantomSlot<real> &S = slots[k];
+      if (dest == kQRefill && sec.has && !leave) {
+        take_secondary(s, ph, sec);
+        ph.t_exit = R<real>(-1);
+        dest = ph.in_image ? kQFly : kQWorld;
+        fresh = true;
+        x.w = 0u;
+      }
+      // ---- the photon back into its slot
+      const bool pend = dest == kQInteract;
+      if (live) {
+        slot_store(S, ph, pend, fresh, smat, pv, trials);
+        e.z = (uint32_t)ph.steps | ((uint32_t)idx << kSlIdx) | ((uint32_t)(ph.exclude + 1) << kSlExcl) |
+              ((uint32_t)sec.has << kSlSec);
+        if (pend) e.z |= (pscored ? 1u << kSlImage : 0u) | (trials ? 1u << kSlRetry : 0u);
+      }
+      S.e = e;
+      if (fresh || leave) S.x.v = x;
+    }
+    if (event == kQRefill) claims.advance(n);
+    Q.put(dest, k, lane, lt_mask);
+  }
+  stage_counters(args.counters, bc, lane, n_wood, n_real, n_world, 0u, n_singles);
+  unsigned long long esc = n_esc;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) esc += __shfl_down_sync(0xffffffffu, esc, o);
+  if (lane == 0 && esc) atomicAdd(&args.counters[GG_CNT_ESCAPED], esc);
+}
+
+// Phantom stage of primary free flight: the checks of every primary's flight
+// (cutoffs, angle, the head its line enters); the optical depth of those that
+// pass is walked by k_spect_walk.  One record per thread, nothing to batch.
+template <typename real>
+__global__ void __launch_bounds__(256) k_spect_primary(Scene<real> s, KernelArgs args, StageArgs q) {
+  __shared__ BlockCounters bc;
+  if (threadIdx.x == 0) bc = BlockCounters{0, 0, 0, 0, 0, 0, 0, 0};
+  __syncthreads();
+  const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
+  const PQueue<real> out = PQueue<real>::carve(q.out_q, q.q_cap);
+  const uint64_t n = args.h_end - args.h_begin;
+  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
+  unsigned int n_world = 0, n_esc = 0;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t h = i0 + threadIdx.x, hid = args.h_begin + h, r = hid - args.rec_first;
+    Photon<real> ph;
+    bool push = false;
+    uint32_t f = kRecDead;
+    if (h < n) f = rec.flags[r];
+    if ((f & 3u) != kRecDead) {
+      ph.pos[0] = rec.px[r];
+      ph.pos[1] = rec.py[r];
+      ph.pos[2] = rec.pz[r];
+      ph.dir[0] = rec.dx[r];
+      ph.dir[1] = rec.dy[r];
+      ph.dir[2] = rec.dz[r];
+      ph.e = rec.e[r];
+      ph.steps = (int)((f >> 2) & 1u) + 1;  // (one flight: far below the step cap)
+      ph.alive = 1;
+      ph.exclude = -1;
+      ph.head = ph.hreg = 0;
+      ph.w = s.s_fd_w;  // 1, or the forced direction's cone weight
+      ph.run = run_of(s, hid);
+      ++n_world;
+      real tb;
+      push = ff_target(s, ph, s.ss_cos, tb) != 0;
+      if (!push) ++n_esc;
+    }
+    const size_t k = queue_claim(q.out_n, push, lane, lt_mask);
+    if (push) {
+      if (k < q.q_cap) {
+        Rng g;
+        rng_resume(g, args.seed, hid, rec.rng_pos[r], rec.rng_buf[r]);
+        real v[kEvSlots];
+        queue_put<real, true>(out, k, ph, g, hid, v, false);
+      } else {
+        atomicOr(args.status, kStatusQueueOverflow);
       }
     }
   }
-  stage_counters(args.counters, bc, lane, n_wood, n_real, n_world, 0u, n_singles);
+  if (n_esc) atomicAdd(&bc.escaped, n_esc);
+  stage_counters(args.counters, bc, lane, 0u, 0u, n_world, 0u, 0u);
 }
 
 // Head stage.  Input: the head queue; output: the return queue.  Each lane
@@ -754,47 +846,57 @@ cudaError_t launch_projection_f64(int kind, const unsigned long long *src, doubl
   return cudaGetLastError();
 }
 
-// MINB / HMINB: register budgets (resident 256-thread blocks per SM) of the
-// phantom and the head stage.
-template <typename real, int MINB, int FFM = kFfOff, int HMINB = MINB>
-static cudaError_t launch_stage_v(int stage, const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid,
-                                  int block, size_t smem, cudaStream_t st) {
-  constexpr bool FF = FFM != kFfOff;
-  static unsigned long long configured[2] = {0, 0};
-  cudaError_t e = stage == 0 ? configure_smem(k_spect_phantom<real, MINB, FFM>, 200 * 1024, configured[0])
-                             : configure_smem(k_spect_head<real, HMINB, FF>, 200 * 1024, configured[1]);
+template <typename real, int MINB, bool FF>
+static cudaError_t launch_head_v(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid, int block,
+                                 size_t smem, cudaStream_t st) {
+  static unsigned long long configured = 0;
+  cudaError_t e = configure_smem(k_spect_head<real, MINB, FF>, 200 * 1024, configured);
   if (e != cudaSuccess) return e;
-  if (stage == 0) k_spect_phantom<real, MINB, FFM><<<grid, block, smem, st>>>(s, a, q);
-  else k_spect_head<real, HMINB, FF><<<grid, block, smem, st>>>(s, a, q);
+  k_spect_head<real, MINB, FF><<<grid, block, smem, st>>>(s, a, q);
   return cudaGetLastError();
 }
 
 template <typename real>
-cudaError_t launch_spect_stage(int stage, const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid,
-                               int block, size_t smem, int minb, cudaStream_t st) {
+cudaError_t launch_spect_head(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int grid, int block,
+                              size_t smem, int minb, cudaStream_t st) {
   // free flight: one register budget (4 blocks of 256 threads per SM); a
   // smaller grid computed for another budget is a valid launch of it
-  // the splitting loop keeps the photon before the interaction live: the
-  // scatter-splitting phantom stage gets the 3-block register budget (80
-  // registers, no spills; 15 % faster than 2 blocks at 90)
-  if (s.ff == kFfScatter) return launch_stage_v<real, 3, kFfScatter, 4>(stage, s, a, q, grid, block, smem, st);
-  if (s.ff) return launch_stage_v<real, 4, kFfPrimary>(stage, s, a, q, grid, block, smem, st);
-  if (minb <= 2) return launch_stage_v<real, 2>(stage, s, a, q, grid, block, smem, st);
-  if (minb == 3) return launch_stage_v<real, 3>(stage, s, a, q, grid, block, smem, st);
-  return launch_stage_v<real, 4>(stage, s, a, q, grid, block, smem, st);
+  if (s.ff) return launch_head_v<real, 4, true>(s, a, q, grid, block, smem, st);
+  if (minb <= 2) return launch_head_v<real, 2, false>(s, a, q, grid, block, smem, st);
+  if (minb == 3) return launch_head_v<real, 3, false>(s, a, q, grid, block, smem, st);
+  return launch_head_v<real, 4, false>(s, a, q, grid, block, smem, st);
 }
 
-template <typename real, int MINB>
-static cudaError_t stage_occupancy_v(int stage, int block, size_t smem, int *bps) {
-  return stage == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_spect_phantom<real, MINB, kFfOff>, block, smem)
-                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_spect_head<real, MINB, false>, block, smem);
+template <typename real, bool SPLIT>
+static cudaError_t launch_phantom_v(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, const PoolPlan &p,
+                                    cudaStream_t st) {
+  static unsigned long long configured = 0;
+  cudaError_t e = configure_smem(k_spect_phantom<real, SPLIT>, 227 * 1024, configured);
+  if (e != cudaSuccess) return e;
+  k_spect_phantom<real, SPLIT><<<p.grid, p.block, p.smem, st>>>(s, a, q, p.slots);
+  return cudaGetLastError();
 }
 
 template <typename real>
-cudaError_t spect_stage_occupancy(int stage, int block, size_t smem, int minb, int *blocks_per_sm) {
-  if (minb <= 2) return stage_occupancy_v<real, 2>(stage, block, smem, blocks_per_sm);
-  if (minb == 3) return stage_occupancy_v<real, 3>(stage, block, smem, blocks_per_sm);
-  return stage_occupancy_v<real, 4>(stage, block, smem, blocks_per_sm);
+cudaError_t launch_spect_phantom(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, const PoolPlan &p,
+                                 int n_sm, cudaStream_t st) {
+  if (s.ff == kFfPrimary) {
+    k_spect_primary<real><<<n_sm * 8, 256, 0, st>>>(s, a, q);
+    return cudaGetLastError();
+  }
+  return s.ff == kFfScatter ? launch_phantom_v<real, true>(s, a, q, p, st) : launch_phantom_v<real, false>(s, a, q, p, st);
+}
+
+template <typename real>
+size_t phantom_slot_bytes() {
+  return sizeof(PhantomSlot<real>);
+}
+
+template <typename real>
+cudaError_t spect_head_occupancy(int block, size_t smem, int minb, int *bps) {
+  if (minb <= 2) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_spect_head<real, 2, false>, block, smem);
+  if (minb == 3) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_spect_head<real, 3, false>, block, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_spect_head<real, 4, false>, block, smem);
 }
 
 template <typename real>
@@ -835,11 +937,17 @@ template cudaError_t launch_spect_split<double>(const Scene<double> &, const Ker
                                                 size_t, int, cudaStream_t);
 template size_t queue_bytes<float>(size_t);
 template size_t queue_bytes<double>(size_t);
-template cudaError_t launch_spect_stage<float>(int, const Scene<float> &, const KernelArgs &, const StageArgs &, int,
-                                               int, size_t, int, cudaStream_t);
-template cudaError_t launch_spect_stage<double>(int, const Scene<double> &, const KernelArgs &, const StageArgs &,
-                                                int, int, size_t, int, cudaStream_t);
-template cudaError_t spect_stage_occupancy<float>(int, int, size_t, int, int *);
-template cudaError_t spect_stage_occupancy<double>(int, int, size_t, int, int *);
+template size_t phantom_slot_bytes<float>();
+template size_t phantom_slot_bytes<double>();
+template cudaError_t launch_spect_phantom<float>(const Scene<float> &, const KernelArgs &, const StageArgs &,
+                                                 const PoolPlan &, int, cudaStream_t);
+template cudaError_t launch_spect_phantom<double>(const Scene<double> &, const KernelArgs &, const StageArgs &,
+                                                  const PoolPlan &, int, cudaStream_t);
+template cudaError_t launch_spect_head<float>(const Scene<float> &, const KernelArgs &, const StageArgs &, int, int,
+                                              size_t, int, cudaStream_t);
+template cudaError_t launch_spect_head<double>(const Scene<double> &, const KernelArgs &, const StageArgs &, int, int,
+                                               size_t, int, cudaStream_t);
+template cudaError_t spect_head_occupancy<float>(int, size_t, int, int *);
+template cudaError_t spect_head_occupancy<double>(int, size_t, int, int *);
 
 }  // namespace gg

@@ -275,8 +275,8 @@ __device__ __forceinline__ int head_flight(const Scene<real> &s, Photon<real> &p
 // World step with the image box and the head boxes as targets.  Returns
 // 1 for an air interaction at the new position, 0 otherwise (ph.alive = 0
 // when the photon left the world).
-template <typename real>
-__device__ __forceinline__ int spect_world_flight(const Scene<real> &s, Photon<real> &ph, Rng &g) {
+template <typename real, typename G>
+__device__ __forceinline__ int spect_world_flight(const Scene<real> &s, Photon<real> &ph, G &g) {
   real inf = gg_inf(real(0));
   real tb = ph.exclude != 0 ? entry_distance(ph.pos, ph.dir, s.bmin, s.bmax) : inf;
   int box = 0, bface = 2;
@@ -309,8 +309,7 @@ __device__ __forceinline__ int spect_world_flight(const Scene<real> &s, Photon<r
   if (tb <= tout) {
     move3(ph.pos, ph.dir, tb);
     if (box == 0) {
-      ph.in_image = 1;
-      ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
+      ph.in_image = 1;  // (the path inside the image is the caller's)
     } else if (s.side_black && bface != 2) {
       ph.alive = 0;  // stopped by the head's side shielding
     } else {

@@ -189,12 +189,6 @@ __device__ __forceinline__ Tally<real> tally_at(const KernelArgs &a, size_t off,
   return Tally<real>{a.acc_e + off, a.acc_e2 ? a.acc_e2 + 2 * off : nullptr};
 }
 
-// Compton trials of one interaction event; a photon that is rejected as often
-// waits for the next event with the photons it meets there, instead of keeping
-// its warp in the loop (a third of the trials fail; the worst of 32 lanes takes
-// five or six).
-constexpr int kKnTrials = 2;
-
 // Transport stage: the pooled event loop of gg_pool.cuh.  Events: a new history
 // (the ended one's voxel list goes to the tallies first), a Woodcock step in
 // the image, a free flight in the world, an interaction; a photon that starts
@@ -222,12 +216,12 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
   const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
   // dynamic shared memory: slots of the gangs, tables
-  PhotonSlot<real> *const slots = reinterpret_cast<PhotonSlot<real> *>(smem_raw) + gang * n_slots;
+  DoseSlot<real> *const slots = reinterpret_cast<DoseSlot<real> *>(smem_raw) + gang * n_slots;
   EventQueues<Shape::kRing> Q;
   Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
          (unsigned)n_slots);
   for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) slots[i].e = make_uint4(0u, 0u, 0u, 0u);
-  stage_tables(sg, s, smem_raw + sizeof(PhotonSlot<real>) * (size_t)(gangs * n_slots), bc);
+  stage_tables(sg, s, smem_raw + sizeof(DoseSlot<real>) * (size_t)(gangs * n_slots), bc);
 
   const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
   Tally<real> t{args.acc_e, args.acc_e2};
@@ -243,8 +237,8 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   ld.gv = reinterpret_cast<uint32_t *>(ld.ga + kHistList * (size_t)all_slots);
   ld.slots = all_slots;
   unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0, n_ent = 0, n_over = 0, n_esc = 0;
-  uint32_t pool_next = 0, pool_end = 0;  // claimed records not yet handed out (the same in the whole gang)
-  bool exhausted = false;
+  ItemClaims claims;
+  claims.init();
 
   for (;;) {
     int k;
@@ -252,31 +246,19 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
     const int event = Q.round(k, n);
     if (event == kQNone) break;
     int dest = kQNone;
-    uint32_t base = 0, got = 0;
-    const uint32_t avail = pool_end - pool_next;
     if (event == kQRefill) {
-      // the n slots take the next n records in thread order (coalesced loads)
-      if (avail < n && !exhausted) {
-        if (Q.tid == 0) s_claim[gang] = atomicAdd(args.next, (unsigned long long)args.chunk);
-        Q.sync();
-        const unsigned long long c = s_claim[gang];
-        if (c < n_hist) {
-          base = (uint32_t)c;
-          got = min((uint32_t)args.chunk, n_hist - base);
-        }
-        exhausted = c + (unsigned long long)args.chunk >= n_hist;
-      }
+      claims.take(Q, n, args.next, args.chunk, n_hist, &s_claim[gang]);
       // the ended histories' voxel lists
       lists_flush(slots, max(k, 0), k >= 0 ? (int)((slots[k].e.z >> kSlList) & 15u) : 0,
                   reinterpret_cast<uint16_t *>(ahead[threadIdx.x & ~31u]), lane,
-                  [&](const PhotonSlot<real> &S) {
+                  [&](const DoseSlot<real> &S) {
                     if constexpr (MULTI) return tally_at(args, sg.sims[S.e.w].vox_off, real(0));
                     else return t;
                   },
                   n_ent);
     }
     if (k >= 0) {
-      PhotonSlot<real> &S = slots[k];
+      DoseSlot<real> &S = slots[k];
       uint4 e = S.e;
       int n_list = (int)((e.z >> kSlList) & 15u);
       if constexpr (DG == 2) {
@@ -301,12 +283,10 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       if (event == kQRefill) {
         n_list = 0;
         if constexpr (DG == 2) ld.flush(td);
-        const uint32_t r = Q.tid;
-        const bool have = r < avail || r - avail < got;
-        const uint32_t h = r < avail ? pool_next + r : base + (r - avail);
-        uint32_t f = kRecDead;
+        uint32_t h, f = kRecDead;
+        const bool have = claims.item(Q.tid, h);
         if (have) f = rec.flags[h];
-        dest = have || !exhausted ? kQRefill : kQNone;
+        dest = have || !claims.exhausted ? kQRefill : kQNone;
         live = (f & 3u) != kRecDead;
         e = make_uint4(0u, h, 0u, 0u);
         if (live) {
@@ -339,24 +319,9 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           }
         }
       } else {
-        const Real4<real> a = S.a, b = S.b, c = S.c;
-        cw = real_bits(c.w);
-        ph.pos[0] = a.x;
-        ph.pos[1] = a.y;
-        ph.pos[2] = a.z;
-        ph.dir[0] = b.x;
-        ph.dir[1] = b.y;
-        ph.dir[2] = b.z;
-        ph.e = b.w;
-        ph.t_exit = a.w;
-        ph.mumax = c.x;
-        ph.inv_mumax = c.y;
-        ph.ei.fe = c.z;
-        ph.ei.ie = (int)(cw & 0xffffu);
-        ph.steps = (int)(e.z & kSlSteps);
+        slot_load(S, e, ph, cw, idx);
         ph.can_enter = (int)((e.z >> kSlExcl) & 1u);
         sec.has = (int)((e.z >> kSlSec) & 1u);
-        idx = (int)((e.z >> kSlIdx) & 7u);
         dest = kQFly;
         aim = event == kQFly && ph.t_exit < R<real>(0);
       }
@@ -373,40 +338,12 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
         pv = real_bits(ph.t_exit);
         EventRng g{buf, ahead[threadIdx.x], k0, k1, 0u, h0, h1, e.x, idx};
         g.begin();
-        const bool retry = (e.z >> kSlRetry) != 0u;
-        const int kind = retry ? kCompton : select_kind(s, ph, pmat, g);
-        real ed = R<real>(0);
-        bool done = true;
-        real cost = R<real>(1), st2 = R<real>(0), eps = R<real>(1);
-        if (kind == kCompton) {
-          const KleinNishina<real> kn(ph.e);
-          trials = retry ? real_bits(ph.mumax) : 0u;
-          real onecost;
-          int left = kKnTrials;
-#pragma unroll 1
-          do {
-            done = kn.trial(g, eps, onecost, st2);
-            if (!done && ++trials >= (uint32_t)kLoopCap) {
-              atomicAdd(&bc.loop_capped, 1u);
-              done = true;
-            }
-          } while (!done && --left > 0);
-          cost = R<real>(1) - onecost;
-        } else if (kind == kPhoto) {
-          ph.alive = 0;
-          ed = ph.e;
-        } else if (kind == kRayleigh) {
-          cost = rayleigh_cost(s, s.mat_comp[pmat], ph, g, &bc);
-          st2 = rayleigh_sint2(cost);
-        } else {
-          ed = pair_conversion(s, ph, g, &bc, sec);
-        }
-        if (done && (kind == kCompton || kind == kRayleigh)) scatter_dir(ph, g, cost, st2);
-        if (done && kind == kCompton) ed = compton_energy(s, ph, eps);
+        real ed;
+        int kind;
+        const bool done = pool_interact(s, ph, g, &bc, sec, pmat, (e.z >> kSlRetry) != 0u, trials, kind, ed);
         g.end();
         e.x = g.blk;
         idx = g.idx;
-        if (done) trials = 0;
         if (!done) {
           dest = kQInteract;
         } else if (pscored) {
@@ -414,7 +351,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           bool in = true;
           if constexpr (DG > 0) in = dose_voxel(s, ph.pos, v);
           if (in) {
-            list_deposit(S, n_list, t, v, ed, n_dep, n_ent, n_over);
+            list_deposit(S.x, n_list, t, v, ed, n_dep, n_ent, n_over);
             if constexpr (DG == 2) {
               real dd = ed * s.drho_min;
               dd = dd / s.mat_rho[pmat];
@@ -460,15 +397,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       // ---- the photon back into its slot
       const bool pend = dest == kQInteract;
       if (live) {
-        S.a = Real4<real>{ph.pos[0], ph.pos[1], ph.pos[2], pend ? bits_real(real(0), pv) : ph.t_exit};
-        cw = (uint32_t)ph.ei.ie | ((uint32_t)pmat << 16);
-        if (fresh) {
-          S.b = Real4<real>{ph.dir[0], ph.dir[1], ph.dir[2], ph.e};
-          S.c = Real4<real>{trials ? bits_real(real(0), trials) : ph.mumax, ph.inv_mumax, ph.ei.fe,
-                            bits_real(real(0), cw)};
-        } else if (pend) {
-          S.c.w = bits_real(real(0), cw);
-        }
+        slot_store(S, ph, pend, fresh, pmat, pv, trials);
         e.z = (uint32_t)ph.steps | ((uint32_t)idx << kSlIdx) | ((uint32_t)ph.can_enter << kSlExcl) |
               ((uint32_t)sec.has << kSlSec) | ((uint32_t)n_list << kSlList);
         if (pend) e.z |= (pscored ? 1u << kSlImage : 0u) | (trials ? 1u << kSlRetry : 0u);
@@ -476,14 +405,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       if constexpr (DG == 2) e.w = (uint32_t)ld.n;
       S.e = e;
     }
-    if (event == kQRefill) {
-      if (n <= avail) {
-        pool_next += n;
-      } else {
-        pool_next = base + min(n - avail, got);
-        pool_end = base + got;
-      }
-    }
+    if (event == kQRefill) claims.advance(n);
     Q.put(dest, k, lane, lt_mask);
   }
   // ---- counters -------------------------------------------------------------
@@ -803,10 +725,10 @@ cudaError_t tle_occupancy(int block, size_t smem, int minb, int *bps) {
 // the rounds full, so they take all shared memory beside the tables, but no
 // more than the run has histories for.  block, blocks: most threads per block
 // and resident blocks per SM (of 256 threads) of the options, 0 for the
-// kernel's register budget; dose_list: the second list of a dose grid.
+// kernel's register budget; slot_bytes, scratch_bytes: of one slot, shared and global.
 template <typename real>
-cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, bool dose_list,
-                      PoolPlan *p) {
+cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
+                      size_t scratch_bytes, PoolPlan *p) {
   int n_sm = 0, optin = 0;
   cudaError_t e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -818,7 +740,7 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
   if (blocks > 0) threads = std::min(threads, 256 * blocks);
   if (block > 0) threads = std::min(threads, block);
   threads = (int)std::min<uint64_t>(threads, (per_sm + 31) / 32 * 32);
-  const size_t slot = sizeof(PhotonSlot<real>), fixed = pool_static<real>() + table_bytes;
+  const size_t slot = slot_bytes, fixed = pool_static<real>() + table_bytes;
   const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
   while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
   const int gangs = (threads + kGang - 1) / kGang;
@@ -830,9 +752,17 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
   p->gangs = gangs;
   p->slots = (int)std::min<uint64_t>(most, (share + 7) / 8 * 8);
   p->smem = slot * p->slots * gangs + table_bytes;
-  p->scratch = (size_t)p->grid * gangs * p->slots *
-               (6 * sizeof(real) + (dose_list ? kHistList * (sizeof(real) + sizeof(uint32_t)) : 0));
+  p->scratch = (size_t)p->grid * gangs * p->slots * scratch_bytes;
   return cudaSuccess;
+}
+
+template <typename real>
+size_t dose_slot_bytes() {
+  return sizeof(DoseSlot<real>);
+}
+template <typename real>
+size_t slot_scratch_bytes(bool two) {
+  return 6 * sizeof(real) + (two ? kHistList * (sizeof(real) + sizeof(uint32_t)) : 0);
 }
 
 // Histories a gang claims at a time: an even share of a small run, else the
@@ -854,8 +784,12 @@ template cudaError_t launch_transport_tle<float>(const Scene<float> &, const Ker
                                                  cudaStream_t);
 template cudaError_t launch_transport_tle<double>(const Scene<double> &, const KernelArgs &, int, int, size_t, int,
                                                   cudaStream_t);
-template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, bool, PoolPlan *);
-template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, bool, PoolPlan *);
+template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, size_t, size_t, PoolPlan *);
+template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, size_t, size_t, PoolPlan *);
+template size_t dose_slot_bytes<float>();
+template size_t dose_slot_bytes<double>();
+template size_t slot_scratch_bytes<float>(bool);
+template size_t slot_scratch_bytes<double>(bool);
 template cudaError_t tle_occupancy<float>(int, size_t, int, int *);
 template cudaError_t tle_occupancy<double>(int, size_t, int, int *);
 

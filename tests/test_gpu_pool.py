@@ -32,3 +32,33 @@ def test_pool_edges_bit_exact(built_lib, precision, n, opts):
     ref = O.run_dose(scene, n, 97, first=5, batch=1 << 20, threads=4, precision=precision)
     assert got[2] == ref[2]
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("mode", ["plain", "split", "forced"])
+@pytest.mark.parametrize("precision,n,opts", [(32, 1, {}), (32, 2433, dict(chunk=1)), (32, 977, dict(block_size=96)),
+                                              (64, 311, {})])
+def test_phantom_stage_edges_bit_exact(built_lib, mode, precision, n, opts):
+    """The SPECT phantom stage at the same edges: analog, with split requests, and the primary
+    free flight that checks one record per thread."""
+    import copy
+
+    from opengate_gb300 import _capi as C
+    from opengate_gb300.engine import SpectEngine
+    from oracle import oracle as O
+
+    scene, sp, _ = W.spect_phantom(shape=(20, 32, 32), spacing=9.6, n_runs=3)
+    if mode == "split":
+        sp.set_scatter_splitting(6, 3, 2, angle_tolerance_max=0.5)
+    if mode == "forced":
+        sp.set_free_flight()
+        src = copy.copy(scene.source)
+        src.dir_type, src.fd_angle_min, src.fd_angle_max = C.GG_DIR_FORCED, 0.0, 0.4
+        scene.set_source(src)
+    with SpectEngine(scene, sp, precision=precision, **opts) as eng:
+        eng.run(n, 41)
+        got = (eng.projection(),) if mode == "plain" else eng.weighted_projection(squared=True)
+        cnt = eng.counters()
+    run = O.run_spect if mode == "plain" else O.run_spect_ff
+    *ref, rcnt = run(scene, sp, n, seed=41, threads=4, precision=precision)
+    assert cnt == rcnt
+    assert all(np.array_equal(a, b) for a, b in zip(got, ref))
