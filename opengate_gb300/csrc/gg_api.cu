@@ -1187,8 +1187,8 @@ static int spect_stages(gg_ctx *c, gg::KernelArgs a, const gg::PoolPlan &plan, s
       if ((st2 = c->cuda(cudaMemsetAsync(nr, 0, sizeof(unsigned long long), c->stream), "memset"))) return st2;
       if ((st2 = stage_event(c, 2, true))) return st2;
       cudaError_t e = c->precision == GG_PREC_F64
-                          ? gg::launch_spect_split<double>(c->scene<double>(), a, q, c->block, smem, c->n_sm, c->stream)
-                          : gg::launch_spect_split<float>(c->scene<float>(), a, q, c->block, smem, c->n_sm, c->stream);
+                          ? gg::launch_spect_split<double>(c->scene<double>(), a, q, c->n_sm, c->stream)
+                          : gg::launch_spect_split<float>(c->scene<float>(), a, q, c->n_sm, c->stream);
       if ((st2 = c->cuda(e, "split kernel launch"))) return st2;
       gg::StageArgs w{c->d_queue[1], nr, c->d_queue[0], nh, c->q_cap, nullptr, nullptr, 0};
       e = c->precision == GG_PREC_F64

@@ -223,8 +223,8 @@ cudaError_t spect_head_occupancy(int block, size_t smem, int minb, int *blocks_p
 // into the walk queue (q.out_q / q.out_n); does nothing when the requests
 // overflowed the buffer.
 template <typename real>
-cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
-                               int n_sm, cudaStream_t st);
+cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int n_sm,
+                               cudaStream_t st);
 template <typename real>
 size_t split_bytes(size_t cap);
 // Free flights of the copies the split kernel queued (q.in_q / q.in_n) into

@@ -126,6 +126,7 @@ template <typename real>
 struct KleinNishina {
   real k, eps0sq, alpha1, alpha2;
 
+  __device__ __forceinline__ KleinNishina(real kk, real e0, real a1, real a2) : k(kk), eps0sq(e0), alpha1(a1), alpha2(a2) {}
   __device__ __forceinline__ explicit KleinNishina(real e) {
     k = e * R<real>(1.0 / kMC2);
     const real twok = R<real>(2) * k;

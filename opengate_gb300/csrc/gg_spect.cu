@@ -99,12 +99,18 @@ __device__ __forceinline__ void stage_counters(unsigned long long *cnt, const Bl
   }
 }
 
-// Whether a photon of direction d scattered by theta (cos, sin^2) can pass the
-// angle check of some head (ff_target): over the azimuth, the largest cosine
-// between the new direction and a head axis u is cos(theta - theta_u) =
-// cos(theta) (d.u) + sin(theta) sqrt(1 - (d.u)^2).  A margin of 1e-4 on the
-// cosine keeps every direction the full check would accept (rounding is far
-// below it), so dropping the others changes no result.
+// Largest cosine that a photon scattered by theta (cos, sin) can make with a
+// head axis u over the azimuth: cos(theta - theta_u) = cos(theta) c0 + sin(theta)
+// s0, c0 = d.u, s0 = sqrt(1 - c0^2).  A copy whose cosine stays below the angle
+// check of every head (ff_target) is dropped before its azimuth is drawn; a
+// margin of 1e-4 keeps every direction the full check would accept (rounding is
+// far below it), so that changes no result.
+template <typename real>
+__device__ __forceinline__ real axis_sine(real c0) {
+  const real s0 = R<real>(1) - c0 * c0;
+  return gg_sqrt(s0 > R<real>(0) ? s0 : R<real>(0));
+}
+
 template <typename real>
 __device__ __forceinline__ bool cone_reachable(const Scene<real> &s, int run, const real d[3], real cost, real sint2,
                                                real cos_min) {
@@ -113,181 +119,376 @@ __device__ __forceinline__ bool cone_reachable(const Scene<real> &s, int run, co
   for (int h = 0; h < s.n_heads; ++h) {
     const HeadFrame<real> f = head_frame(s, run, h);
     const real c0 = dot3(d, f.u);
-    real s0 = R<real>(1) - c0 * c0;
-    s0 = gg_sqrt(s0 > R<real>(0) ? s0 : R<real>(0));
     real m = cost * c0;
-    m = m + sint * s0;
+    m = m + sint * axis_sine(c0);
     if (!(m < lim)) return true;
   }
   return false;
 }
 
-// Copies of one warp that passed the scattering-angle test and wait for the
-// rest of their scattering and the head checks, kSplitPend at most: the copy
-// index, the sampled (eps, 1 - cos, sin^2) of a Compton or (cos, -, -) of a
-// Rayleigh scattering, and the words of the copy's stream drawn so far.
-constexpr int kSplitPend = 64;
-template <typename real>
-struct SplitPending {
-  uint64_t i[kSplitPend];
-  real a[kSplitPend], b[kSplitPend], c[kSplitPend];
-  uint32_t words[kSplitPend];
+// Words p .. p + 3 of a stream, p = 3 t: a trial's three draws, and the azimuth
+// drawn after it when it is accepted.  w3: word 3, when t = 1 (kept from the
+// first trial, so that the second makes one block too).
+struct TrialWords {
+  uint32_t w[4];
+
+  __device__ __forceinline__ void draw(uint32_t t, uint32_t w3, uint32_t stream, uint32_t h0, uint32_t h1, uint32_t k0,
+                                       uint32_t k1) {
+    const uint32_t p = 3u * t, at = p & 3u;
+    // (in line: the round keys of the launch's seed stay in uniform registers)
+    uint32_t ctr[4] = {(p >> 2) + (t == 1u ? 1u : 0u), stream, h0, h1}, o[4];
+    philox4x32_10(ctr, k0, k1, o);
+    uint4 a = make_uint4(o[0], o[1], o[2], o[3]), b = a;
+    if (t == 1u) a.w = w3;
+    else if (at != 0u) b = philox_block((p >> 2) + 1u, stream, h0, h1, k0, k1);
+    w[0] = at == 0u ? a.x : (at == 1u ? a.y : (at == 2u ? a.z : a.w));
+    w[1] = at == 0u ? a.y : (at == 1u ? a.z : (at == 2u ? a.w : b.x));
+    w[2] = at == 0u ? a.z : (at == 1u ? a.w : (at == 2u ? b.x : b.y));
+    w[3] = at == 0u ? a.w : (at == 1u ? b.x : (at == 2u ? b.y : b.z));
+  }
 };
 
-// Scatter splitting, the copies (GateScatterSplittingFreeFlightOptn.cpp:69-149):
-// one thread per copy.  Request r of the phantom stage holds the photon
-// before a Compton (or Rayleigh) interaction; its copy c re-samples that
-// interaction from there on Philox stream 2 + base + c of the history, with
-// 1 / n of the weight, and flies freely to a head: the intersection check of
-// the angular acceptance is the flight itself (a copy that misses every head
-// cannot be detected), the angle check comes before the optical depth.
-// A copy whose line enters a head (past the checks) goes to the walk queue
-// (q.out_q), where k_spect_walk computes its optical depth: the few copies
-// that pass then walk the voxels with full warps.  Compton requests fill the
-// buffer from the front and Rayleigh requests from the back; when together
-// they overflowed it, nothing is done (the host repeats the pass on fewer
-// histories).
-// Most copies scatter away from every head: right after the rejection loop
-// the scattering angle alone decides that (cone_reachable), and only the
-// others draw their azimuth and meet the full check.  Those wait in a
-// per-warp buffer until 32 of them fill the warp's lanes, so the azimuth,
-// the rotation and the head checks run on full warps; each copy's arithmetic
-// and draws are those of the plain sequence.
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fast_sqrt(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// What is certain about a Klein-Nishina trial and the direction it leads to from
+// approximate arithmetic (hardware exp2, reciprocal, square root: relative
+// errors at most 2^-22, 2^-23, 2^-23; sine, cosine: absolute 2^-20.5):
+//   kTrialRejected  KleinNishina::trial() rejects it;
+//   kTrialDropped   it is accepted, and the copy dies below the energy cut;
+//   kTrialMissed    it is accepted above the cut, and the new direction fails the
+//                   angle check against every head axis (ff_target());
+//   kTrialUnsure    anything else: the exact trial decides.
+// eps carries a relative error below 1.5e-6 (the exponent is at most ln(1 + 2k) <
+// 2 below 1.022 MeV: its rounding adds 7e-7), so 1 - cos = (1 - eps) / (eps k)
+// one below 1.5e-6 / (eps k) + 1e-6, 1 / (eps k) <= 2 + 1 / k; sin^2 twice and the
+// acceptance function once that.  tol = 4e-6 (2 + 1 / k) covers each with a factor
+// of two; the sine lies between those of sin^2 - 2 tol and sin^2 + 2 tol, and 2e-5
+// covers the azimuth's sine and cosine and the exact check's own rounding.
+enum : int { kTrialRejected = 0, kTrialDropped = 1, kTrialMissed = 2, kTrialUnsure = 3 };
+
+struct TrialFilter {
+  float k, eps0sq, alpha1, alpha2, e, tol;
+  // the head axes in the scattering frame of rotate_dir(): along the direction,
+  // and along its two transverse axes (azimuth 0 and a quarter turn)
+  float c0[2], a1[2], a2[2];
+
+  __device__ __forceinline__ int operator()(const uint32_t w[4], float e_min, float cos_min, bool check) const {
+    constexpr float kU = 5.9604644775390625e-08f;
+    const float r0 = (float)(w[0] >> 8) * kU, r1 = (float)(w[1] >> 8) * kU, r2 = (float)(w[2] >> 8) * kU;
+    const float d = alpha1 - alpha2 * r0;
+    const float sq = fmaf(1.0f - eps0sq, r1, eps0sq);
+    const bool log_part = d > 0.0f;
+    const float eps = log_part ? fast_exp2(alpha1 * r1 * -1.44269504f) : fast_sqrt(sq);
+    const float epssq = log_part ? eps * eps : sq;
+    const float onecost = (1.0f - eps) * fast_rcp(eps * k);
+    const float sint2 = onecost * (2.0f - onecost);
+    const float gr = 1.0f - eps * sint2 * fast_rcp(1.0f + epssq);
+    const float ed = eps * e;
+    if (fabsf(d) < 1e-5f * alpha1 || !(fabsf(gr - r2) > tol) || fabsf(ed - e_min) < 1e-5f * e_min) return kTrialUnsure;
+    if (gr < r2) return kTrialRejected;
+    if (ed < e_min) return kTrialDropped;
+    if (!check) return kTrialUnsure;
+    const float phi = (float)(w[3] >> 8) * (kU * 6.28318531f) - 3.14159265f;  // (half a turn off: the signs below)
+    const float cp = __cosf(phi), sp = __sinf(phi);
+    const float cost = 1.0f - onecost, hi = fast_sqrt(fmaxf(sint2 + 2.0f * tol, 0.0f)),
+                lo = fast_sqrt(fmaxf(sint2 - 2.0f * tol, 0.0f));
+    bool miss = true;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float t = -(cp * a1[h] + sp * a2[h]);
+      miss = miss && fmaf(cost, c0[h], (t > 0.0f ? hi : lo) * t) + tol + 2e-5f < cos_min;
+    }
+    return miss ? kTrialMissed : kTrialUnsure;
+  }
+};
+
+// What a warp of the split kernel keeps in shared memory.
+constexpr int kSplitBatch = 32;  // requests at a time
+constexpr int kSplitPend = 64;
+struct SplitWarp {
+  TrialFilter f[kSplitBatch];  // the requests' constants, and their streams
+  uint32_t h0[kSplitBatch], h1[kSplitBatch], stream[kSplitBatch];
+  // copies rejected so far, waiting for their next trial: copy of the batch | trial << 20
+  uint32_t retry[kSplitPend], word3[kSplitPend];  // (word 3 of its stream)
+  // copies of the batch whose trial the filter leaves open: copy | trial << 20
+  uint32_t open[kSplitPend];
+};
+static_assert(GG_MAX_SPLITTING * kSplitBatch < (1 << 20) && kLoopCap < (1 << 12), "a retry packs copy and trial");
+
+// Scatter splitting, the copies (GateScatterSplittingFreeFlightOptn.cpp:69-149).
+// Request r of the phantom stage holds the photon before a Compton (or
+// Rayleigh) interaction; its copy c re-samples that interaction from there on
+// Philox stream 2 + base + c of the history, with 1 / n of the weight, and flies
+// freely to a head: the intersection check of the angular acceptance is the
+// flight itself (a copy that misses every head cannot be detected), the angle
+// check comes before the optical depth.  A copy whose line enters a head (past
+// the checks) goes to the walk queue (q.out_q), where k_spect_walk computes its
+// optical depth.  Compton requests fill the buffer from the front and Rayleigh
+// requests from the back; when together they overflowed it, nothing is done
+// (the host repeats the pass on fewer histories).
+//
+// A warp takes 32 Compton requests: each lane computes one request's constants
+// for all its copies, then the lanes run the copies one trial at a time.  Trial
+// t of a copy draws words 3t .. 3t + 2 of its stream, so a copy needs no state
+// but t between trials: rejected ones wait until 32 such fill a round.  Nearly
+// every trial is settled by approximate arithmetic (TrialFilter); the others
+// wait for a round of the exact trial, the rest of the scattering and the head
+// checks, whose arithmetic and draws are those of the plain sequence.
+// Bound by instruction issue (70 % active, 25.6 lanes): 2.2e8 copies at 140 keV 9 ->
+// 4.1 ms against one thread per copy from request to end; of that, constants per
+// request and full rounds 6.6, the approximate trial with the azimuth 4.3, the
+// generator in line 4.1.
 template <typename real>
-__global__ void __launch_bounds__(256) k_spect_split(Scene<real> sg, KernelArgs args, StageArgs q) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+__global__ void __launch_bounds__(256) k_spect_split(Scene<real> s, KernelArgs args, StageArgs q) {
   __shared__ BlockCounters bc;
-  __shared__ SplitPending<real> pend_all[kBlock / 32];
-  Scene<real> s = sg;
-  stage_tables(sg, s, smem_raw, bc);
+  __shared__ SplitWarp warps[kBlock / 32];
+  if (threadIdx.x == 0) bc = BlockCounters{0, 0, 0, 0, 0, 0, 0, 0};
+  __syncthreads();
   const uint64_t n_c = *q.split_n, n_r = q.split_n[1];
   if (n_c + n_r > (uint64_t)q.split_cap) return;
-  const uint64_t per_c = (uint64_t)s.ss_nc, per_r = (uint64_t)s.ss_nr;
-  const uint64_t all_c = n_c * per_c, total = all_c + n_r * per_r;
   const SplitQueue<real> sq = SplitQueue<real>::carve(q.split_q, q.split_cap);
   const PQueue<real> out = PQueue<real>::carve(q.out_q, q.q_cap);
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
-  SplitPending<real> &P = pend_all[threadIdx.x >> 5];
-  int np = 0;  // copies waiting in P (the same in every lane of the warp)
-  unsigned int n_world = 0;
-  // copy i: its request, the photon before the interaction, its stream
-  auto load_copy = [&](uint64_t i, Photon<real> &cp, Rng &gc, uint64_t &hid) {
-    uint64_t r;
-    uint32_t c, n;
-    if (i < all_c) {
-      r = i / per_c;
-      c = (uint32_t)(i - r * per_c);
-      n = (uint32_t)per_c;
-    } else {
-      const uint64_t j = i - all_c, rr = j / per_r;
-      c = (uint32_t)(j - rr * per_r);
-      r = (uint64_t)q.split_cap - 1 - rr;
-      n = (uint32_t)per_r;
-    }
-    hid = sq.hid[r];
+  SplitWarp &P = warps[threadIdx.x >> 5];
+  const uint32_t k0 = (uint32_t)args.seed, k1 = (uint32_t)(args.seed >> 32);
+  const bool check = s.ss_cos > R<real>(-1);
+  const float cos_min = (float)s.ss_cos, e_min = (float)s.e_min;
+  unsigned int n_world = 0, n_esc = 0;
+
+  // Request r's photon before the interaction, its copy c's stream.
+  auto load_copy = [&](size_t r, uint32_t c, int n, Photon<real> &cp, Rng &g) {
     cp.pos[0] = sq.px[r];
     cp.pos[1] = sq.py[r];
     cp.pos[2] = sq.pz[r];
     cp.dir[0] = sq.dx[r];
     cp.dir[1] = sq.dy[r];
     cp.dir[2] = sq.dz[r];
-    cp.e = sq.e[r];  // the energy-grid state only where a sampling uses it (set_energy)
+    cp.e = sq.e[r];
     cp.w = sq.w[r] / (real)n;
     cp.alive = 1;
     cp.run = sq.run[r];
-    gc.init(args.seed, hid, 2u + sq.base[r] + c);
-    return r;
+    const uint64_t hid = sq.hid[r];
+    g.init(args.seed, hid, 2u + sq.base[r] + c);
+    return hid;
   };
-  // the waiting copies P[k0 + lane] (lane < cnt): the rest of the scattering,
-  // the head checks, and the walk queue (every lane of the warp calls it)
-  auto finish = [&](int k0, int cnt) {
-    Photon<real> cp;
-    Rng gc;
-    uint64_t hid = 0;
+  // A scattered copy's head checks and its place in the walk queue (every lane of the warp calls it).
+  auto to_walk = [&](bool live, Photon<real> &cp, const Rng &g, uint64_t hid) {
     bool push = false;
-    if ((int)lane < cnt) {
-      const int k = k0 + (int)lane;
-      const uint64_t i = P.i[k];
-      load_copy(i, cp, gc, hid);
-      // the stream after its first `w` words: the state an Rng reaches by drawing them
-      const uint32_t w = P.words[k];
-      if ((w & 3u) == 0u) {
-        gc.blk = w >> 2;
-        gc.idx = 4;
-      } else {
-        const uint4 b = philox_block(w >> 2, gc.stream, gc.h0, gc.h1, gc.k0, gc.k1);
-        gc.buf[0] = b.x;
-        gc.buf[1] = b.y;
-        gc.buf[2] = b.z;
-        gc.buf[3] = b.w;
-        gc.blk = (w >> 2) + 1u;
-        gc.idx = (int)(w & 3u);
-      }
-      if (i < all_c) compton_finish(s, cp, gc, P.a[k], P.b[k], P.c[k]);
-      else rayleigh_finish(cp, gc, P.a[k]);
-      if (cp.alive) {
-        cp.exclude = -1;
-        cp.steps = 0;
-        cp.head = 0;
-        cp.hreg = 0;
-        ++n_world;
-        real tb;
-        push = ff_target(s, cp, s.ss_cos, tb) != 0;  // with the angle check of the angular acceptance
-        if (!push) atomicAdd(&bc.escaped, 1u);
-      }
+    if (live) {
+      cp.exclude = -1;
+      cp.steps = 0;
+      cp.head = 0;
+      cp.hreg = 0;
+      ++n_world;
+      real tb;
+      push = ff_target(s, cp, s.ss_cos, tb) != 0;  // with the angle check of the angular acceptance
+      if (!push) ++n_esc;
     }
     const size_t kq = queue_claim(q.out_n, push, lane, lt_mask);
     if (push && kq < q.q_cap) {
       real v[kEvSlots];
-      queue_put<real, true>(out, kq, cp, gc, hid, v, false);
+      queue_put<real, true>(out, kq, cp, g, hid, v, false);
     }
   };
-  // the loop bound is the same for all threads of a block: queue claims stay warp-collective
-  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < total; i0 += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t i = i0 + threadIdx.x;
-    bool wait = false;
-    real a = R<real>(0), b = R<real>(0), c = R<real>(0);
-    Rng gc;
-    if (i < total) {
-      Photon<real> cp;
-      uint64_t hid;
-      const uint64_t r = load_copy(i, cp, gc, hid);
-      bool dead = false, out_of_cone;
-      if (i < all_c) {
-        compton_kn(cp.e, gc, &bc, a, b, c);
-        // (below the energy cut the copy dies in compton_finish)
-        dead = a * cp.e < s.e_min;
-        out_of_cone = !dead && s.ss_cos > R<real>(-1) && !cone_reachable(s, cp.run, cp.dir, R<real>(1) - b, c, s.ss_cos);
+
+  const uint64_t n_warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  // ---- Compton requests, `batch` at a time (fewer when there are not enough for all warps)
+  const uint32_t per = (uint32_t)s.ss_nc;
+  const uint32_t batch = (uint32_t)min((uint64_t)kSplitBatch, max(n_c / n_warps, (uint64_t)1));
+  const uint32_t step_r = per ? 32u / per : 0u, step_c = per ? 32u % per : 0u;  // 32 copies on
+  for (uint64_t r0 = warp * batch; per && r0 < n_c; r0 += n_warps * batch) {
+    const uint32_t nb = (uint32_t)min((uint64_t)batch, n_c - r0);
+    if (lane < nb) {
+      const uint64_t r = r0 + lane;
+      const uint64_t hid = sq.hid[r];
+      const real d[3] = {sq.dx[r], sq.dy[r], sq.dz[r]};
+      const KleinNishina<real> kn(sq.e[r]);
+      TrialFilter f;
+      f.k = (float)kn.k;
+      f.eps0sq = (float)kn.eps0sq;
+      f.alpha1 = (float)kn.alpha1;
+      f.alpha2 = (float)kn.alpha2;
+      f.e = (float)sq.e[r];
+      f.tol = 4e-6f * (2.0f + 1.0f / f.k);
+      const int run = sq.run[r];
+      real t1[3] = {R<real>(1), R<real>(0), R<real>(0)}, t2[3] = {R<real>(0), R<real>(1), R<real>(0)};
+      const real pp = gg_sqrt(d[0] * d[0] + d[1] * d[1]);
+      if (pp > R<real>(1e-4)) {
+        t1[0] = d[0] * d[2] / pp;
+        t1[1] = d[1] * d[2] / pp;
+        t1[2] = -pp;
+        t2[0] = -d[1] / pp;
+        t2[1] = d[0] / pp;
       } else {
-        set_energy(s, cp, cp.e);
-        a = rayleigh_cost(s, sq.comp[r], cp, gc, &bc);
-        out_of_cone = s.ss_cos > R<real>(-1) && !cone_reachable(s, cp.run, cp.dir, a, rayleigh_sint2(a), s.ss_cos);
+        f.tol = 4.0f;  // (along z: rounding of the frame counts; the exact trial decides)
       }
-      if (out_of_cone) {  // a live copy that fails the head checks, as counted there
-        ++n_world;
-        atomicAdd(&bc.escaped, 1u);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {  // (one head: twice the same)
+        const HeadFrame<real> fr = head_frame(s, run, h < s.n_heads ? h : 0);
+        f.c0[h] = (float)dot3(d, fr.u);
+        f.a1[h] = (float)dot3(t1, fr.u);
+        f.a2[h] = (float)dot3(t2, fr.u);
       }
-      wait = !dead && !out_of_cone;
+      P.f[lane] = f;
+      P.h0[lane] = (uint32_t)hid;
+      P.h1[lane] = (uint32_t)(hid >> 32);
+      P.stream[lane] = 2u + sq.base[r];
     }
-    const unsigned m = __ballot_sync(0xffffffffu, wait);
-    if (wait) {
-      const int k = np + __popc(m & lt_mask);
-      P.i[k] = i;
-      P.a[k] = a;
-      P.b[k] = b;
-      P.c[k] = c;
-      P.words[k] = (gc.blk - 1u) * 4u + (uint32_t)gc.idx;  // (the loops drew at least one word)
-    }
-    np += __popc(m);
     __syncwarp();
-    if (np >= 32) {
-      finish(np - 32, 32);
-      np -= 32;
+    const uint32_t total = nb * per;
+    uint32_t next = 0;                               // copies not begun
+    uint32_t fr = lane / per, fc = lane - fr * per;  // request and copy of copy next + lane
+    int nr = 0, no = 0;                              // copies waiting in P.retry, P.open (the same in every lane)
+    for (;;) {
+      const bool last = next >= total;
+      if (no >= 32 || (last && nr == 0)) {
+        // ---- a round of exact trials
+        if (no == 0) break;
+        const int n = min(no, 32);
+        no -= n;
+        bool live = false, again = false;
+        uint32_t id = 0, w3 = 0;
+        Photon<real> cp;
+        Rng g;
+        uint64_t hid = 0;
+        if ((int)lane < n) {
+          id = P.open[no + (int)lane];
+          const uint32_t t = id >> 20, r = (id & 0xfffffu) / per;
+          hid = load_copy((size_t)(r0 + r), (id & 0xfffffu) - r * per, s.ss_nc, cp, g);
+          // the stream after 3t words: the state an Rng reaches by drawing them
+          const uint32_t p = 3u * t;
+          if ((p & 3u) == 0u) {
+            g.blk = p >> 2;
+          } else {
+            const uint4 b = philox_block(p >> 2, g.stream, g.h0, g.h1, g.k0, g.k1);
+            g.buf[0] = b.x;
+            g.buf[1] = b.y;
+            g.buf[2] = b.z;
+            g.buf[3] = b.w;
+            g.blk = (p >> 2) + 1u;
+            g.idx = (int)(p & 3u);
+          }
+          const KleinNishina<real> kn(cp.e);
+          real eps, onecost, sint2;
+          bool done = kn.trial(g, eps, onecost, sint2);
+          w3 = g.buf[3];  // (after a first trial: word 3)
+          if (!done && t + 1u >= (uint32_t)kLoopCap) {
+            atomicAdd(&bc.loop_capped, 1u);
+            done = true;
+          }
+          again = !done;
+          id += 1u << 20;
+          if (done && !(eps * cp.e < s.e_min)) {  // (below the energy cut the copy dies)
+            live = !check || cone_reachable(s, cp.run, cp.dir, R<real>(1) - onecost, sint2, s.ss_cos);
+            if (live) {
+              scatter_dir(cp, g, R<real>(1) - onecost, sint2);
+              cp.e = eps * cp.e;  // (the walk kernel sets its energy-grid state)
+            } else {              // a live copy that fails the head checks, as counted there
+              ++n_world;
+              ++n_esc;
+            }
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, again);
+        if (again) {
+          P.retry[nr + __popc(m & lt_mask)] = id;
+          P.word3[nr + __popc(m & lt_mask)] = w3;
+        }
+        nr += __popc(m);
+        to_walk(live, cp, g, hid);
+        __syncwarp();
+        continue;
+      }
+      // ---- a round of filtered trials: of rejected copies when 32 wait (or no other is left), else first ones
+      bool on;
+      uint32_t r = 0, c = 0, t = 0, w3 = 0;
+      if (nr >= 32 || last) {
+        const int n = min(nr, 32);
+        nr -= n;
+        on = (int)lane < n;
+        if (on) {
+          const uint32_t id = P.retry[nr + (int)lane];
+          w3 = P.word3[nr + (int)lane];
+          t = id >> 20;
+          r = (id & 0xfffffu) / per;
+          c = (id & 0xfffffu) - r * per;
+        }
+      } else {
+        on = next + lane < total;
+        r = on ? fr : 0u;
+        c = fc;
+        next += 32u;
+        fr += step_r;
+        fc += step_c;
+        if (fc >= per) fc -= per, ++fr;
+      }
+      __syncwarp();
+      int res = kTrialDropped;
+      if (on) {
+        TrialWords g;
+        g.draw(t, w3, P.stream[r] + c, P.h0[r], P.h1[r], k0, k1);
+        w3 = g.w[3];
+        res = P.f[r](g.w, e_min, cos_min, check);
+        if (res == kTrialRejected && t + 1u >= (uint32_t)kLoopCap) res = kTrialUnsure;
+        if (res == kTrialMissed) {  // a live copy that fails the head checks, as counted there
+          ++n_world;
+          ++n_esc;
+        }
+      }
+      const unsigned mr = __ballot_sync(0xffffffffu, res == kTrialRejected);
+      const unsigned mo = __ballot_sync(0xffffffffu, res == kTrialUnsure);
+      const uint32_t id = (r * per + c) | (t << 20);
+      if (res == kTrialRejected) {
+        P.retry[nr + __popc(mr & lt_mask)] = id + (1u << 20);
+        P.word3[nr + __popc(mr & lt_mask)] = w3;
+      }
+      if (res == kTrialUnsure) P.open[no + __popc(mo & lt_mask)] = id;
+      nr += __popc(mr);
+      no += __popc(mo);
       __syncwarp();
     }
   }
-  if (np > 0) finish(0, np);
+  // ---- Rayleigh requests: one thread per copy (their copies are few)
+  const uint64_t per_r = (uint64_t)s.ss_nr, all_r = n_r * per_r;
+  for (uint64_t i0 = warp * 32u; i0 < all_r; i0 += n_warps * 32u) {
+    const uint64_t i = i0 + lane;
+    bool live = false;
+    Photon<real> cp;
+    Rng g;
+    uint64_t hid = 0;
+    if (i < all_r) {
+      const uint64_t req = i / per_r;
+      const size_t r = q.split_cap - 1 - (size_t)req;
+      hid = load_copy(r, (uint32_t)(i - req * per_r), s.ss_nr, cp, g);
+      cp.ei = energy_index(s, cp.e);
+      const real cost = rayleigh_cost(s, sq.comp[r], cp, g, &bc);
+      live = !check || cone_reachable(s, cp.run, cp.dir, cost, rayleigh_sint2(cost), s.ss_cos);
+      if (live) {
+        rayleigh_finish(cp, g, cost);
+      } else {
+        ++n_world;
+        ++n_esc;
+      }
+    }
+    to_walk(live, cp, g, hid);
+  }
+  if (n_esc) atomicAdd(&bc.escaped, n_esc);
   stage_counters(args.counters, bc, lane, 0u, 0u, n_world, 0u, 0u);
 }
 
@@ -900,15 +1101,13 @@ cudaError_t spect_head_occupancy(int block, size_t smem, int minb, int *bps) {
 }
 
 template <typename real>
-cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int block, size_t smem,
-                               int n_sm, cudaStream_t st) {
-  static unsigned long long configured = 0;
-  cudaError_t e = configure_smem(k_spect_split<real>, 200 * 1024, configured);
+cudaError_t launch_spect_split(const Scene<real> &s, const KernelArgs &a, const StageArgs &q, int n_sm,
+                               cudaStream_t st) {
   int bps = 1;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_spect_split<real>, block, smem);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_spect_split<real>, kBlock, 0);
   if (e != cudaSuccess) return e;
   if (bps < 1) bps = 1;
-  k_spect_split<real><<<n_sm * bps, block, smem, st>>>(s, a, q);
+  k_spect_split<real><<<n_sm * bps, kBlock, 0, st>>>(s, a, q);
   return cudaGetLastError();
 }
 
@@ -932,9 +1131,9 @@ template cudaError_t launch_spect_walk<double>(const Scene<double> &, const Kern
 template size_t split_bytes<float>(size_t);
 template size_t split_bytes<double>(size_t);
 template cudaError_t launch_spect_split<float>(const Scene<float> &, const KernelArgs &, const StageArgs &, int,
-                                               size_t, int, cudaStream_t);
+                                               cudaStream_t);
 template cudaError_t launch_spect_split<double>(const Scene<double> &, const KernelArgs &, const StageArgs &, int,
-                                                size_t, int, cudaStream_t);
+                                                cudaStream_t);
 template size_t queue_bytes<float>(size_t);
 template size_t queue_bytes<double>(size_t);
 template size_t phantom_slot_bytes<float>();
