@@ -5,6 +5,8 @@
 // fixed-point tallies and the float64 edep / edep-squared images.  Host
 // buffers passed in are copied; nothing is retained past a call.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -13,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/gate_gpu.h"
@@ -24,6 +27,44 @@
 namespace {
 
 std::string g_create_error;
+
+// Makes the pages of a large output buffer that are not there yet, by several
+// threads, before a copy to it: a copy takes one page fault after the other (94 MB
+// of fresh pages 5.0 ms, 3.1 ms after this; four threads touch them in 0.9 ms, more
+// are no faster).  The whole range is about to
+// be overwritten.  A buffer whose pages are present is left alone, and so is one
+// below kPrefaultMin, where starting threads costs more than the faults.
+constexpr size_t kPrefaultMin = (size_t)16 << 20;
+
+void prefault(void *out, size_t bytes) noexcept {
+  if (bytes < kPrefaultMin) return;
+  try {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = ((uintptr_t)out + page - 1) / page * page, hi = ((uintptr_t)out + bytes) / page * page;
+    if (hi <= lo) return;
+    const size_t n = (hi - lo) / page;
+    std::vector<unsigned char> present(n);
+    if (mincore((void *)lo, hi - lo, present.data()) != 0) return;
+    size_t missing = 0;
+    for (unsigned char p : present) missing += (p & 1u) ? 0 : 1;
+    if (missing * page < kPrefaultMin / 2) return;
+    const size_t threads = std::min<size_t>(4, std::max(1u, std::thread::hardware_concurrency()));
+    auto touch = [&](size_t t) {
+      for (size_t i = t; i < n; i += threads)
+        if (!(present[i] & 1u)) *(volatile unsigned char *)(lo + i * page) = 0;
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(threads);
+    size_t started = 1;
+    try {
+      for (; started < threads; ++started) pool.emplace_back(touch, started);
+    } catch (...) {  // (no more threads: the copy takes the remaining faults)
+    }
+    touch(0);
+    for (auto &t : pool) t.join();
+  } catch (...) {
+  }
+}
 
 template <typename T>
 void dfree(T *&p) {
@@ -209,6 +250,7 @@ struct gg_ctx {
     return st ? st : cuda(cudaStreamSynchronize(stream), what);
   }
   int d2h(void *dst, const void *src, size_t bytes, const char *what) {
+    prefault(dst, bytes);
     int st = cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream), what);
     return st ? st : cuda(cudaStreamSynchronize(stream), what);
   }
@@ -1544,9 +1586,7 @@ int gg_get_image(gg_ctx *c, int32_t which, double *out, size_t n) {
   else if (which == GG_IMG_DOSE) src = c->dgrid_on && c->ddose ? c->d_dose : nullptr;
   else if (which == GG_IMG_DOSE_SQUARED) src = c->dgrid_on && c->ddose && c->squared ? c->d_dose2 : nullptr;
   if (!src) return c->fail(GG_ERR_ARG, "gg_get_image: image %d not scored", which);
-  int st = c->cuda(cudaMemcpyAsync(out, src, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "download");
-  if (st) return st;
-  return c->cuda(cudaStreamSynchronize(c->stream), "download");
+  return c->d2h(out, src, n * sizeof(double), "download");
 }
 
 int gg_get_image_device(gg_ctx *c, int32_t which, void **ptr, size_t *n) {

@@ -301,11 +301,12 @@ class ArfNetwork:
         return a
 
     def dataset(self, sampling, n, seed, first=0):
-        rows = np.zeros((max(n, 1), 4), dtype=np.float32)
+        rows = np.empty((max(n, 1), 4), dtype=np.float32)
         m = ctypes.c_uint64()
         self.eng._call("gg_arf_dataset", ctypes.byref(sampling), ctypes.c_uint64(n), ctypes.c_uint64(seed),
                        ctypes.c_uint64(first), C.ptr(rows, ctypes.c_float), ctypes.c_uint64(n), ctypes.byref(m))
-        return rows[: m.value].copy()
+        # (every sample kept: no second array)
+        return rows if m.value == len(rows) else rows[: m.value].copy()
 
     def train(self, sampling, n_samples, seed, epochs=4, batch=8192, lr=1e-3, init_seed=1, beta1=0.9,
               beta2=0.999, eps=1e-8, lr_final=None):
@@ -356,7 +357,7 @@ class ArfNetwork:
 
     def predict(self, rows):
         rows = np.ascontiguousarray(rows, dtype=np.float32)
-        out = np.zeros((len(rows), self.model.n_classes), dtype=np.float32)
+        out = np.empty((len(rows), self.model.n_classes), dtype=np.float32)
         self.eng._call("gg_arf_predict", C.ptr(rows, ctypes.c_float), ctypes.c_uint64(len(rows)),
                        C.ptr(out, ctypes.c_float))
         return out
