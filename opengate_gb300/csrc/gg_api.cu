@@ -1870,7 +1870,7 @@ int gg_arf_gradient(gg_ctx *c, const float *rows, uint64_t n, float *grad, doubl
   a.row0 = 0;
   a.n_rows = n;
   a.inv_batch = 1.0f / (float)n;
-  if ((st = c->cuda(gg::launch_mlp_train(a, tiles, c->stream), "ARF gradient"))) return st;
+  if ((st = c->cuda(gg::launch_mlp_train(a, tiles, false, c->stream), "ARF gradient"))) return st;
   gg::MlpAdamArgs g{};
   g.partial = c->d_partial;
   g.n_tiles = tiles;
@@ -1878,7 +1878,7 @@ int gg_arf_gradient(gg_ctx *c, const float *rows, uint64_t n, float *grad, doubl
   g.wbf = c->d_wbf;
   g.grad_out = c->d_grad;
   g.lr = 0.0f;
-  if ((st = c->cuda(gg::launch_mlp_adam(g, c->stream), "ARF gradient sum"))) return st;
+  if ((st = c->cuda(gg::launch_mlp_adam(g, false, c->stream), "ARF gradient sum"))) return st;
   std::vector<float> lp(tiles);
   if ((st = c->d2h(grad, c->d_grad, gg::kNParams * sizeof(float), "download")))
     return st;
@@ -1966,13 +1966,6 @@ int gg_arf_train_rows(gg_ctx *c, const float *rows, uint64_t n_rows, const gg_ar
       !(domain->theta_max_deg <= 90.0) || !(domain->russian_roulette >= 1.0))
     return c->fail(GG_ERR_ARG, "gg_arf_train_rows: domain needs 0 < e_min < e_max, 0 < theta_max <= 90, rr >= 1");
   const int n_classes = c->spect.n_windows + 1;
-  for (uint64_t i = 0; i < n_rows; ++i) {
-    const float *r = rows + 4 * i;
-    if (!std::isfinite(r[0]) || !std::isfinite(r[1]) || !std::isfinite(r[2]) || !(r[3] >= 0.0f) ||
-        !(r[3] < (float)n_classes) || r[3] != std::floor(r[3]))
-      return c->fail(GG_ERR_ARG, "gg_arf_train_rows: row %llu: non-finite input or class outside [0, %d)",
-                     (unsigned long long)i, n_classes);
-  }
   if (n_rows > c->arf_rows_cap) {
     dfree(c->d_arf_rows);
     c->arf_rows_cap = 0;
@@ -1980,6 +1973,15 @@ int gg_arf_train_rows(gg_ctx *c, const float *rows, uint64_t n_rows, const gg_ar
     c->arf_rows_cap = n_rows;
   }
   if ((st = c->h2d(c->d_arf_rows, rows, n_rows * sizeof(float4), "upload ARF rows"))) return st;
+  // (checked on the device: on the host the rows cost more than the upload)
+  if ((st = c->cuda(cudaMemsetAsync(c->d_next, 0xff, sizeof(unsigned long long), c->stream), "memset"))) return st;
+  if ((st = c->cuda(gg::launch_check_rows(c->d_arf_rows, n_rows, n_classes, c->d_next, c->n_sm, c->stream),
+                    "check ARF rows")))
+    return st;
+  unsigned long long bad = 0;
+  if ((st = c->d2h(&bad, c->d_next, sizeof(bad), "check ARF rows"))) return st;
+  if (bad != ~0ull)
+    return c->fail(GG_ERR_ARG, "gg_arf_train_rows: row %llu: non-finite input or class outside [0, %d)", bad, n_classes);
   const gg_arf_model m = arf_domain_model(c, domain->e_min, domain->e_max, domain->theta_max_deg,
                                           domain->russian_roulette);
   return arf_train_impl(c, n_rows, m, o, model_out, loss);
@@ -2016,15 +2018,20 @@ static int arf_train_impl(gg_ctx *c, uint64_t n_rows, const gg_arf_model &m, con
   const double total_steps = (double)steps_per_epoch * (double)o->epochs;
   const double decay = o->lr_final > 0.0f ? std::log((double)o->lr_final / (double)o->lr) : 0.0;
   uint64_t t = 0;
+  // overlapped launches: each kernel sets itself up while the one before ends, 5 us a step, as
+  // long as the last wave of tiles (one per SM, all its registers) leaves SMs free: 64 tiles
+  // 28.8 -> 23.9 us a step, 128 32.9 -> 31.9, 512 114 -> 109; but 152 34.9 -> 45.1, 304 64 -> 83
+  const int rem = tiles % c->n_sm;
+  const bool overlap = rem != 0 && 8 * rem <= 7 * c->n_sm;
   for (int ep = 0; ep < o->epochs; ++ep) {
     g.loss_acc = c->d_loss_acc + ep;
     for (uint64_t k = 0; k < steps_per_epoch; ++k, ++t) {
       a.row0 = (t * (uint64_t)o->batch) % n_rows;
-      if ((st = c->cuda(gg::launch_mlp_train(a, tiles, c->stream), "ARF train step"))) return st;
+      if ((st = c->cuda(gg::launch_mlp_train(a, tiles, overlap, c->stream), "ARF train step"))) return st;
       g.lr = (float)((double)o->lr * std::exp(decay * (double)t / total_steps));
       g.c1 = (float)(1.0 / (1.0 - std::pow((double)o->beta1, (double)(t + 1))));
       g.c2 = (float)(1.0 / (1.0 - std::pow((double)o->beta2, (double)(t + 1))));
-      if ((st = c->cuda(gg::launch_mlp_adam(g, c->stream), "ARF Adam step"))) return st;
+      if ((st = c->cuda(gg::launch_mlp_adam(g, overlap, c->stream), "ARF Adam step"))) return st;
     }
   }
   std::vector<double> lacc(o->epochs);

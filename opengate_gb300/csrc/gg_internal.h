@@ -30,6 +30,23 @@ inline cudaError_t configure_smem(K kernel, int bytes, unsigned long long &done)
   return e;
 }
 
+// Launch of a kernel that may start (overlap) while the stream's previous kernel ends: it
+// calls cudaGridDependencySynchronize() before it touches that kernel's data.
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(bool overlap, void (*kernel)(P...), int grid, int block, size_t smem,
+                                     cudaStream_t st, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
 
 template <typename real>
 struct Scene;
@@ -93,7 +110,7 @@ struct MlpTrainArgs {
   uint64_t row0, n_rows;         // tile t reads rows (row0 + 128 t + r) % n_rows
   const float *params;           // FP32 parameters
   const __nv_bfloat16 *wbf;      // BF16 copies of W2, W3, W4
-  float *partial;                // [tiles][kNParams] gradient of each tile
+  float *partial;                // [tiles][kNParams] gradient of each tile (param_of_partial order)
   float *loss_part;              // [tiles] loss sum of each tile
   float mean[3], inv_std[3];     // standardisation of (theta, phi, E)
   int n_classes;
@@ -108,7 +125,7 @@ struct MlpAdamArgs {
   int n_tiles;
   float *params;
   __nv_bfloat16 *wbf;
-  float *m, *v;                  // Adam moments
+  float *m, *v;                  // Adam moments (param_of_partial order)
   float *grad_out;               // summed gradient (or null)
   float lr, beta1, beta2, eps;   // lr = 0: gradient only, no update
   float c1, c2;                  // 1 / (1 - beta1^t), 1 / (1 - beta2^t)
@@ -139,8 +156,11 @@ struct ArfStageArgs {
 };
 
 size_t mlp_train_smem_bytes();
-cudaError_t launch_mlp_train(const MlpTrainArgs &a, int n_tiles, cudaStream_t st);
-cudaError_t launch_mlp_adam(const MlpAdamArgs &a, cudaStream_t st);
+cudaError_t launch_mlp_train(const MlpTrainArgs &a, int n_tiles, bool overlap, cudaStream_t st);
+cudaError_t launch_mlp_adam(const MlpAdamArgs &a, bool overlap, cudaStream_t st);
+// *bad = number of the first invalid training row, if below its value
+cudaError_t launch_check_rows(const float4 *rows, uint64_t n, int n_classes, unsigned long long *bad, int n_sm,
+                              cudaStream_t st);
 cudaError_t launch_mlp_to_bf16(const float *params, __nv_bfloat16 *wbf, cudaStream_t st);
 size_t mlp_tc_smem_bytes();
 cudaError_t launch_mlp_predict(const MlpTrainArgs &a, float *out, uint64_t n, int grid, unsigned int *status,

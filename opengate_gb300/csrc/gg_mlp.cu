@@ -21,28 +21,69 @@
 
 namespace gg {
 
-// Sum of the tile gradients (tile order) and one Adam step; refreshes the BF16 copies.
-__global__ void k_mlp_adam(MlpAdamArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p == 0 && a.loss_acc) {
+// Sum of the tile gradients (tile order) and one Adam step; refreshes the BF16
+// copies.  The last block adds the tiles' losses (tile order) instead.  Bound by
+// the latency of the tile loads: 64 tiles, cold cache, 11.4 -> 8.4 us with 16 of
+// them in flight per thread and the loss off the parameters' path.
+constexpr int kAdamThreads = 128;
+constexpr int kAdamBlocks = (kNParams + kAdamThreads - 1) / kAdamThreads;
+
+__global__ void __launch_bounds__(kAdamThreads) k_mlp_adam(MlpAdamArgs a) {
+  cudaTriggerProgrammaticLaunchCompletion();  // (the next step's kernel may set itself up)
+  cudaGridDependencySynchronize();            // the tile gradients
+  if (blockIdx.x == kAdamBlocks) {
+    if (!a.loss_acc || threadIdx.x >= 32) return;
     double s = 0.0;
-    for (int t = 0; t < a.n_tiles; ++t) s += (double)a.loss_part[t];
-    *a.loss_acc += s;
+    for (int t0 = 0; t0 < a.n_tiles; t0 += 32) {
+      const int t = t0 + (int)threadIdx.x, n = min(32, a.n_tiles - t0);
+      const float l = t < a.n_tiles ? a.loss_part[t] : 0.0f;
+      for (int k = 0; k < n; ++k) s += (double)__shfl_sync(0xffffffffu, l, k);
+    }
+    if (threadIdx.x == 0) *a.loss_acc += s;
+    return;
   }
-  if (p >= kNParams) return;
+  const int q = blockIdx.x * kAdamThreads + threadIdx.x;  // in the tile gradients' order, as the moments
+  if (q >= kNParams) return;
+  const int p = param_of_partial(q);
+  const bool update = a.lr != 0.0f;  // (else: gradient only)
+  float m = 0.0f, v = 0.0f, w0 = 0.0f;
+  if (update) {
+    m = a.m[q];
+    v = a.v[q];
+    w0 = a.params[p];
+  }
   float g = 0.0f;
-  for (int t = 0; t < a.n_tiles; ++t) g += a.partial[(size_t)t * kNParams + p];
+  const float *part = a.partial + q;
+  int t = 0;
+  for (; t + 16 <= a.n_tiles; t += 16) {
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = part[(size_t)(t + i) * kNParams];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) g += x[i];
+  }
+  for (; t < a.n_tiles; ++t) g += part[(size_t)t * kNParams];
   if (a.grad_out) a.grad_out[p] = g;
-  if (a.lr == 0.0f) return;  // gradient only
-  float m = a.m[p], v = a.v[p];
+  if (!update) return;
   m = a.beta1 * m + (1.0f - a.beta1) * g;
   v = a.beta2 * v + (1.0f - a.beta2) * g * g;
-  a.m[p] = m;
-  a.v[p] = v;
+  a.m[q] = m;
+  a.v[q] = v;
   const float mh = m * a.c1, vh = v * a.c2;
-  const float w = a.params[p] - a.lr * mh / (sqrtf(vh) + a.eps);
+  const float w = w0 - a.lr * mh / (sqrtf(vh) + a.eps);
   a.params[p] = w;
   bf16_store_weight(a.wbf, p, w);
+}
+
+// The first row (E, theta, phi, class) that is not finite or whose class is not
+// a whole number in [0, n_classes): its number into *bad (atomicMin).
+__global__ void __launch_bounds__(256) k_check_rows(const float4 *rows, uint64_t n, float n_classes,
+                                                    unsigned long long *bad) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const float4 r = rows[i];
+    const bool ok = isfinite(r.x) && isfinite(r.y) && isfinite(r.z) && r.w >= 0.0f && r.w < n_classes && r.w == floorf(r.w);
+    if (!ok) atomicMin(bad, (unsigned long long)i);
+  }
 }
 
 // BF16 copies of W2 / W3 / W4 from the FP32 parameters.
@@ -88,8 +129,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   tc_net_teardown(sm);
 }
 
-cudaError_t launch_mlp_adam(const MlpAdamArgs &a, cudaStream_t st) {
-  k_mlp_adam<<<(kNParams + 255) / 256, 256, 0, st>>>(a);
+cudaError_t launch_mlp_adam(const MlpAdamArgs &a, bool overlap, cudaStream_t st) {
+  return launch_overlapped(overlap, k_mlp_adam, kAdamBlocks + 1, kAdamThreads, 0, st, a);
+}
+
+cudaError_t launch_check_rows(const float4 *rows, uint64_t n, int n_classes, unsigned long long *bad, int n_sm,
+                              cudaStream_t st) {
+  k_check_rows<<<n_sm * 4, 256, 0, st>>>(rows, n, (float)n_classes, bad);
   return cudaGetLastError();
 }
 

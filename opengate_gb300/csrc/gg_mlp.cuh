@@ -32,6 +32,17 @@ constexpr int kOffW4 = kOffB3 + kHid;            // [16][128] (rows >= n_classes
 constexpr int kOffB4 = kOffW4 + kOutPad * kHid;  // [16]
 constexpr int kNParams = kOffB4 + kOutPad;       // 35600
 
+// Tile gradients (MlpTrainArgs::partial) and Adam moments keep W2 and W3 as [in]
+// [out]: thread `out` of the training kernel reads one row of dW from tensor
+// memory, and its stores of one column are contiguous over the lanes.  The
+// parameter of entry q:
+__host__ __device__ constexpr int param_of_partial(int q) {
+  const int off = q >= kOffW2 && q < kOffB2 ? kOffW2 : (q >= kOffW3 && q < kOffB3 ? kOffW3 : -1);
+  if (off < 0) return q;
+  const int i = (q - off) / kHid, o = (q - off) % kHid;
+  return off + o * kHid + i;
+}
+
 // BF16 weight copies used by the tensor cores: W2, W3, W4 back to back,
 // row-major [out][in] (the training kernel's ldmatrix operands), then the same
 // three matrices again as 5th-generation tensor-core operands (K-major core
