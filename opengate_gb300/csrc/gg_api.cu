@@ -1329,12 +1329,9 @@ static int spect_stages(gg_ctx *c, gg::KernelArgs a, const gg::PoolPlan &plan, s
 static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool capturing = false) {
   size_t smem = c->precision == GG_PREC_F64 ? gg::transport_smem_bytes<double>(c->n_comp, c->n_e, c->n_mat)
                                             : gg::transport_smem_bytes<float>(c->n_comp, c->n_e, c->n_mat);
-  // kernel variant (SPECT stages, track-length estimator): register budget for `minb` resident
-  // 256-thread blocks; the estimator's voxel walks: 3 (80 registers: 34.3 ms per 1e7 pencil
-  // primaries against 36.5 at 4 blocks / SM)
   const bool tle_run = c->tle && !c->have_spect && !c->have_batch;
-  int minb = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, 4)
-                                  : (c->precision == GG_PREC_F64 ? 2 : (tle_run ? 3 : 4));
+  // SPECT head stage: register budget for `minb` resident 256-thread blocks
+  int minb = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, 4) : (c->precision == GG_PREC_F64 ? 2 : 4);
   // the compacted wavefront kernel: single dose simulations with analog scoring
   if (c->dgrid_on && c->tle && !c->have_spect && !c->have_batch)
     return c->fail(GG_ERR_STATE, "gg_run: the track-length estimator scores on the image grid (no dose grid)");
@@ -1381,26 +1378,20 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     if (st) return st;
     c->rec_cap = cap;
   }
-  // launch shape of the dose transport: the pooled kernel, or the estimator's persistent grid
+  // launch shape of the pooled transport
   gg::PoolPlan plan{};
-  int tle_grid = 0;
-  if (tle_run) {
-    int bps = 0;
-    cudaError_t e = c->precision == GG_PREC_F64 ? gg::tle_occupancy<double>(c->block, smem, minb, &bps)
-                                                : gg::tle_occupancy<float>(c->block, smem, minb, &bps);
-    if (e != cudaSuccess) return c->cuda(e, "occupancy");
-    tle_grid = c->n_sm * std::max(bps, 1);
-  } else if (!wave) {
+  if (!wave) {
     const bool f64 = c->precision == GG_PREC_F64, sp = c->have_spect;
     const bool two = c->dgrid_on && c->ddose && !c->have_batch && !sp;
+    const int queues = tle_run ? 5 : 4;  // (the estimator's walks are events of their own)
     const int pool_threads = c->block == gg::kBlock ? 0 : c->block;  // (the default: the kernel's own block size)
     cudaError_t e =
         f64 ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
-                                    sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(),
-                                    gg::slot_scratch_bytes<double>(two), &plan)
+                                    sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(tle_run),
+                                    gg::slot_scratch_bytes<double>(two), queues, &plan)
             : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
-                                   sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(),
-                                   gg::slot_scratch_bytes<float>(two), &plan);
+                                   sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(tle_run),
+                                   gg::slot_scratch_bytes<float>(two), queues, &plan);
     if (e != cudaSuccess) return c->cuda(e, "transport launch shape");
     if (plan.scratch > c->slot_bytes) {
       dfree(c->d_slot);
@@ -1485,13 +1476,8 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
               : gg::launch_wavefront<float>(c->scene<float>(), a, wgrid, wsmem, wminb, c->stream);
       if ((st = c->cuda(e, "wavefront transport launch"))) return st;
     } else {
-      if (tle_run)
-        e = c->precision == GG_PREC_F64
-                ? gg::launch_transport_tle<double>(c->scene<double>(), a, tle_grid, c->block, smem, minb, c->stream)
-                : gg::launch_transport_tle<float>(c->scene<float>(), a, tle_grid, c->block, smem, minb, c->stream);
-      else
-        e = c->precision == GG_PREC_F64 ? gg::launch_transport<double>(c->scene<double>(), a, plan, c->stream)
-                                        : gg::launch_transport<float>(c->scene<float>(), a, plan, c->stream);
+      e = c->precision == GG_PREC_F64 ? gg::launch_transport<double>(c->scene<double>(), a, plan, c->stream)
+                                      : gg::launch_transport<float>(c->scene<float>(), a, plan, c->stream);
       if ((st = c->cuda(e, "transport launch"))) return st;
     }
     if (!capturing && (st = c->cuda(cudaEventRecord(c->ev[3 * b + 2], c->stream), "event"))) return st;

@@ -207,19 +207,19 @@ template <>
 struct PoolShape<double> {
   static constexpr int kBlock = 288, kGang = 3, kRing = 512;
 };
-// static shared memory of a pooled kernel, at most
+// static shared memory of a pooled kernel with as many event queues, at most
 template <typename real>
-__host__ __device__ constexpr int pool_static() {
+__host__ __device__ constexpr int pool_static(int queues) {
   using P = PoolShape<real>;
-  return 1024 + 16 * P::kBlock + (P::kBlock / (32 * P::kGang)) * (8 * P::kRing + 64);
+  return 1024 + 16 * P::kBlock + (P::kBlock / (32 * P::kGang)) * (2 * queues * P::kRing + (queues > 4 ? 112 : 64));
 }
 template <typename real>
 cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
-                      size_t scratch_bytes, PoolPlan *p);
+                      size_t scratch_bytes, int queues, PoolPlan *p);
 int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist);
-// Shared memory of a dose slot; its global scratch (two: the second list of a dose grid).
+// Shared memory of a dose slot (tle: with the track-length estimator); its global scratch (two: the second list of a dose grid).
 template <typename real>
-size_t dose_slot_bytes();
+size_t dose_slot_bytes(bool tle);
 template <typename real>
 size_t slot_scratch_bytes(bool two);
 // Rows of p.n samples appended to rows[*total ...] (capacity rows); *total advances on the device.
@@ -262,12 +262,6 @@ template <typename real>
 cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStream_t st);
 template <typename real>
 cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st);
-// track-length estimator; minb selects the kernel variant compiled for that many resident blocks per SM
-template <typename real>
-cudaError_t launch_transport_tle(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem, int minb,
-                                 cudaStream_t st);
-template <typename real>
-cudaError_t tle_occupancy(int block, size_t smem, int minb, int *blocks_per_sm);
 // Compacted wavefront dose transport (gg_wavefront.cu): 256-thread blocks,
 // dynamic shared memory = tables + photon slots.
 template <typename real>

@@ -897,29 +897,71 @@ __device__ __forceinline__ void voxel_walk(const Scene<real> &s, const real p[3]
   }
 }
 
-// Label gathers in flight per lane in the track-length estimator's walks.
-constexpr int kTleGroup = 2;
+// One straight path through the voxels, boundary by boundary (voxel_walk's
+// arithmetic, step for step): next boundary and boundary spacing per axis,
+// path so far, voxel.
+template <typename real>
+struct VoxelWalk {
+  real tn[3], td[3], tc;
+  int i[3], k;
 
-template <typename real, int GROUP, typename Visit>
-__device__ __forceinline__ void voxel_walk_grouped(const Scene<real> &s, const real p[3], const real d[3], real len,
-                                                   Visit &&visit);
-
-// Track-length estimator (GateTLEDoseActor::ScoreTLEDepositStep,
-// core/opengate_core/opengate_lib/GateTLEDoseActor.cpp:249-299): the straight
-// path [p, p + len d) of a photon of energy e (table index ei) scores
-// e * mu_en(E, material) * length in every voxel it crosses.
-template <typename real, int GROUP = kTleGroup>
-__device__ __forceinline__ void tle_path(const Scene<real> &s, const real p[3], const real d[3], real len, real e,
-                                         const EIdx<real> &ei, HistList<real> &l, const Tally<real> &t,
-                                         BlockCounters *bc, unsigned int &n_dep) {
-  voxel_walk_grouped<real, GROUP>(s, p, d, len, [&](uint32_t v, int m, real seg) {
-    real mu = interp_row(s.muen + (size_t)s.mat_comp[m] * s.n_e, ei);
-    mu = s.mat_rho[m] * mu;
-    real ed = e * mu;
-    ed = ed * seg;
-    deposit(l, t, bc, v, ed, n_dep);
-  });
-}
+  __device__ __forceinline__ void start(const Scene<real> &s, const real p[3], const real d[3]) {
+    const int n[3] = {s.nx, s.ny, s.nz};
+    const real inf = gg_inf(real(0));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      int ia = (int)((p[a] - s.bmin[a]) * s.inv_sp[a]);
+      ia = ia < 0 ? 0 : (ia >= n[a] ? n[a] - 1 : ia);
+      i[a] = ia;
+      tn[a] = td[a] = inf;
+      const real da = d[a];
+      if (da > R<real>(0)) {
+        real b = (real)(ia + 1) * s.sp[a];
+        b = s.bmin[a] + b;
+        b = b - p[a];
+        tn[a] = b / da;
+        td[a] = s.sp[a] / da;
+      } else if (da < R<real>(0)) {
+        real b = (real)ia * s.sp[a];
+        b = s.bmin[a] + b;
+        b = b - p[a];
+        tn[a] = b / da;
+        td[a] = -s.sp[a];
+        td[a] = td[a] / da;
+      }
+      if (tn[a] < R<real>(0)) tn[a] = R<real>(0);
+    }
+    tc = R<real>(0);
+    k = 0;
+  }
+  // Crosses one boundary (fewer than nx + ny + nz + 3 so far): the voxel and the path in it
+  // (none if not positive); false: the path of length len ends.
+  __device__ __forceinline__ bool step(const Scene<real> &s, const real d[3], real len, uint32_t &v, real &seg) {
+    int a = 0;
+    real tb = tn[0];
+    if (tn[1] < tn[0]) a = 1, tb = tn[1];
+    if (tn[2] < tb) a = 2, tb = tn[2];
+    const real te = tb < len ? tb : len;
+    seg = te - tc;
+    v = (uint32_t)i[0] + (uint32_t)s.nx * ((uint32_t)i[1] + (uint32_t)s.ny * (uint32_t)i[2]);
+    tc = te;
+    ++k;
+    if (!(tc < len)) return false;
+    const int n[3] = {s.nx, s.ny, s.nz};
+    bool in = true;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {  // (every axis' values, the crossed one's kept: no branch)
+      const int ib = i[b] + (d[b] > R<real>(0) ? 1 : (d[b] < R<real>(0) ? -1 : 0));
+      const real t = tn[b] + td[b];
+      if (a == b) {
+        i[b] = ib;
+        tn[b] = t;
+        in = ib >= 0 && ib < n[b];
+      }
+    }
+    return in && k < n[0] + n[1] + n[2] + 3;
+  }
+};
 
 // voxel_walk in groups of GROUP boundary crossings: the crossings of a group
 // are computed first (voxel_walk's arithmetic, step for step), then their
@@ -1044,61 +1086,51 @@ __device__ __forceinline__ real image_depth(const Scene<real> &s, const real p[3
   return tau;
 }
 
-// Scoring state handed to the flights of the track-length estimator.
-template <typename real>
-struct TleScore {
-  HistList<real> *l;
-  const Tally<real> *t;
-  unsigned int *n_dep;
-};
-
-// One Woodcock tentative step of a photon inside the image box.  With TLE, a
-// photon at or below the estimator's threshold first stops (depositing its
-// energy in its voxel) when at or below the kill energy, else scores the
-// path of the step.
-template <typename real, bool TLE = false, typename G = Rng>
-__device__ __forceinline__ int image_flight(const Scene<real> &s, Photon<real> &ph, G &g, int &pmat, uint32_t &pv,
-                                            int &pscored, unsigned int &n_wood, unsigned int &n_real,
-                                            BlockCounters *bc = nullptr, TleScore<real> sc = {nullptr, nullptr, nullptr}) {
-  {
-    if constexpr (TLE) {
-      if (ph.e <= s.tle_thr && ph.e <= s.tle_emin) {
-        deposit(*sc.l, *sc.t, bc, voxel_of(s, ph.pos), ph.e, *sc.n_dep);
-        ph.alive = 0;
-        return kRefill;
-      }
-    }
-    real u = u01_open0<real>(g);
-    real sd = -gg_log(u);
-    sd = sd * ph.inv_mumax;
-    if constexpr (TLE) {
-      if (ph.e <= s.tle_thr)
-        tle_path(s, ph.pos, ph.dir, sd < ph.t_exit ? sd : ph.t_exit, ph.e, ph.ei, *sc.l, *sc.t, bc, *sc.n_dep);
-    }
-    if (sd >= ph.t_exit) {
+// A photon inside the image box after a drawn path sd: it leaves the box (kFly,
+// not in the image), meets no real collision (kFly) or one (kInteract).
+template <typename real, typename G>
+__device__ __forceinline__ int image_arrive(const Scene<real> &s, Photon<real> &ph, G &g, real sd, int &pmat,
+                                            uint32_t &pv, int &pscored, unsigned int &n_wood, unsigned int &n_real) {
+  if (sd >= ph.t_exit) {
 #pragma unroll
-      for (int a = 0; a < 3; ++a) ph.pos[a] = ph.pos[a] + ph.t_exit * ph.dir[a];
-      ph.in_image = 0;
-      ph.can_enter = 0;
-      ph.exclude = 0;
-      return kFly;
-    }
-    ph.t_exit = ph.t_exit - sd;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) ph.pos[a] = ph.pos[a] + sd * ph.dir[a];
-    ++n_wood;
-    const uint32_t v = voxel_of(s, ph.pos);
-    int m = __ldg(s.labels + v);
-    real mu = interp_row(s.sig + (size_t)s.mat_comp[m] * s.n_e, ph.ei);
-    mu = s.mat_rho[m] * mu;
-    real u2 = u01<real>(g);
-    if (u2 * ph.mumax >= mu) return kFly;
-    ++n_real;
-    pmat = m;
-    pv = v;
-    pscored = 1;
-    return kInteract;
+    for (int a = 0; a < 3; ++a) ph.pos[a] = ph.pos[a] + ph.t_exit * ph.dir[a];
+    ph.in_image = 0;
+    ph.can_enter = 0;
+    ph.exclude = 0;
+    return kFly;
   }
+  ph.t_exit = ph.t_exit - sd;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) ph.pos[a] = ph.pos[a] + sd * ph.dir[a];
+  ++n_wood;
+  const uint32_t v = voxel_of(s, ph.pos);
+  int m = __ldg(s.labels + v);
+  real mu = interp_row(s.sig + (size_t)s.mat_comp[m] * s.n_e, ph.ei);
+  mu = s.mat_rho[m] * mu;
+  real u2 = u01<real>(g);
+  if (u2 * ph.mumax >= mu) return kFly;
+  ++n_real;
+  pmat = m;
+  pv = v;
+  pscored = 1;
+  return kInteract;
+}
+
+// The path to the next tentative collision in the image.
+template <typename real, typename G>
+__device__ __forceinline__ real woodcock_path(const Photon<real> &ph, G &g) {
+  real u = u01_open0<real>(g);
+  real sd = -gg_log(u);
+  sd = sd * ph.inv_mumax;
+  return sd;
+}
+
+// One Woodcock tentative step of a photon inside the image box.
+template <typename real, typename G = Rng>
+__device__ __forceinline__ int image_flight(const Scene<real> &s, Photon<real> &ph, G &g, int &pmat, uint32_t &pv,
+                                            int &pscored, unsigned int &n_wood, unsigned int &n_real) {
+  const real sd = woodcock_path(ph, g);
+  return image_arrive(s, ph, g, sd, pmat, pv, pscored, n_wood, n_real);
 }
 
 // One free flight in the world (dose path): to a collision in the world
@@ -1134,17 +1166,17 @@ __device__ __forceinline__ int dose_world_flight(const Scene<real> &s, Photon<re
   return kRefill;
 }
 
-template <typename real, bool TLE = false>
+template <typename real>
 __device__ __forceinline__ int flight(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc, int &pmat,
                                       uint32_t &pv, int &pscored, unsigned int &n_wood, unsigned int &n_real,
-                                      unsigned int &n_world, TleScore<real> sc = {nullptr, nullptr, nullptr}) {
+                                      unsigned int &n_world) {
   if (++ph.steps > kStepCap) {
     atomicAdd(&bc->loop_capped, 1u);
     ph.alive = 0;
     return kRefill;
   }
   if (ph.in_image) {
-    const int r = image_flight<real, TLE>(s, ph, g, pmat, pv, pscored, n_wood, n_real, bc, sc);
+    const int r = image_flight(s, ph, g, pmat, pv, pscored, n_wood, n_real);
     if (r != kFly || ph.in_image) return r;
     // Left the image box: take the world step at once (the same flight
     // count and draws as a separate phase, one block iteration fewer).
@@ -1179,19 +1211,15 @@ __device__ __forceinline__ void event_add(const Scene<real> &s, Event<real> &ev,
   }
 }
 
-// With TLE, the energy a photon at or below the estimator's threshold gives
-// to electrons is not scored (GateTLEDoseActor.cpp:236-243: secondaries of a
-// track-length-scored photon deposit nothing); its path scores instead.
-template <typename real, bool SPECT, bool TLE = false>
+template <typename real, bool SPECT>
 __device__ __forceinline__ int do_interaction(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc,
                                               int pmat, uint32_t pv, int pscored, HistList<real> &l,
                                               const Tally<real> &t, Secondary<real> &sec, unsigned int &n_dep,
                                               Event<real> &ev, int *kind = nullptr) {
-  const real e_pre = ph.e;
   real ed = interact(s, ph, pmat, g, bc, sec, kind);
   if (pscored == 1) {
     if constexpr (!SPECT) {
-      if (!TLE || e_pre > s.tle_thr) deposit(l, t, bc, pv, ed, n_dep);
+      deposit(l, t, bc, pv, ed, n_dep);
     }
     if (ph.alive && ph.in_image) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
   } else if (pscored == 0) {

@@ -29,15 +29,18 @@
 
 namespace gg {
 
-enum : int { kQRefill = 0, kQFly = 1, kQWorld = 2, kQInteract = 3, kQueues = 4, kQNone = 4 };
+// kQWalk: the track-length estimator's only
+enum : int { kQRefill = 0, kQFly = 1, kQWorld = 2, kQInteract = 3, kQueues = 4, kQWalk = 4, kTleQueues = 5, kQNone = 8 };
 // A gang's event queues.  cnt / tail are the same in every thread: queue
-// lengths and ring positions, 16 bits each (queues 0, 1 in x, 2, 3 in y).
-template <int kPoolRing>
+// lengths and ring positions, 16 bits each (queue q in half q & 1 of word q >> 1).
+template <int kPoolRing, int NQ = kQueues>
 struct EventQueues {
+  static constexpr int kWords = (NQ + 1) / 2, kSet = NQ <= 4 ? 4 : 8;  // kSet: words of a push set
+  static_assert(NQ <= 6, "round() and put() select among three words");
   static_assert((kPoolRing & (kPoolRing - 1)) == 0 && kPoolRing <= 1024, "ring positions are masked, packed in 16 bits");
-  uint16_t *ring;     // [kQueues][kPoolRing]
-  unsigned *push;     // [3][kQueues]
-  uint2 cnt, tail;
+  uint16_t *ring;     // [NQ][kPoolRing]
+  unsigned *push;     // [3][kSet]
+  unsigned cnt[kWords], tail[kWords];
   unsigned rd;        // push set of this round's barrier, rotates through 0, 1, 2
   unsigned tid, size; // the thread in its gang, the gang's threads
   int bar;            // named barrier
@@ -50,9 +53,11 @@ struct EventQueues {
     ring = r;
     push = p;
     for (unsigned i = tid; i < slots; i += size) ring[kQRefill * kPoolRing + i] = (uint16_t)i;
-    if (tid < 3 * kQueues) push[tid] = 0u;
-    cnt = make_uint2(slots, 0u);  // (kQRefill is queue 0)
-    tail = make_uint2(slots & (kPoolRing - 1u), 0u);
+    if (tid < 3 * kSet) push[tid] = 0u;
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) cnt[w] = tail[w] = 0u;
+    cnt[0] = slots;  // (kQRefill is queue 0)
+    tail[0] = slots & (kPoolRing - 1u);
     rd = 0u;
   }
   __device__ __forceinline__ void sync() const { named_bar(bar, (int)size); }
@@ -62,40 +67,56 @@ struct EventQueues {
   __device__ __forceinline__ int round(int &slot, unsigned &n) {
     constexpr unsigned kMask = (kPoolRing - 1u) * 0x10001u;
     sync();
-    const uint4 p = reinterpret_cast<const uint4 *>(push)[rd];
     const unsigned clr = rd == 0u ? 2u : rd - 1u;  // (rd + 2) % 3: the set after next
-    if (tid == 0) reinterpret_cast<uint4 *>(push)[clr] = make_uint4(0u, 0u, 0u, 0u);
+    unsigned best = 0u;                            // the longest queue: length * 8 + queue
+#pragma unroll
+    for (int h = 0; h < kSet / 4; ++h) {
+      const uint4 p = reinterpret_cast<const uint4 *>(push + rd * kSet)[h];
+      if (tid == 0) reinterpret_cast<uint4 *>(push + clr * kSet)[h] = make_uint4(0u, 0u, 0u, 0u);
+      const unsigned add[2] = {p.x | (p.y << 16), p.z | (p.w << 16)};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int w = 2 * h + j;
+        if (w < kWords) {
+          cnt[w] += add[j];
+          tail[w] = (tail[w] + add[j]) & kMask;
+          best = max(best, max(((cnt[w] & 0xffffu) << 3) | (2u * w), ((cnt[w] >> 13) & ~7u) | (2u * w + 1u)));
+        }
+      }
+    }
     rd = rd == 2u ? 0u : rd + 1u;  // the set this round pushes to
-    const unsigned ax = p.x | (p.y << 16), ay = p.z | (p.w << 16);
-    cnt.x += ax;
-    cnt.y += ay;
-    tail.x = (tail.x + ax) & kMask;
-    tail.y = (tail.y + ay) & kMask;
-    // the longest queue: length * 4 + queue
-    const unsigned best = max(max((cnt.x & 0xffffu) << 2, ((cnt.x >> 14) & ~3u) | 1u),
-                              max(((cnt.y & 0xffffu) << 2) | 2u, ((cnt.y >> 14) & ~3u) | 3u));
-    const unsigned q = best & 3u, len = best >> 2, sh = (q & 1u) << 4;
+    const unsigned q = best & 7u, len = best >> 3, sh = (q & 1u) << 4;
     n = min(min(len, size), (unsigned)kPoolRing - len);
     slot = -1;
     if (len == 0u) return kQNone;
-    const unsigned head = ((q & 2u ? tail.y : tail.x) >> sh) - len;
+    const unsigned head = (tail_word((int)q) >> sh) - len;
     if (tid < n) slot = ring[q * kPoolRing + ((head + tid) & (kPoolRing - 1u))];
-    if (q & 2u) cnt.y -= n << sh;
-    else cnt.x -= n << sh;
+#pragma unroll
+    for (int w = 0; w < kWords; ++w)
+      if ((int)(q >> 1) == w) cnt[w] -= n << sh;
     return (int)q;
+  }
+
+  __device__ __forceinline__ unsigned tail_word(int q) const {
+    if (NQ > 4 && (q & 4)) return tail[kWords - 1];
+    return q & 2 ? tail[1] : tail[0];
   }
 
   // Appends the lane's slot to queue `dest` (kQNone: nowhere); every lane of the warp calls it.
   __device__ __forceinline__ void put(int dest, int slot, unsigned lane, unsigned lt_mask) {
     const unsigned b0 = __ballot_sync(0xffffffffu, dest == 0), b1 = __ballot_sync(0xffffffffu, dest == 1),
                    b2 = __ballot_sync(0xffffffffu, dest == 2), b3 = __ballot_sync(0xffffffffu, dest == 3);
-    const unsigned m = dest & 2 ? (dest & 1 ? b3 : b2) : (dest & 1 ? b1 : b0);
+    unsigned m = dest & 2 ? (dest & 1 ? b3 : b2) : (dest & 1 ? b1 : b0);
+    if constexpr (NQ > 4) {
+      const unsigned b4 = __ballot_sync(0xffffffffu, dest == 4);
+      if (dest == 4) m = b4;
+    }
     const unsigned rank = __popc(m & lt_mask);
     unsigned off = 0u;
-    if (dest < kQueues && rank == 0u) off = atomicAdd(&push[rd * kQueues + (unsigned)dest], __popc(m));
+    if (dest < NQ && rank == 0u) off = atomicAdd(&push[rd * kSet + (unsigned)dest], __popc(m));
     off = __shfl_sync(0xffffffffu, off, __ffs(m) - 1);  // (the lane's own value is unused when m is 0)
-    const unsigned t = (dest & 2 ? tail.y : tail.x) >> ((dest & 1) << 4);
-    if (dest < kQueues) ring[(unsigned)dest * kPoolRing + ((t + off + rank) & (kPoolRing - 1u))] = (uint16_t)slot;
+    const unsigned t = tail_word(dest) >> ((dest & 1) << 4);
+    if (dest < NQ) ring[(unsigned)dest * kPoolRing + ((t + off + rank) & (kPoolRing - 1u))] = (uint16_t)slot;
   }
 };
 
@@ -337,17 +358,34 @@ struct VoxelList<double> {
 };
 template <typename real>
 using DoseSlot = PhotonSlot<real, VoxelList<real>>;
-static_assert(sizeof(DoseSlot<float>) % 32 == 16 && sizeof(DoseSlot<double>) % 32 == 16, "odd 16-byte stride");
+// ... and, with the track-length estimator, its walk through the voxels: next
+// boundary per axis and path so far, boundary spacing per axis and drawn path,
+// voxel per axis and boundaries crossed.
+template <typename real>
+struct TlePad {};
+template <>
+struct TlePad<float> {
+  uint4 pad;
+};
+template <typename real>
+struct VoxelWalkList : TlePad<real> {
+  uint32_t vox[kHistList];
+  alignas(16) real acc[kHistList];
+  Real4<real> tn, td;
+  int4 it;
+};
+template <typename real>
+using TleSlot = PhotonSlot<real, VoxelWalkList<real>>;
+static_assert(sizeof(DoseSlot<float>) % 32 == 16 && sizeof(DoseSlot<double>) % 32 == 16 &&
+                  sizeof(TleSlot<float>) % 32 == 16 && sizeof(TleSlot<double>) % 32 == 16,
+              "odd 16-byte stride");
 static_assert(kHistList == 8, "list_deposit reads the voxels as two 16-byte words");
 
 // A history's voxel list in its slot (the entries of HistList, in their order).
-// deposit(): all voxels are compared at once - a loop over the entries makes
-// the warp wait for its longest list.
-template <typename real>
-__device__ __forceinline__ void list_deposit(VoxelList<real> &S, int &n, const Tally<real> &t, uint32_t v, real e,
-                                             unsigned int &n_dep, unsigned int &n_entries, unsigned int &n_over) {
-  if (!(e > R<real>(0))) return;
-  ++n_dep;
+// list_add(): all voxels are compared at once - a loop over the entries makes
+// the warp wait for its longest list; false: a new voxel, and the list is full.
+template <typename real, typename List>
+__device__ __forceinline__ bool list_add(List &S, int &n, uint32_t v, real e) {
   const uint4 a = *reinterpret_cast<const uint4 *>(S.vox), b = *reinterpret_cast<const uint4 *>(S.vox + 4);
   const uint32_t u[kHistList] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   int at = n;
@@ -356,26 +394,35 @@ __device__ __forceinline__ void list_deposit(VoxelList<real> &S, int &n, const T
     if (k < n && u[k] == v) at = k;
   if (at < n) {
     S.acc[at] = S.acc[at] + e;
-    return;
+    return true;
   }
-  if (n == kHistList) {
-    ++n_over;
-    n_entries += kHistList;
-#pragma unroll 1
-    for (int k = 0; k < kHistList; ++k) tally_entry(t, S.vox[k], S.acc[k]);
-    n = at = 0;
-  }
+  if (n == kHistList) return false;
   S.vox[at] = v;
   S.acc[at] = e;
   n = at + 1;
+  return true;
+}
+template <typename real, typename List>
+__device__ __forceinline__ void list_deposit(List &S, int &n, const Tally<real> &t, uint32_t v, real e,
+                                             unsigned int &n_dep, unsigned int &n_entries, unsigned int &n_over) {
+  if (!(e > R<real>(0))) return;
+  ++n_dep;
+  if (list_add(S, n, v, e)) return;
+  ++n_over;
+  n_entries += kHistList;
+#pragma unroll 1
+  for (int k = 0; k < kHistList; ++k) tally_entry(t, S.vox[k], S.acc[k]);
+  S.vox[0] = v;
+  S.acc[0] = e;
+  n = 1;
 }
 
 // The lists of the warp's ended histories (`n` entries of the lane's slot
 // `slot`) into the tallies: the entries are dealt over the lanes, one each -
 // about 1.5 per history, but the longest of 32 lists has 4 or 5.  ids: 32 *
 // kHistList numbers of the warp's own.  tally_of(slot): the slot's tally.
-template <typename real, typename TallyOf>
-__device__ __forceinline__ void lists_flush(const DoseSlot<real> *slots, int slot, int n, uint16_t *ids, unsigned lane,
+template <typename Slot, typename TallyOf>
+__device__ __forceinline__ void lists_flush(const Slot *slots, int slot, int n, uint16_t *ids, unsigned lane,
                                             TallyOf &&tally_of, unsigned int &n_entries) {
   unsigned end = (unsigned)n;
 #pragma unroll
@@ -392,11 +439,58 @@ __device__ __forceinline__ void lists_flush(const DoseSlot<real> *slots, int slo
 #pragma unroll 1
   for (unsigned i = lane; i < total; i += 32u) {
     const unsigned id = ids[i];
-    const DoseSlot<real> &S = slots[id / kHistList];
+    const Slot &S = slots[id / kHistList];
     tally_entry(tally_of(S), S.x.vox[id % kHistList], S.x.acc[id % kHistList]);
   }
   n_entries += (unsigned)n;
   __syncwarp();
+}
+
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
+  unsigned long long r = __reduce_add_sync(0xffffffffu, (unsigned)x & 0xffffffu);
+  r += (unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(x >> 24) & 0xffffffu) << 24;
+  return r + ((unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(x >> 48)) << 48);
+}
+
+// The first n entries of each lane's list into the tally, entry by entry;
+// entries of the voxel that the first such lane holds are summed first and added
+// once when they are several.  The photons of a narrow beam cross the same voxels in the
+// same rounds, and their atomics otherwise queue at a few L2 slices.
+constexpr int kSameVoxel = 3;
+template <typename real, typename List>
+__device__ __forceinline__ void lists_flush_same(const List &S, int n, const Tally<real> &t, unsigned lane) {
+#pragma unroll 1
+  for (int k = 0;; ++k) {
+    const bool has = k < n;
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    if (m == 0u) break;
+    const int first = __ffs(m) - 1;
+    const uint32_t v = S.vox[min(k, kHistList - 1)];
+    const unsigned long long q = has ? (unsigned long long)to_fixed(S.acc[k]) : 0ull;
+    const uint32_t v0 = __shfl_sync(0xffffffffu, v, first);
+    bool mine = has && v == v0;
+    const unsigned same = __ballot_sync(0xffffffffu, mine);
+    unsigned long long e = q, lo = (q * q) & 0xffffffffull, hi = (__umul64hi(q, q) << 32) | ((q * q) >> 32);
+    if (__popc(same) >= kSameVoxel) {
+      const unsigned long long se = warp_sum(mine ? e : 0ull);
+      const unsigned long long sl = warp_sum(mine ? lo : 0ull), sh = warp_sum(mine ? hi : 0ull);
+      if ((int)lane == first) {
+        e = se;
+        lo = sl;
+        hi = sh;
+        mine = false;
+      }
+    } else {
+      mine = false;
+    }
+    if (has && !mine) {
+      atomicAdd(&t.acc_e[v], e);
+      if (t.acc_e2) {
+        atomicAdd(&t.acc_e2[2 * (size_t)v], lo);
+        atomicAdd(&t.acc_e2[2 * (size_t)v + 1], hi);
+      }
+    }
+  }
 }
 
 // The second list of a dose grid that scores dose too, in global memory:

@@ -9,8 +9,7 @@
 // Kernel design (one GB300, one process):
 //   * a source stage samples the primaries into coalesced records;
 //   * the transport stage keeps more photons than threads in shared memory and
-//     runs one kind of event at a time on full warps (gg_pool.cuh); only the
-//     track-length estimator still carries one photon per thread;
+//     runs one kind of event at a time on full warps (gg_pool.cuh);
 //   * Woodcock (delta) tracking against a per-energy majorant inside the image
 //     box; analytic free flight in the world material outside it;
 //   * the majorant, total attenuation rows and the label->(composition,
@@ -27,6 +26,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "gg_device.cuh"
 #include "gg_internal.h"
@@ -189,6 +189,109 @@ __device__ __forceinline__ Tally<real> tally_at(const KernelArgs &a, size_t off,
   return Tally<real>{a.acc_e + off, a.acc_e2 ? a.acc_e2 + 2 * off : nullptr};
 }
 
+// Boundaries a walk of the track-length estimator crosses in one round: their
+// label loads are in flight together, but a path's last round leaves lanes idle
+// (2 / 3 / 4 / 5 / 6 / 8 boundaries: 9.5 / 7.8 / 6.9 / 7.1 / 7.0 / 7.5 ms, the
+// workload of k_transport_pool).
+constexpr int kTleSteps = 4;
+static_assert(kTleSteps <= kHistList, "the list holds what is left of a round after a flush");
+
+template <typename real>
+__device__ __forceinline__ void tle_store(VoxelWalkList<real> &X, const VoxelWalk<real> &w, real sd) {
+  X.tn = Real4<real>{w.tn[0], w.tn[1], w.tn[2], w.tc};
+  X.td = Real4<real>{w.td[0], w.td[1], w.td[2], sd};
+  X.it = make_int4(w.i[0], w.i[1], w.i[2], w.k);
+}
+
+// One round of the estimator's walks (slot k of each lane, -1: none); the
+// slot's next event.  The warp calls it together.
+template <typename real>
+__device__ __forceinline__ int tle_walk(const Scene<real> &s, TleSlot<real> *slots, int k, unsigned lane,
+                                        const Tally<real> &t, unsigned int &n_dep, unsigned int &n_ent,
+                                        unsigned int &n_over) {
+  TleSlot<real> &S = slots[max(k, 0)];
+  const uint4 e = S.e;
+  const Real4<real> b = S.b, tn = S.x.tn, td = S.x.td;
+  const int4 it = S.x.it;
+  VoxelWalk<real> w{{tn.x, tn.y, tn.z}, {td.x, td.y, td.z}, tn.w, {it.x, it.y, it.z}, it.w};
+  const real d[3] = {b.x, b.y, b.z}, len = td.w < S.a.w ? td.w : S.a.w;
+  EIdx<real> ei;
+  ei.fe = S.c.z;
+  ei.ie = (int)(real_bits(S.c.w) & 0xffffu);
+  // the crossings, then their labels with all loads in flight, then the energies
+  uint32_t v[kTleSteps];
+  real ed[kTleSteps];
+  bool more = k >= 0;
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    v[j] = 0u;
+    ed[j] = R<real>(0);
+    if (more) more = w.step(s, d, len, v[j], ed[j]);
+  }
+  int m[kTleSteps];
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) m[j] = (int)__ldg(s.labels + v[j]);
+  int last = -1;
+  real mu_e = R<real>(0);
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    if (m[j] != last) {
+      last = m[j];
+      real mu = interp_row(s.muen + (size_t)s.mat_comp[last] * s.n_e, ei);
+      mu = s.mat_rho[last] * mu;
+      mu_e = b.w * mu;
+    }
+    ed[j] = ed[j] > R<real>(0) ? mu_e * ed[j] : R<real>(0);
+  }
+  // into the list: a walk never comes back to a voxel, so only the entries from
+  // before this round can be a crossing's voxel, and none once the list is flushed
+  int n = (int)((e.z >> kSlList) & 15u), n_old = n;
+  const uint4 ua = *reinterpret_cast<const uint4 *>(S.x.vox), ub = *reinterpret_cast<const uint4 *>(S.x.vox + 4);
+  const uint32_t u[kHistList] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+  bool full = false;
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    if (ed[j] > R<real>(0) && !full) {
+      int at = n;
+#pragma unroll
+      for (int q = 0; q < kHistList; ++q)
+        if (q < n_old && u[q] == v[j]) at = q;
+      if (at == kHistList) {
+        full = true;
+      } else {
+        const bool add = at == n;
+        S.x.vox[at] = v[j];
+        S.x.acc[at] = add ? ed[j] : S.x.acc[at] + ed[j];
+        n += add ? 1 : 0;
+        ++n_dep;
+        ed[j] = R<real>(0);
+      }
+    }
+  }
+  __syncwarp();
+  if (__any_sync(0xffffffffu, full)) {
+    lists_flush_same(S.x, full ? n : 0, t, lane);
+    if (full) {
+      ++n_over;
+      n_ent += kHistList;
+      n = 0;
+#pragma unroll
+      for (int j = 0; j < kTleSteps; ++j)
+        if (ed[j] > R<real>(0)) {
+          S.x.vox[n] = v[j];
+          S.x.acc[n] = ed[j];
+          ++n;
+          ++n_dep;
+        }
+    }
+  }
+  if (k < 0) return kQNone;
+  S.x.tn = Real4<real>{w.tn[0], w.tn[1], w.tn[2], w.tc};
+  S.x.it = make_int4(w.i[0], w.i[1], w.i[2], w.k);
+  S.e.z = (e.z & ~(15u << kSlList)) | ((uint32_t)n << kSlList);
+  return more ? kQWalk : kQFly;
+}
+
 // Transport stage: the pooled event loop of gg_pool.cuh.  Events: a new history
 // (the ended one's voxel list goes to the tallies first), a Woodcock step in
 // the image, a free flight in the world, an interaction; a photon that starts
@@ -200,28 +303,42 @@ __device__ __forceinline__ Tally<real> tally_at(const KernelArgs &a, size_t off,
 // (203 warp instructions per history at 21.5 active lanes; 379 at 8.6); 24
 // batched simulations 22.8 -> 14.1 ms, FP64 9.2 -> 4.2 ms per 1e6.
 // MULTI: batched simulations; DG: dose tally on a grid of its own (1: edep,
-// 2: edep and dose), Scene::dgrid.
-template <typename real, bool MULTI, int DG>
+// 2: edep and dose), Scene::dgrid; TLE: track-length estimator
+// (GateTLEDoseActor::ScoreTLEDepositStep,
+// core/opengate_core/opengate_lib/GateTLEDoseActor.cpp:249-299): a photon at or
+// below its threshold energy scores e * mu_en(E, material) * length in every
+// voxel its flights cross, and its interactions deposit nothing
+// (GateTLEDoseActor.cpp:236-243).  Such a flight is two kinds of event: its path
+// is drawn, then walked kTleSteps boundaries a round.  64^3 voxels of 2 mm,
+// 3e6 photons of 1 MeV in a pencil beam (81 voxels each): 13.5 -> 6.9 ms
+// against one photon per thread with each path walked at once (2088 warp
+// instructions per history at 7.4 lanes; now 880 at 25).  Two things count
+// together: without the sums of equal voxels (lists_flush_same) the atomics of
+// the beam's axis queue at a few L2 slices, 12.2 ms.
+template <typename real, bool MULTI, int DG, bool TLE>
 __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(Scene<real> sg, KernelArgs args, int n_slots) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
+  using Slot = std::conditional_t<TLE, TleSlot<real>, DoseSlot<real>>;
   constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
-  __shared__ __align__(16) unsigned push[kGangs][3 * kQueues];
+  constexpr int kNq = TLE ? kTleQueues : kQueues;
+  using Queues = EventQueues<Shape::kRing, kNq>;
+  __shared__ __align__(16) unsigned push[kGangs][3 * Queues::kSet];
   __shared__ __align__(16) uint32_t ahead[Shape::kBlock][4];  // EventRng's second block of each thread
-  __shared__ uint16_t ring[kGangs][kQueues * Shape::kRing];
+  __shared__ uint16_t ring[kGangs][kNq * Shape::kRing];
   __shared__ unsigned long long s_claim[kGangs];
   Scene<real> s = sg;
   const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
   const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
   const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
   // dynamic shared memory: slots of the gangs, tables
-  DoseSlot<real> *const slots = reinterpret_cast<DoseSlot<real> *>(smem_raw) + gang * n_slots;
-  EventQueues<Shape::kRing> Q;
+  Slot *const slots = reinterpret_cast<Slot *>(smem_raw) + gang * n_slots;
+  Queues Q;
   Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
          (unsigned)n_slots);
   for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) slots[i].e = make_uint4(0u, 0u, 0u, 0u);
-  stage_tables(sg, s, smem_raw + sizeof(DoseSlot<real>) * (size_t)(gangs * n_slots), bc);
+  stage_tables(sg, s, smem_raw + sizeof(Slot) * (size_t)(gangs * n_slots), bc);
 
   const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
   Tally<real> t{args.acc_e, args.acc_e2};
@@ -249,16 +366,28 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
     if (event == kQRefill) {
       claims.take(Q, n, args.next, args.chunk, n_hist, &s_claim[gang]);
       // the ended histories' voxel lists
-      lists_flush(slots, max(k, 0), k >= 0 ? (int)((slots[k].e.z >> kSlList) & 15u) : 0,
-                  reinterpret_cast<uint16_t *>(ahead[threadIdx.x & ~31u]), lane,
-                  [&](const DoseSlot<real> &S) {
-                    if constexpr (MULTI) return tally_at(args, sg.sims[S.e.w].vox_off, real(0));
-                    else return t;
-                  },
-                  n_ent);
+      const int n_old = k >= 0 ? (int)((slots[k].e.z >> kSlList) & 15u) : 0;
+      if constexpr (TLE) {
+        lists_flush_same(slots[max(k, 0)].x, n_old, t, lane);
+        n_ent += (unsigned)n_old;
+      } else {
+        lists_flush(slots, max(k, 0), n_old, reinterpret_cast<uint16_t *>(ahead[threadIdx.x & ~31u]), lane,
+                    [&](const Slot &S) {
+                      if constexpr (MULTI) return tally_at(args, sg.sims[S.e.w].vox_off, real(0));
+                      else return t;
+                    },
+                    n_ent);
+      }
+    }
+    if constexpr (TLE) {
+      if (event == kQWalk) {
+        dest = tle_walk(s, slots, k, lane, t, n_dep, n_ent, n_over);
+        Q.put(dest, k, lane, lt_mask);
+        continue;
+      }
     }
     if (k >= 0) {
-      DoseSlot<real> &S = slots[k];
+      Slot &S = slots[k];
       uint4 e = S.e;
       int n_list = (int)((e.z >> kSlList) & 15u);
       if constexpr (DG == 2) {
@@ -336,6 +465,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
         pmat = (int)(cw >> 16);
         pscored = (int)((e.z >> kSlImage) & 1u);
         pv = real_bits(ph.t_exit);
+        const bool score = !TLE || ph.e > s.tle_thr;
         EventRng g{buf, ahead[threadIdx.x], k0, k1, 0u, h0, h1, e.x, idx};
         g.begin();
         real ed;
@@ -350,6 +480,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           uint32_t v = pv;
           bool in = true;
           if constexpr (DG > 0) in = dose_voxel(s, ph.pos, v);
+          if constexpr (TLE) in = score;
           if (in) {
             list_deposit(S.x, n_list, t, v, ed, n_dep, n_ent, n_over);
             if constexpr (DG == 2) {
@@ -368,18 +499,42 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       if (aim) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
       if (event == kQWorld || dest == kQFly) {
         // ---- a flight
-        if (++ph.steps > kStepCap) {
+        TwoWords g;
+        g.draw(buf, e.x, idx, 0u, h0, h1, k0, k1);
+        if constexpr (TLE) {
+          if (event == kQFly && e.w) {  // a scored path has been walked; no collision: the next flight
+            e.w = 0u;
+            ph.in_image = 1;
+            const int r = image_arrive(s, ph, g, S.x.td.w, pmat, pv, pscored, n_wood, n_real);
+            dest = r == kInteract ? kQInteract : (ph.in_image ? kQFly : kQWorld);
+          }
+        }
+        if (TLE && event != kQWorld && dest != kQFly) {
+          g.end(buf, e.x, idx);
+        } else if (++ph.steps > kStepCap) {
           atomicAdd(&bc.loop_capped, 1u);
+          if constexpr (TLE) g.end(buf, e.x, idx);
           dest = kQRefill;
         } else {
-          TwoWords g;
-          g.draw(buf, e.x, idx, 0u, h0, h1, k0, k1);
           if (event == kQWorld) {
             ++n_world;
             const int r = dose_world_flight(s, ph, g, pmat, pscored);
             if (r == kRefill) ++n_esc;
             ph.t_exit = R<real>(-1);
             dest = r == kInteract ? kQInteract : (r == kFly ? kQFly : kQRefill);
+          } else if (TLE && ph.e <= s.tle_thr) {
+            if (ph.e <= s.tle_emin) {  // the kill energy: the rest is left where the photon is
+              list_deposit(S.x, n_list, t, voxel_of(s, ph.pos), ph.e, n_dep, n_ent, n_over);
+              dest = kQRefill;
+            } else {
+              if constexpr (TLE) {
+                VoxelWalk<real> w;
+                w.start(s, ph.pos, ph.dir);
+                tle_store(S.x, w, woodcock_path(ph, g));
+              }
+              e.w = 1u;
+              dest = kQWalk;
+            }
           } else {
             ph.in_image = 1;
             const int r = image_flight(s, ph, g, pmat, pv, pscored, n_wood, n_real);
@@ -422,200 +577,6 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
     if (bc.loop_capped) atomicAdd(&cnt[GG_CNT_LOOP_CAPPED], (unsigned long long)bc.loop_capped);
     if (bc.stack_overflow) atomicAdd(&cnt[GG_CNT_STACK_OVERFLOW], (unsigned long long)bc.stack_overflow);
     if (bc.secondaries) atomicAdd(&cnt[GG_CNT_SECONDARIES], (unsigned long long)bc.secondaries);
-  }
-}
-
-// Transport stage with the track-length estimator (a history scores every voxel
-// it crosses: its list fills and empties many times, so it stays with its
-// thread).  Persistent grid; each lane carries one history at a time
-// and is in one of the states kRefill (needs a history), kFly (next event is
-// a flight) or kInteract (a collision is pending).  Every iteration the block
-// picks ONE phase from counts of its lanes' states - refill when at least
-// refill_min lanes per warp wait for a history, interact when at least
-// interact_min collisions per warp are pending, otherwise fly - and only the
-// lanes in that state execute it.  Expensive code (source-record loads, tally
-// flushes, Compton sampling) therefore runs with many lanes active instead of
-// one lane at a time, all warps of a block execute the same code region at
-// the same time (the kernel is bound by instruction fetch, not arithmetic),
-// and the order of operations inside each history, hence its result, is
-// unchanged.
-// MINB = resident blocks per SM the register budget is sized for.
-template <typename real, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_transport_tle(Scene<real> sg, KernelArgs args) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ BlockCounters bc;
-  __shared__ real sec_store[6 * 256];
-  // ---- stage tables in shared memory --------------------------------------
-  Scene<real> s = sg;
-  {
-    real *sh = reinterpret_cast<real *>(smem_raw);
-    const int nsig = sg.n_comp * sg.n_e;
-    real *ssig = sh;
-    real *smaj = ssig + nsig;
-    real *srho = smaj + sg.n_e;
-    int *scomp = reinterpret_cast<int *>(srho + sg.n_mat);
-    for (int i = threadIdx.x; i < nsig; i += blockDim.x) ssig[i] = sg.sig[i];
-    for (int i = threadIdx.x; i < sg.n_e; i += blockDim.x) smaj[i] = sg.maj[i];
-    for (int i = threadIdx.x; i < sg.n_mat; i += blockDim.x) {
-      srho[i] = sg.mat_rho[i];
-      scomp[i] = sg.mat_comp[i];
-    }
-    if (threadIdx.x == 0) bc = BlockCounters{0, 0, 0, 0, 0, 0, 0, 0};
-    __syncthreads();
-    s.sig = ssig;
-    s.maj = smaj;
-    s.mat_rho = srho;
-    s.mat_comp = scomp;
-  }
-  const Records<real> rec = Records<real>::carve(args.records, args.rec_cap);
-  Tally<real> t{args.acc_e, args.acc_e2};
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  const uint64_t n_hist = args.h_end - args.h_begin;
-  __shared__ uint64_t wpool[kBlock / 32][2];  // per warp: claimed histories not yet handed out
-  uint64_t *pool = wpool[threadIdx.x >> 5];
-  if (lane == 0) pool[0] = pool[1] = 0;
-  __syncwarp();
-
-  Photon<real> ph;
-  ph.alive = 0;
-  Secondary<real> sec;
-  sec.base = sec_store;
-  sec.stride = blockDim.x;
-  sec.tid = threadIdx.x;
-  sec.has = 0;
-  // history lists after the tables: [list][vox | acc][kHistList][blockDim.x]
-  HistList<real> l;
-  {
-    const int nt = (int)blockDim.x;
-    unsigned char *lists = smem_raw + transport_smem_bytes<real>(sg.n_comp, sg.n_e, sg.n_mat);
-    l.vox = reinterpret_cast<uint32_t *>(lists) + threadIdx.x;
-    l.acc = reinterpret_cast<real *>(lists + (size_t)kHistList * nt * sizeof(uint32_t)) + threadIdx.x;
-    l.stride = nt;
-    l.n = 0;
-  }
-  Event<real> ev;
-  ev.clear();
-  Rng g;
-  int state = kRefill;
-  bool in_hist = false;
-  int pmat = 0, pscored = 0;
-  uint32_t pv = 0;
-  unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0;
-
-  for (;;) {
-    // phase chosen per block: all warps run the same code region at the same
-    // time (instruction-cache locality); thresholds are per warp
-    const unsigned m_ref = __ballot_sync(0xffffffffu, state == kRefill);
-    const int c_ref = __syncthreads_count(state == kRefill);
-    const int c_fly = __syncthreads_count(state == kFly);
-    const int c_int = __syncthreads_count(state == kInteract);
-    if (c_ref + c_fly + c_int == 0) break;
-    const int n_warps = (int)(blockDim.x >> 5);
-    int phase;
-    if (c_ref >= args.refill_min * n_warps || (c_fly + c_int) == 0) phase = kRefill;
-    else if (c_int >= args.interact_min * n_warps || c_fly == 0) phase = kInteract;
-    else phase = kFly;
-
-    if (phase == kRefill) {
-      const bool need = state == kRefill;
-      // per-lane atomics: a warp-aggregated flush (same-voxel entries of the warp summed
-      // first, __match_any_sync + shuffles) issued as many atomic instructions here and
-      // made the transport 28 % slower, so it is not used
-      if (need && in_hist) hlist_flush(l, t, &bc);
-      if (need) in_hist = false;
-      const uint64_t h = warp_pool_claim(pool, m_ref, lane, lt_mask, args.next, args.chunk);
-      if (need) {
-        if (h >= n_hist) {
-          state = kDone;
-        } else {
-          const uint32_t f = rec.flags[h];
-          const uint32_t rs = f & 3u;
-          if (rs != kRecDead) {
-            const uint64_t hid = args.h_begin + h;
-            const uint64_t key = args.seed;
-            ph.pos[0] = rec.px[h];
-            ph.pos[1] = rec.py[h];
-            ph.pos[2] = rec.pz[h];
-            ph.dir[0] = rec.dx[h];
-            ph.dir[1] = rec.dy[h];
-            ph.dir[2] = rec.dz[h];
-            set_energy(s, ph, rec.e[h]);
-            ph.steps = (int)((f >> 2) & 1u);
-            ph.alive = 1;
-            ph.can_enter = 1;
-            ph.in_head = 0;
-            ph.exclude = -1;
-            ph.w = s.s_fd_w;  // 1, or the forced direction's cone weight
-            const uint32_t rp = rec.rng_pos[h];
-            const uint4 b = rec.rng_buf[h];
-            g.k0 = (uint32_t)key;
-            g.k1 = (uint32_t)(key >> 32);
-            g.stream = 0u;
-            g.h0 = (uint32_t)hid;
-            g.h1 = (uint32_t)(hid >> 32);
-            g.blk = rp >> 3;
-            g.idx = (int)(rp & 7u);
-            g.buf[0] = b.x;
-            g.buf[1] = b.y;
-            g.buf[2] = b.z;
-            g.buf[3] = b.w;
-            if (rs == kRecInImage) {
-              ph.in_image = 1;
-              ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-              state = kFly;
-            } else if (rs == kRecWorld) {
-              ph.in_image = 0;
-              state = kFly;
-            } else {
-              ph.in_image = 0;
-              pmat = s.world_mat;
-              pscored = 0;
-              state = kInteract;
-            }
-            in_hist = true;
-          }
-        }
-      }
-    } else if (phase == kInteract) {
-      if (state == kInteract) {
-        state = do_interaction<real, false, true>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev);
-        if (state == kRefill && sec.has) {
-          pop_secondary(s, ph, sec);
-          state = kFly;
-        }
-      }
-    } else {
-      if (state == kFly) {
-        state = flight<real, true>(s, ph, g, &bc, pmat, pv, pscored, n_wood, n_real, n_world,
-                                   TleScore<real>{&l, &t, &n_dep});
-        if (state == kRefill && sec.has) {
-          pop_secondary(s, ph, sec);
-          state = kFly;
-        }
-      }
-    }
-  }
-  // ---- counters -------------------------------------------------------------
-  unsigned long long *cnt = args.counters;
-  auto warp_add = [&](unsigned int v, int slot) {
-    unsigned long long x = v;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0 && x) atomicAdd(&cnt[slot], x);
-  };
-  warp_add(n_wood, GG_CNT_WOODCOCK_STEPS);
-  warp_add(n_real, GG_CNT_REAL_INTERACTIONS);
-  warp_add(n_dep, GG_CNT_DEPOSITS);
-  warp_add(n_world, GG_CNT_WORLD_STEPS);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&cnt[GG_CNT_TALLY_ENTRIES], (unsigned long long)bc.tally_entries);
-    atomicAdd(&cnt[GG_CNT_LIST_OVERFLOWS], (unsigned long long)bc.list_overflows);
-    atomicAdd(&cnt[GG_CNT_ESCAPED], (unsigned long long)bc.escaped);
-    atomicAdd(&cnt[GG_CNT_LOOP_CAPPED], (unsigned long long)bc.loop_capped);
-    atomicAdd(&cnt[GG_CNT_STACK_OVERFLOW], (unsigned long long)bc.stack_overflow);
-    atomicAdd(&cnt[GG_CNT_SECONDARIES], (unsigned long long)bc.secondaries);
   }
 }
 
@@ -664,31 +625,23 @@ cudaError_t launch_generate(const Scene<real> &s, const KernelArgs &a, cudaStrea
   return cudaGetLastError();
 }
 
-template <typename real, bool MULTI, int DG>
+template <typename real, bool MULTI, int DG, bool TLE = false>
 static cudaError_t launch_pool_v(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st) {
   static unsigned long long configured = 0;
-  cudaError_t e = configure_smem(k_transport_pool<real, MULTI, DG>, 227 * 1024, configured);
+  cudaError_t e = configure_smem(k_transport_pool<real, MULTI, DG, TLE>, 227 * 1024, configured);
   if (e != cudaSuccess) return e;
-  k_transport_pool<real, MULTI, DG><<<p.grid, p.block, p.smem, st>>>(s, a, p.slots);
-  return cudaGetLastError();
-}
-
-template <typename real, int MINB>
-static cudaError_t launch_tle_v(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem,
-                                cudaStream_t st) {
-  static unsigned long long configured = 0;
-  cudaError_t e = configure_smem(k_transport_tle<real, MINB>, kTransportSmemMax, configured);
-  if (e != cudaSuccess) return e;
-  smem += hist_list_bytes<real>(1, block);
-  if (smem > (size_t)kTransportSmemMax) return cudaErrorInvalidValue;
-  k_transport_tle<real, MINB><<<grid, block, smem, st>>>(s, a);
+  k_transport_pool<real, MULTI, DG, TLE><<<p.grid, p.block, p.smem, st>>>(s, a, p.slots);
   return cudaGetLastError();
 }
 
 template <typename real>
 cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const PoolPlan &p, cudaStream_t st) {
-  // SPECT runs use the stage kernels of gg_spect.cu, the track-length estimator launch_transport_tle
-  if (s.spect || s.muen || p.block <= 0 || p.block > PoolShape<real>::kBlock || p.slots < 8 || p.slots > PoolShape<real>::kRing) return cudaErrorInvalidValue;
+  // SPECT runs use the stage kernels of gg_spect.cu
+  if (s.spect || p.block <= 0 || p.block > PoolShape<real>::kBlock || p.slots < 8 || p.slots > PoolShape<real>::kRing) return cudaErrorInvalidValue;
+  if (s.muen) {  // track-length estimator: single simulations on the image grid only
+    if (s.dgrid || s.n_sims > 0) return cudaErrorInvalidValue;
+    return launch_pool_v<real, false, 0, true>(s, a, p, st);
+  }
   if (s.dgrid) {
     // dose grid of its own (single simulations, analog scoring)
     if (s.n_sims > 0) return cudaErrorInvalidValue;
@@ -697,28 +650,10 @@ cudaError_t launch_transport(const Scene<real> &s, const KernelArgs &a, const Po
   return s.n_sims > 0 ? launch_pool_v<real, true, 0>(s, a, p, st) : launch_pool_v<real, false, 0>(s, a, p, st);
 }
 
-template <typename real>
-cudaError_t launch_transport_tle(const Scene<real> &s, const KernelArgs &a, int grid, int block, size_t smem, int minb,
-                                 cudaStream_t st) {
-  // single simulations on the image grid only
-  if (s.spect || !s.muen || s.dgrid || s.n_sims > 0 || block <= 0 || block > kBlock) return cudaErrorInvalidValue;
-  if (minb <= 2) return launch_tle_v<real, 2>(s, a, grid, block, smem, st);
-  if (minb == 3) return launch_tle_v<real, 3>(s, a, grid, block, smem, st);
-  return launch_tle_v<real, 4>(s, a, grid, block, smem, st);
-}
-
 cudaError_t launch_flush(unsigned long long *acc_e, unsigned long long *acc_e2, double *edep, double *edep2,
                          size_t n, int grid, cudaStream_t st, double scale) {
   k_flush<<<grid, 256, 0, st>>>(acc_e, acc_e2, edep, edep2, n, scale, scale * scale);
   return cudaGetLastError();
-}
-
-template <typename real>
-cudaError_t tle_occupancy(int block, size_t smem, int minb, int *bps) {
-  smem += hist_list_bytes<real>(1, block);
-  if (minb <= 2) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 2>, block, smem);
-  if (minb == 3) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 3>, block, smem);
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_transport_tle<real, 4>, block, smem);
 }
 
 // Launch shape of a pooled run: one block per SM.  More slots per thread keep
@@ -728,7 +663,7 @@ cudaError_t tle_occupancy(int block, size_t smem, int minb, int *bps) {
 // kernel's register budget; slot_bytes, scratch_bytes: of one slot, shared and global.
 template <typename real>
 cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
-                      size_t scratch_bytes, PoolPlan *p) {
+                      size_t scratch_bytes, int queues, PoolPlan *p) {
   int n_sm = 0, optin = 0;
   cudaError_t e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -740,7 +675,7 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
   if (blocks > 0) threads = std::min(threads, 256 * blocks);
   if (block > 0) threads = std::min(threads, block);
   threads = (int)std::min<uint64_t>(threads, (per_sm + 31) / 32 * 32);
-  const size_t slot = slot_bytes, fixed = pool_static<real>() + table_bytes;
+  const size_t slot = slot_bytes, fixed = pool_static<real>(queues) + table_bytes;
   const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
   while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
   const int gangs = (threads + kGang - 1) / kGang;
@@ -757,8 +692,8 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
 }
 
 template <typename real>
-size_t dose_slot_bytes() {
-  return sizeof(DoseSlot<real>);
+size_t dose_slot_bytes(bool tle) {
+  return tle ? sizeof(TleSlot<real>) : sizeof(DoseSlot<real>);
 }
 template <typename real>
 size_t slot_scratch_bytes(bool two) {
@@ -780,17 +715,11 @@ template cudaError_t launch_generate<double>(const Scene<double> &, const Kernel
 template cudaError_t launch_transport<float>(const Scene<float> &, const KernelArgs &, const PoolPlan &, cudaStream_t);
 template cudaError_t launch_transport<double>(const Scene<double> &, const KernelArgs &, const PoolPlan &,
                                               cudaStream_t);
-template cudaError_t launch_transport_tle<float>(const Scene<float> &, const KernelArgs &, int, int, size_t, int,
-                                                 cudaStream_t);
-template cudaError_t launch_transport_tle<double>(const Scene<double> &, const KernelArgs &, int, int, size_t, int,
-                                                  cudaStream_t);
-template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, size_t, size_t, PoolPlan *);
-template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, size_t, size_t, PoolPlan *);
-template size_t dose_slot_bytes<float>();
-template size_t dose_slot_bytes<double>();
+template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
+template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
+template size_t dose_slot_bytes<float>(bool);
+template size_t dose_slot_bytes<double>(bool);
 template size_t slot_scratch_bytes<float>(bool);
 template size_t slot_scratch_bytes<double>(bool);
-template cudaError_t tle_occupancy<float>(int, size_t, int, int *);
-template cudaError_t tle_occupancy<double>(int, size_t, int, int *);
 
 }  // namespace gg
