@@ -510,7 +510,7 @@ static int arf_generate(gg_ctx *c, const gg_arf_sampling *a, uint64_t n, uint64_
                         uint64_t capacity) {
   int st;
   if (!c->d_arf_stage) {
-    const uint64_t blocks = kArfChunk / 256;
+    const uint64_t blocks = kArfChunk / gg::kArfBlock;
     if ((st = c->cuda(cudaMalloc(&c->d_arf_stage, kArfChunk * sizeof(float4)), "cudaMalloc ARF staging"))) return st;
     if ((st = c->cuda(cudaMalloc(&c->d_arf_bcount, blocks * sizeof(unsigned int)), "cudaMalloc"))) return st;
     if ((st = c->cuda(cudaMalloc(&c->d_arf_boff, blocks * sizeof(unsigned long long)), "cudaMalloc"))) return st;
@@ -544,6 +544,7 @@ static int arf_generate(gg_ctx *c, const gg_arf_sampling *a, uint64_t n, uint64_
   p.theta_uniform = a->theta_uniform ? 1 : 0;
   p.theta_max_turn = std::acos(a->cos_theta_max) / (2.0 * M_PI);
   p.stage = c->d_arf_stage;
+  p.next = c->d_next;
   p.block_count = c->d_arf_bcount;
   p.block_off = c->d_arf_boff;
   p.counters = c->d_counters;
@@ -551,7 +552,7 @@ static int arf_generate(gg_ctx *c, const gg_arf_sampling *a, uint64_t n, uint64_
   for (uint64_t done = 0; done < n; done += kArfChunk) {
     p.first = first + done;
     p.n = std::min<uint64_t>(kArfChunk, n - done);
-    if ((st = c->cuda(gg::launch_arf_dataset<real>(s, p, c->d_arf_rows, capacity, c->d_arf_total, c->stream),
+    if ((st = c->cuda(gg::launch_arf_dataset<real>(s, p, c->n_sm, c->d_arf_rows, capacity, c->d_arf_total, c->stream),
                       "ARF dataset launch")))
       return st;
   }

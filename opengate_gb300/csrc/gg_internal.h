@@ -93,13 +93,16 @@ struct StageArgs {
 };
 
 // One launch of the ARF training-row generator (see gg_arf.cu).
+constexpr int kArfBlock = 256;
+
 struct ArfArgs {
   uint64_t seed, first, n;        // samples [first, first + n), Philox stream 1
   double e_min, e_max, cos_theta_max, half_extent[2], russian_roulette;
   int theta_uniform;              // theta = u theta_max instead of cos(theta) uniform
   double theta_max_turn;          // acos(cos_theta_max) / (2 pi)
   float4 *stage;                  // [n] row per sample (w = -1: dropped)
-  unsigned int *block_count;      // [blocks] kept rows per block
+  unsigned long long *next;       // work counter
+  unsigned int *block_count;      // [blocks] kept rows per block of kArfBlock samples
   unsigned long long *block_off;  // [blocks] first output row of each block
   unsigned long long *counters;   // GG_N_COUNTERS slots
 };
@@ -224,7 +227,7 @@ template <typename real>
 size_t slot_scratch_bytes(bool two);
 // Rows of p.n samples appended to rows[*total ...] (capacity rows); *total advances on the device.
 template <typename real>
-cudaError_t launch_arf_dataset(const Scene<real> &s, const ArfArgs &p, float4 *rows, uint64_t capacity,
+cudaError_t launch_arf_dataset(const Scene<real> &s, const ArfArgs &p, int n_sm, float4 *rows, uint64_t capacity,
                                unsigned long long *total, cudaStream_t st);
 template <typename real>
 size_t queue_bytes(size_t cap);
