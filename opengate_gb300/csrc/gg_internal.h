@@ -210,6 +210,10 @@ template <>
 struct PoolShape<double> {
   static constexpr int kBlock = 288, kGang = 3, kRing = 512;
 };
+// (a block has 16 named barriers: number 0 for the block, one for each gang)
+static_assert(PoolShape<float>::kBlock / (32 * PoolShape<float>::kGang) <= 15 &&
+                  PoolShape<double>::kBlock / (32 * PoolShape<double>::kGang) <= 15,
+              "more gangs than named barriers");
 // static shared memory of a pooled kernel with as many event queues, at most
 template <typename real>
 __host__ __device__ constexpr int pool_static(int queues) {

@@ -631,7 +631,7 @@ __device__ __forceinline__ void stream_pair(const Rng &g, uint32_t q, uint32_t &
 // the warp's longest loop.  On return g stands after the accepted trial.
 template <typename real>
 __device__ __forceinline__ int warp_iso_direction_accepted(const Scene<real> &s, RngAhead &g, Photon<real> &ph,
-                                                           bool need, BlockCounters *bc) {
+                                                           bool need, BlockCounters *bc, uint8_t *waiting) {
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t p0 = (g.blk - 1u) * 4u + (uint32_t)g.idx;  // words drawn so far (Rng / RngAhead state)
   const uint32_t max_rej = (uint32_t)s.max_rejection;
@@ -643,8 +643,12 @@ __device__ __forceinline__ int warp_iso_direction_accepted(const Scene<real> &s,
     const unsigned m = __ballot_sync(0xffffffffu, pending);
     if (m == 0u) break;
     const int np = __popc(m);
-    const int r = (int)lane % np;
-    const int owner = (int)__fns(m, 0u, r + 1);
+    const int rk = __popc(m & ((1u << lane) - 1u));  // this history's rank among the waiting ones
+    if (pending) waiting[rk] = (uint8_t)lane;
+    __syncwarp();
+    const int turn = (int)(((float)lane + 0.5f) * __frcp_rn((float)np));  // lane / np
+    const int owner = waiting[(int)lane - turn * np];
+    __syncwarp();
     const uint32_t o_p0 = __shfl_sync(0xffffffffu, p0, owner);
     const uint32_t o_next = __shfl_sync(0xffffffffu, next, owner);
     Rng o = g;  // the owner's stream: key and counter words
@@ -653,7 +657,7 @@ __device__ __forceinline__ int warp_iso_direction_accepted(const Scene<real> &s,
     real op[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) op[a] = __shfl_sync(0xffffffffu, ph.pos[a], owner);
-    const uint32_t q = o_p0 + 2u * (o_next + (uint32_t)((int)lane / np));
+    const uint32_t q = o_p0 + 2u * (o_next + (uint32_t)turn);
     uint32_t wu, wv;
     stream_pair(o, q, wu, wv);
     const real u = (real)(wu >> 8) * R<real>(5.9604644775390625e-08);
@@ -664,7 +668,6 @@ __device__ __forceinline__ int warp_iso_direction_accepted(const Scene<real> &s,
     int src = (int)lane;
     bool won = false;
     if (pending) {
-      const int rk = __popc(m & ((1u << lane) - 1u));  // this history's rank among the waiting ones
       unsigned grp = 0u;
       for (int l = rk; l < 32; l += np) grp |= 1u << l;
       const unsigned hits = am & grp;

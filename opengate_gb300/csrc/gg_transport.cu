@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(256) k_generate(Scene<real> s, KernelArgs a) {
     Photon<real> ph;
     const bool live = i < n;
     if (live) sample_position(s, g, ph, &bc);
-    int st = warp_iso_direction_accepted(s, g, ph, live, &bc);
+    __shared__ uint8_t waiting[256 / 32][32];
+    int st = warp_iso_direction_accepted(s, g, ph, live, &bc, waiting[threadIdx.x >> 5]);
     if (live) {
       uint32_t state = kRecDead, steps = 0;
       if (st != GG_OK) {
