@@ -1388,11 +1388,11 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     const int pool_threads = c->block == gg::kBlock ? 0 : c->block;  // (the default: the kernel's own block size)
     cudaError_t e =
         f64 ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
-                                    sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(tle_run),
-                                    gg::slot_scratch_bytes<double>(two), queues, &plan)
+                                    sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(tle_run, two),
+                                    gg::slot_scratch_bytes<double>(), queues, &plan)
             : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
-                                   sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(tle_run),
-                                   gg::slot_scratch_bytes<float>(two), queues, &plan);
+                                   sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(tle_run, two),
+                                   gg::slot_scratch_bytes<float>(), queues, &plan);
     if (e != cudaSuccess) return c->cuda(e, "transport launch shape");
     if (plan.scratch > c->slot_bytes) {
       dfree(c->d_slot);

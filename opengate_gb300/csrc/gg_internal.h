@@ -224,11 +224,12 @@ template <typename real>
 cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
                       size_t scratch_bytes, int queues, PoolPlan *p);
 int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist);
-// Shared memory of a dose slot (tle: with the track-length estimator); its global scratch (two: the second list of a dose grid).
+// Shared memory of a dose slot (tle: with the track-length estimator; two: a
+// dose grid that scores edep and dose); its global scratch.
 template <typename real>
-size_t dose_slot_bytes(bool tle);
+size_t dose_slot_bytes(bool tle, bool two);
 template <typename real>
-size_t slot_scratch_bytes(bool two);
+size_t slot_scratch_bytes();
 // Rows of p.n samples appended to rows[*total ...] (capacity rows); *total advances on the device.
 template <typename real>
 cudaError_t launch_arf_dataset(const Scene<real> &s, const ArfArgs &p, int n_sm, float4 *rows, uint64_t capacity,

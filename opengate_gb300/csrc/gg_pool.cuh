@@ -358,6 +358,23 @@ struct VoxelList<double> {
 };
 template <typename real>
 using DoseSlot = PhotonSlot<real, VoxelList<real>>;
+// ... with the dose per entry beside it, for a dose grid that scores both; the
+// two lists have the same voxels
+template <typename real>
+struct VoxelListDose {
+  uint32_t vox[kHistList];
+  alignas(16) real acc[kHistList];
+  alignas(16) real dose[kHistList];
+};
+template <>
+struct VoxelListDose<double> {
+  uint32_t vox[kHistList];
+  alignas(16) double acc[kHistList];
+  alignas(16) double dose[kHistList];
+  uint4 pad;
+};
+template <typename real>
+using GridSlot = PhotonSlot<real, VoxelListDose<real>>;
 // ... and, with the track-length estimator, its walk through the voxels: next
 // boundary per axis and path so far, boundary spacing per axis and drawn path,
 // voxel per axis and boundaries crossed.
@@ -377,15 +394,20 @@ struct VoxelWalkList : TlePad<real> {
 template <typename real>
 using TleSlot = PhotonSlot<real, VoxelWalkList<real>>;
 static_assert(sizeof(DoseSlot<float>) % 32 == 16 && sizeof(DoseSlot<double>) % 32 == 16 &&
-                  sizeof(TleSlot<float>) % 32 == 16 && sizeof(TleSlot<double>) % 32 == 16,
+                  sizeof(TleSlot<float>) % 32 == 16 && sizeof(TleSlot<double>) % 32 == 16 &&
+                  sizeof(GridSlot<float>) % 32 == 16 && sizeof(GridSlot<double>) % 32 == 16,
               "odd 16-byte stride");
 static_assert(kHistList == 8, "list_deposit reads the voxels as two 16-byte words");
 
 // A history's voxel list in its slot (the entries of HistList, in their order).
-// list_add(): all voxels are compared at once - a loop over the entries makes
-// the warp wait for its longest list; false: a new voxel, and the list is full.
-template <typename real, typename List>
-__device__ __forceinline__ bool list_add(List &S, int &n, uint32_t v, real e) {
+// list_deposit(): all voxels are compared at once - a loop over the entries makes
+// the warp wait for its longest list.  Returns the entry (-1: nothing to score);
+// flush(k): entry k of a full list into the tallies.
+template <typename real, typename List, typename Flush>
+__device__ __forceinline__ int list_deposit(List &S, int &n, uint32_t v, real e, unsigned int &n_dep,
+                                            unsigned int &n_entries, unsigned int &n_over, Flush &&flush) {
+  if (!(e > R<real>(0))) return -1;
+  ++n_dep;
   const uint4 a = *reinterpret_cast<const uint4 *>(S.vox), b = *reinterpret_cast<const uint4 *>(S.vox + 4);
   const uint32_t u[kHistList] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   int at = n;
@@ -394,36 +416,28 @@ __device__ __forceinline__ bool list_add(List &S, int &n, uint32_t v, real e) {
     if (k < n && u[k] == v) at = k;
   if (at < n) {
     S.acc[at] = S.acc[at] + e;
-    return true;
+    return at;
   }
-  if (n == kHistList) return false;
+  if (n == kHistList) {
+    ++n_over;
+    n_entries += kHistList;
+#pragma unroll 1
+    for (int k = 0; k < kHistList; ++k) flush(k);
+    n = at = 0;
+  }
   S.vox[at] = v;
   S.acc[at] = e;
   n = at + 1;
-  return true;
-}
-template <typename real, typename List>
-__device__ __forceinline__ void list_deposit(List &S, int &n, const Tally<real> &t, uint32_t v, real e,
-                                             unsigned int &n_dep, unsigned int &n_entries, unsigned int &n_over) {
-  if (!(e > R<real>(0))) return;
-  ++n_dep;
-  if (list_add(S, n, v, e)) return;
-  ++n_over;
-  n_entries += kHistList;
-#pragma unroll 1
-  for (int k = 0; k < kHistList; ++k) tally_entry(t, S.vox[k], S.acc[k]);
-  S.vox[0] = v;
-  S.acc[0] = e;
-  n = 1;
+  return at;
 }
 
 // The lists of the warp's ended histories (`n` entries of the lane's slot
 // `slot`) into the tallies: the entries are dealt over the lanes, one each -
 // about 1.5 per history, but the longest of 32 lists has 4 or 5.  ids: 32 *
-// kHistList numbers of the warp's own.  tally_of(slot): the slot's tally.
-template <typename Slot, typename TallyOf>
+// kHistList numbers of the warp's own.  flush(slot, k): its entry k.
+template <typename Slot, typename Flush>
 __device__ __forceinline__ void lists_flush(const Slot *slots, int slot, int n, uint16_t *ids, unsigned lane,
-                                            TallyOf &&tally_of, unsigned int &n_entries) {
+                                            Flush &&flush, unsigned int &n_entries) {
   unsigned end = (unsigned)n;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -439,8 +453,7 @@ __device__ __forceinline__ void lists_flush(const Slot *slots, int slot, int n, 
 #pragma unroll 1
   for (unsigned i = lane; i < total; i += 32u) {
     const unsigned id = ids[i];
-    const Slot &S = slots[id / kHistList];
-    tally_entry(tally_of(S), S.x.vox[id % kHistList], S.x.acc[id % kHistList]);
+    flush(slots[id / kHistList], id % kHistList);
   }
   n_entries += (unsigned)n;
   __syncwarp();
@@ -492,34 +505,5 @@ __device__ __forceinline__ void lists_flush_same(const List &S, int n, const Tal
     }
   }
 }
-
-// The second list of a dose grid that scores dose too, in global memory:
-// [kHistList][slots] sums and voxels.
-template <typename real>
-struct GlobalList {
-  real *ga;
-  uint32_t *gv;
-  size_t slots, at;
-  int n;
-
-  __device__ __forceinline__ void flush(const Tally<real> &t) {
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) tally_entry(t, gv[(size_t)k * slots + at], ga[(size_t)k * slots + at]);
-    n = 0;
-  }
-  __device__ __forceinline__ void deposit(const Tally<real> &t, uint32_t v, real e) {
-    if (!(e > R<real>(0))) return;
-#pragma unroll 1
-    for (int k = 0; k < n; ++k)
-      if (gv[(size_t)k * slots + at] == v) {
-        ga[(size_t)k * slots + at] += e;
-        return;
-      }
-    if (n == kHistList) flush(t);
-    gv[(size_t)n * slots + at] = v;
-    ga[(size_t)n * slots + at] = e;
-    ++n;
-  }
-};
 
 }  // namespace gg

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
-  using Slot = std::conditional_t<TLE, TleSlot<real>, DoseSlot<real>>;
+  using Slot = std::conditional_t<TLE, TleSlot<real>, std::conditional_t<DG == 2, GridSlot<real>, DoseSlot<real>>>;
   constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
   constexpr int kNq = TLE ? kTleQueues : kQueues;
   using Queues = EventQueues<Shape::kRing, kNq>;
@@ -350,10 +350,12 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   Secondary<real> sec;
   sec.base = reinterpret_cast<real *>(args.slot_scratch);
   sec.stride = (int)all_slots;
-  GlobalList<real> ld;
-  ld.ga = sec.base + 6 * (size_t)all_slots;
-  ld.gv = reinterpret_cast<uint32_t *>(ld.ga + kHistList * (size_t)all_slots);
-  ld.slots = all_slots;
+  // an entry of a slot's list into the tallies
+  auto list_entry = [&](const Slot &S, int k) {
+    if constexpr (MULTI) tally_entry(tally_at(args, sg.sims[S.e.w].vox_off, real(0)), S.x.vox[k], S.x.acc[k]);
+    else tally_entry(t, S.x.vox[k], S.x.acc[k]);
+    if constexpr (DG == 2) tally_entry(td, S.x.vox[k], S.x.dose[k]);
+  };
   unsigned int n_wood = 0, n_real = 0, n_dep = 0, n_world = 0, n_ent = 0, n_over = 0, n_esc = 0;
   ItemClaims claims;
   claims.init();
@@ -373,11 +375,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
         n_ent += (unsigned)n_old;
       } else {
         lists_flush(slots, max(k, 0), n_old, reinterpret_cast<uint16_t *>(ahead[threadIdx.x & ~31u]), lane,
-                    [&](const Slot &S) {
-                      if constexpr (MULTI) return tally_at(args, sg.sims[S.e.w].vox_off, real(0));
-                      else return t;
-                    },
-                    n_ent);
+                    list_entry, n_ent);
       }
     }
     if constexpr (TLE) {
@@ -391,16 +389,16 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       Slot &S = slots[k];
       uint4 e = S.e;
       int n_list = (int)((e.z >> kSlList) & 15u);
-      if constexpr (DG == 2) {
-        ld.at = slot0 + (uint32_t)k;
-        ld.n = (int)e.w;
-      }
       auto bind = [&](uint32_t sim) {  // batched simulations: the history's geometry, majorant and tally
         const SimDesc<real> &d = sg.sims[sim];
         bind_geometry(s, d, sg.labels, sg.sim_maj + (size_t)sim * sg.n_e);
         t = tally_at(args, d.vox_off, real(0));
       };
       if constexpr (MULTI) bind(e.w);
+      auto here = [&](int q) {  // (t is the bound simulation's)
+        tally_entry(t, S.x.vox[q], S.x.acc[q]);
+        if constexpr (DG == 2) tally_entry(td, S.x.vox[q], S.x.dose[q]);
+      };
       Photon<real> ph;
       ph.alive = 1;
       uint32_t cw = 0, pv = 0, trials = 0;
@@ -412,7 +410,6 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
       uint32_t *const buf = &S.rng.x;
       if (event == kQRefill) {
         n_list = 0;
-        if constexpr (DG == 2) ld.flush(td);
         uint32_t h, f = kRecDead;
         const bool have = claims.item(Q.tid, h);
         if (have) f = rec.flags[h];
@@ -483,11 +480,14 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           if constexpr (DG > 0) in = dose_voxel(s, ph.pos, v);
           if constexpr (TLE) in = score;
           if (in) {
-            list_deposit(S.x, n_list, t, v, ed, n_dep, n_ent, n_over);
+            const int n_before = n_list;
+            const int at = list_deposit(S.x, n_list, v, ed, n_dep, n_ent, n_over, here);
             if constexpr (DG == 2) {
-              real dd = ed * s.drho_min;
-              dd = dd / s.mat_rho[pmat];
-              ld.deposit(td, v, dd);
+              if (at >= 0) {
+                real dd = ed * s.drho_min;
+                dd = dd / s.mat_rho[pmat];
+                S.x.dose[at] = n_list == n_before ? S.x.dose[at] + dd : dd;  // (one entry more, or only it after a flush)
+              }
             }
           }
           aim = ph.alive;
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
             dest = r == kInteract ? kQInteract : (r == kFly ? kQFly : kQRefill);
           } else if (TLE && ph.e <= s.tle_thr) {
             if (ph.e <= s.tle_emin) {  // the kill energy: the rest is left where the photon is
-              list_deposit(S.x, n_list, t, voxel_of(s, ph.pos), ph.e, n_dep, n_ent, n_over);
+              list_deposit(S.x, n_list, voxel_of(s, ph.pos), ph.e, n_dep, n_ent, n_over, here);
               dest = kQRefill;
             } else {
               if constexpr (TLE) {
@@ -558,7 +558,6 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
               ((uint32_t)sec.has << kSlSec) | ((uint32_t)n_list << kSlList);
         if (pend) e.z |= (pscored ? 1u << kSlImage : 0u) | (trials ? 1u << kSlRetry : 0u);
       }
-      if constexpr (DG == 2) e.w = (uint32_t)ld.n;
       S.e = e;
     }
     if (event == kQRefill) claims.advance(n);
@@ -693,12 +692,12 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
 }
 
 template <typename real>
-size_t dose_slot_bytes(bool tle) {
-  return tle ? sizeof(TleSlot<real>) : sizeof(DoseSlot<real>);
+size_t dose_slot_bytes(bool tle, bool two) {
+  return tle ? sizeof(TleSlot<real>) : (two ? sizeof(GridSlot<real>) : sizeof(DoseSlot<real>));
 }
 template <typename real>
-size_t slot_scratch_bytes(bool two) {
-  return 6 * sizeof(real) + (two ? kHistList * (sizeof(real) + sizeof(uint32_t)) : 0);
+size_t slot_scratch_bytes() {
+  return 6 * sizeof(real);
 }
 
 // Histories a gang claims at a time: an even share of a small run, else the
@@ -718,9 +717,9 @@ template cudaError_t launch_transport<double>(const Scene<double> &, const Kerne
                                               cudaStream_t);
 template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
 template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
-template size_t dose_slot_bytes<float>(bool);
-template size_t dose_slot_bytes<double>(bool);
-template size_t slot_scratch_bytes<float>(bool);
-template size_t slot_scratch_bytes<double>(bool);
+template size_t dose_slot_bytes<float>(bool, bool);
+template size_t dose_slot_bytes<double>(bool, bool);
+template size_t slot_scratch_bytes<float>();
+template size_t slot_scratch_bytes<double>();
 
 }  // namespace gg
