@@ -61,11 +61,11 @@ struct KernelArgs {
   unsigned long long *counters;     // GG_N_COUNTERS slots
   unsigned int *status;             // OR of error codes raised by the kernel
   int chunk;                        // histories claimed per warp refill
-  void *records;                    // primary records of the batch (k_generate -> k_transport)
+  void *records;                    // primary records of the batch (k_generate -> transport)
   size_t rec_cap;                   // records capacity (histories per batch)
   uint64_t rec_first;               // history of record 0 (<= h_begin; a SPECT pass can start later)
-  int refill_min;                   // lanes that must wait for a history before a refill phase (phase kernels)
-  int interact_min;                 // pending collisions that trigger an interaction phase (phase kernels)
+  int refill_min;                   // lanes that must wait before a refill phase (SPECT head stage)
+  int interact_min;                 // pending collisions that trigger its interaction phase
   unsigned long long *acc_d;        // dose grid: fixed-point sum(edep * rho_min / rho) (or null)
   unsigned long long *acc_d2;       // its history-by-history squares (or null)
   void *slot_scratch;               // pooled kernels: PoolPlan::scratch bytes
@@ -192,6 +192,7 @@ __host__ __device__ constexpr size_t hist_list_bytes(int lists, int threads = kB
 // Launch shape of a pooled transport kernel (gg_pool.cuh).
 struct PoolPlan {
   int grid, block, gangs, slots;  // blocks, threads and gangs per block, photon slots per gang
+  int gang_threads;               // (the last gang may have fewer)
   size_t smem, scratch;           // dynamic shared memory; global scratch (KernelArgs::slot_scratch)
 };
 // Threads of a block (one block per SM), warps of a gang, entries of an event

@@ -575,23 +575,24 @@ static __device__ __noinline__ unsigned score_returned(const Scene<real> &s, voi
 // 291-360), made by the split kernel.
 template <typename real, bool SPLIT>
 __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1)
-    k_spect_phantom(const __grid_constant__ Scene<real> sg, KernelArgs args, StageArgs q, int n_slots) {
+    k_spect_phantom(const __grid_constant__ Scene<real> sg, KernelArgs args, StageArgs q, int n_slots,
+                    int gang_threads) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
-  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
+  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang);
   __shared__ __align__(16) unsigned push[kGangs][3 * kQueues];
   __shared__ __align__(16) uint32_t ahead[Shape::kBlock][4];  // EventRng's second block of each thread
   __shared__ uint16_t ring[kGangs][kQueues * Shape::kRing];
   __shared__ unsigned long long s_claim[kGangs];
   Scene<real> s = sg;
   const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
-  const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
-  const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
+  const int gang = (int)threadIdx.x / gang_threads, gang0 = gang * gang_threads;
+  const int gangs = ((int)blockDim.x + gang_threads - 1) / gang_threads;
   // dynamic shared memory: slots of the gangs, tables
   PhantomSlot<real> *const slots = reinterpret_cast<PhantomSlot<real> *>(smem_raw) + gang * n_slots;
   EventQueues<Shape::kRing> Q;
-  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
+  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)gang_threads, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
          (unsigned)n_slots);
   for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) {
     slots[i].e = make_uint4(0u, 0u, 0u, 0u);
@@ -1074,7 +1075,7 @@ static cudaError_t launch_phantom_v(const Scene<real> &s, const KernelArgs &a, c
   static unsigned long long configured = 0;
   cudaError_t e = configure_smem(k_spect_phantom<real, SPLIT>, 227 * 1024, configured);
   if (e != cudaSuccess) return e;
-  k_spect_phantom<real, SPLIT><<<p.grid, p.block, p.smem, st>>>(s, a, q, p.slots);
+  k_spect_phantom<real, SPLIT><<<p.grid, p.block, p.smem, st>>>(s, a, q, p.slots, p.gang_threads);
   return cudaGetLastError();
 }
 

@@ -317,12 +317,12 @@ __device__ __forceinline__ int tle_walk(const Scene<real> &s, TleSlot<real> *slo
 // together: without the sums of equal voxels (lists_flush_same) the atomics of
 // the beam's axis queue at a few L2 slices, 12.2 ms.
 template <typename real, bool MULTI, int DG, bool TLE>
-__global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(Scene<real> sg, KernelArgs args, int n_slots) {
+__global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(Scene<real> sg, KernelArgs args, int n_slots, int gang_threads) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
   using Slot = std::conditional_t<TLE, TleSlot<real>, std::conditional_t<DG == 2, GridSlot<real>, DoseSlot<real>>>;
-  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang), kGang = 32 * Shape::kGang;
+  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang);
   constexpr int kNq = TLE ? kTleQueues : kQueues;
   using Queues = EventQueues<Shape::kRing, kNq>;
   __shared__ __align__(16) unsigned push[kGangs][3 * Queues::kSet];
@@ -331,12 +331,12 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   __shared__ unsigned long long s_claim[kGangs];
   Scene<real> s = sg;
   const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
-  const int gang = (int)threadIdx.x / kGang, gang0 = gang * kGang;
-  const int gangs = ((int)blockDim.x + kGang - 1) / kGang;
+  const int gang = (int)threadIdx.x / gang_threads, gang0 = gang * gang_threads;
+  const int gangs = ((int)blockDim.x + gang_threads - 1) / gang_threads;
   // dynamic shared memory: slots of the gangs, tables
   Slot *const slots = reinterpret_cast<Slot *>(smem_raw) + gang * n_slots;
   Queues Q;
-  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)kGang, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
+  Q.init(gang, threadIdx.x - (unsigned)gang0, min((unsigned)gang_threads, blockDim.x - (unsigned)gang0), ring[gang], push[gang],
          (unsigned)n_slots);
   for (int i = (int)Q.tid; i < n_slots; i += (int)Q.size) slots[i].e = make_uint4(0u, 0u, 0u, 0u);
   stage_tables(sg, s, smem_raw + sizeof(Slot) * (size_t)(gangs * n_slots), bc);
@@ -630,7 +630,7 @@ static cudaError_t launch_pool_v(const Scene<real> &s, const KernelArgs &a, cons
   static unsigned long long configured = 0;
   cudaError_t e = configure_smem(k_transport_pool<real, MULTI, DG, TLE>, 227 * 1024, configured);
   if (e != cudaSuccess) return e;
-  k_transport_pool<real, MULTI, DG, TLE><<<p.grid, p.block, p.smem, st>>>(s, a, p.slots);
+  k_transport_pool<real, MULTI, DG, TLE><<<p.grid, p.block, p.smem, st>>>(s, a, p.slots, p.gang_threads);
   return cudaGetLastError();
 }
 
@@ -678,13 +678,19 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
   const size_t slot = slot_bytes, fixed = pool_static<real>(queues) + table_bytes;
   const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
   while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
-  const int gangs = (threads + kGang - 1) / kGang;
+  // a small run's block has as many gangs as a full one: a photon then waits for fewer others'
+  // events (2e4 / 4e4 / 6e4 histories, us, gangs of kGang: 64^3 water 94 / 100 / 109 -> 85 / 94 /
+  // 96, 128 x 128 x 80 CT 219 / 233 / 244 -> 189 / 211 / 229; from a full block on the same)
+  constexpr int kGangs = Shape::kBlock / kGang;
+  const int gang = room < threads ? kGang : (threads + 32 * kGangs - 1) / (32 * kGangs) * 32;
+  const int gangs = (threads + gang - 1) / gang;
   const int most = std::min(room / gangs, Shape::kRing - 32) / 8 * 8;
   if (most < 8) return cudaErrorInvalidValue;
   const uint64_t share = std::max<uint64_t>((per_sm + gangs - 1) / gangs, 32);
   p->grid = n_sm;
   p->block = threads;
   p->gangs = gangs;
+  p->gang_threads = gang;
   p->slots = (int)std::min<uint64_t>(most, (share + 7) / 8 * 8);
   p->smem = slot * p->slots * gangs + table_bytes;
   p->scratch = (size_t)p->grid * gangs * p->slots * scratch_bytes;
