@@ -33,12 +33,12 @@ import numpy as np  # noqa: E402
 METRIC = "primaries/s at matched sigma (plain GPU transport, CT phantom dose)"
 UNIT = "primaries/s"
 PRIMARIES_PER_STEP = 100_000_000
-TRANSPORT_DRAM_PER_PRIMARY = (407.04e6 + 110.38e6) / 3e6  # bytes, ncu capture of the dose workload
+TRANSPORT_DRAM_PER_PRIMARY = (424.53e6 + 127.51e6) / 3e6  # bytes, ncu capture of the dose workload
 # warp instructions per primary of the dose transport kernels and their active lanes per warp
 # instruction (ncu captures of the same workload, 3e6 primaries: smsp__inst_executed.sum and
-# smsp__thread_inst_executed_per_inst_executed.ratio; phase kernel, compacted wavefront kernel
+# smsp__thread_inst_executed_per_inst_executed.ratio; pooled kernel, compacted wavefront kernel
 # (the latter captured before the history lists moved to shared memory))
-TRANSPORT_ISSUE = {"phased": (1.136376062e9 / 3e6, 8.60), "wavefront": (1.045618891e9 / 3e6, 14.12)}
+TRANSPORT_ISSUE = {"phased": (6.12672716e8 / 3e6, 20.96), "wavefront": (1.045618891e9 / 3e6, 14.12)}
 WORKLOAD = "ct_phantom_256x256x160_1.2mm_ssd100_field10x10_spectrum60_0.1-6MeV"
 
 # SPECT acquisition: CT phantom as attenuation map, Tc-99m activity image,
@@ -1171,7 +1171,7 @@ def run_ours_batched(args, ws, rank, local, dist, use_cuda):
                     "d2h_bytes_per_step": int(d2h)},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak_bw, "unit": "GB/s",
                          "frac": achieved / peak_bw, "traffic": args.traffic, "peak_kind": peak_kind,
-                         "kernel": "k_transport<float, MULTI> (batched transport)",
+                         "kernel": "k_transport_pool<float, MULTI> (batched transport)",
                          "bytes_alg_per_step": bytes_alg, "note": "graph replay time includes source and flush"},
             "cpu_baseline": None,
             "clocks": clk.summary(),
@@ -1351,7 +1351,7 @@ def run_ours_tle(args, ws, rank, local, dist, use_cuda):
             "fp64_error": fp64,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": None, "peak_kind": peak_kind, "kernel": "k_transport<float> (estimator)",
+                         "traffic": None, "peak_kind": peak_kind, "kernel": "k_transport_pool<float, TLE> (estimator)",
                          "bytes_alg_per_step": bytes_alg,
                          "units": {"woodcock_steps": counters["woodcock_steps"],
                                    "tally_entries": counters["tally_entries"], "deposits": counters["deposits"]},
@@ -1473,15 +1473,14 @@ def run_ours(args):
     bytes_alg = 32.0 * counters["woodcock_steps"] + 64.0 * counters["tally_entries"]
     achieved = bytes_alg / (transport_ms / 1e3) / 1e9
     # DRAM traffic of the transport kernel: an ncu capture of the same workload at 3e6
-    # primaries (one launch: dram__bytes_read.sum 478.16 MB + dram__bytes_write.sum
-    # 200.48 MB) scaled by primaries to this launch, unless measured and passed in
+    # primaries (one launch: dram__bytes_read.sum + dram__bytes_write.sum) scaled by primaries to this launch, unless measured and passed in
     traffic = args.traffic if args.traffic is not None else TRANSPORT_DRAM_PER_PRIMARY * n
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
                 "traffic_note": None if args.traffic is not None else
                 "ncu dram bytes of a 3e6-primary launch of this workload, scaled by primaries",
                 "peak_kind": peak_kind,
-                "kernel": "k_transport<float>" if args.transport_kernel == "phased" else "k_wavefront<float>",
+                "kernel": "k_transport_pool<float>" if args.transport_kernel == "phased" else "k_wavefront<float>",
                 "bytes_alg_per_step": bytes_alg,
                 "units": {"woodcock_steps": counters["woodcock_steps"], "tally_entries": counters["tally_entries"],
                           "transport_launches_per_step": transport_launches},
@@ -1584,7 +1583,7 @@ def main():
     ap.add_argument("--seed", type=int, default=20240611)
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--transport-kernel", default="phased", choices=["phased", "wavefront"],
-                    help="dose workload: the phase kernel (default) or the compacted wavefront kernel")
+                    help="dose workload: the pooled kernel (default) or the compacted wavefront kernel")
     ap.add_argument("--no-arf-summary", action="store_true",
                     help="dose workload: skip the reduced spect_arf comparison carried by its line")
     ap.add_argument("--fp64-primaries", type=int, default=10_000_000,

@@ -263,16 +263,16 @@ typedef struct {
   int32_t blocks_per_sm; /* 0 = default */
   int32_t chunk;      /* histories a warp claims per queue fetch, 0 = default */
   int64_t batch;      /* histories per tally batch, 0 = default (2^26; buffers sized to min(batch, run)) */
-  int32_t refill_min;   /* 1..32: lanes waiting for a history that trigger a refill phase (kernels that
-                           carry one photon per thread: SPECT, track-length estimator), 0 = default */
-  int32_t interact_min; /* 1..32: pending collisions that trigger an interaction phase (the same), 0 = default */
+  int32_t refill_min;   /* 1..32: lanes waiting for a photon that trigger a refill phase of the SPECT head
+                           stage (one photon per thread), 0 = default */
+  int32_t interact_min; /* 1..32: pending collisions that trigger its interaction phase, 0 = default */
 } gg_device_opts;
 
 /* Dose transport kernel of gg_run for single simulations with analog scoring
-   (the track-length estimator and batched simulations always use the phase
+   (the track-length estimator and batched simulations always use the pooled
    kernel).  Both give identical results; they differ in speed only. */
 #define GG_KERNEL_WAVEFRONT 0 /* per-block wavefront compacted by event type */
-#define GG_KERNEL_PHASED 1    /* block-synchronous phases, one history per thread (default) */
+#define GG_KERNEL_PHASED 1    /* pooled photons, one kind of event per round of a gang of warps (default) */
 
 int gg_create(const gg_device_opts *opts, gg_ctx **out);
 int gg_destroy(gg_ctx *ctx);
@@ -596,8 +596,9 @@ int gg_get_arf_projection(gg_ctx *ctx, double *counts, double *squared, size_t n
    accumulate: call gg_reset_tally between replays to repeat a step).
    gg_batch_autotune searches the launch configuration of the one persistent
    transport launch that takes the histories of all simulations from one
-   device work counter: first blocks per SM x refill / interaction thresholds,
-   then, at the best of those, the per-warp claim chunk x the batch length
+   device work counter: first blocks per SM (of 256 threads; at most the pooled
+   kernel's block) x refill / interaction thresholds (which that kernel
+   ignores), then, at the best of those, the per-warp claim chunk x the batch length
    (histories per generate / transport / flush sequence).  Every point is
    timed as the median of three gg_batch_run calls; the fastest stays in the
    context (*best, may be NULL) and gg_batch_autotune_result reports the

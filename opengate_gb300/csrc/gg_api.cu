@@ -85,7 +85,7 @@ struct gg_ctx {
   int64_t batch = 1 << 26;
   int refill_min = 8;
   int interact_min = 16;
-  // dose transport kernel of single simulations: the block-synchronous phase kernel (default,
+  // dose transport kernel of single simulations: the pooled kernel (default,
   // also used for the track-length estimator and batches) or the compacted wavefront
   int transport_kernel = GG_KERNEL_PHASED;
   uint64_t last_batch = 0;  // histories per tally batch of the last run (after the overflow cap)
@@ -1348,7 +1348,7 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
                                         : gg::wavefront_smem_bytes<float>(c->n_comp, c->n_e, c->n_mat);
     if (wsmem > 220 * 1024)
       return c->fail(GG_ERR_ARG, "gg_run: tables and photon slots need %zu bytes of shared memory (max 220 KiB); "
-                     "use the phase kernel (gg_set_transport_kernel)", wsmem);
+                     "use the pooled kernel (gg_set_transport_kernel)", wsmem);
     int wbps = 0;
     cudaError_t e = c->precision == GG_PREC_F64 ? gg::wavefront_occupancy<double>(wsmem, wminb, &wbps)
                                                 : gg::wavefront_occupancy<float>(wsmem, wminb, &wbps);

@@ -768,7 +768,7 @@ __device__ __forceinline__ int sample_primary(const Scene<real> &s, G &g, Photon
   return GG_OK;
 }
 
-// Primary records written by k_generate and consumed by k_transport (SoA,
+// Primary records written by k_generate and consumed by k_transport_pool (SoA,
 // one entry per history of the batch).  The state field says how the first
 // transport iteration left the photon; the RNG position lets the transport
 // kernel continue the history's Philox stream exactly where it stopped.

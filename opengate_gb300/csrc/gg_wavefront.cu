@@ -1,6 +1,6 @@
 // gg_wavefront.cu - dose transport as a per-block wavefront compacted by event type.
 //
-// The same transport as k_transport (GateImageNestedParameterisation::
+// The same transport as k_transport_pool (GateImageNestedParameterisation::
 // ComputeMaterial stepping and GateDoseActor scoring, see gg_transport.cu),
 // scheduled differently.  Each 256-thread block owns 256 photon slots whose
 // whole state - position, direction, energy index, Philox stream position,
@@ -10,11 +10,11 @@
 // warp takes up to 32 slots of one queue, so its lanes run one code path, and
 // the warps of a block work independently of each other (no block barrier).
 //
-// Each history still runs the exact operation sequence of k_transport and of
+// Each history still runs the exact operation sequence of k_transport_pool and of
 // the oracle: the first draw of an interaction (the process selection,
 // select_kind) is taken at the end of the flight that found it, which is the
 // same position of the stream; deposits go to the same per-history list and
-// the same fixed-point tallies.  Results are bit-identical to k_transport.
+// the same fixed-point tallies.  Results are bit-identical to k_transport_pool.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kWSlots, MINB) k_wavefront(Scene<real> sg, Ker
   __shared__ int pool_lock;
   __shared__ unsigned long long pool_next, pool_end;  // the block's claimed, unused history offsets
   __shared__ unsigned int stop;                      // a bounded wait ran out
-  // ---- tables in shared memory (as k_transport) ------------------------------
+  // ---- tables in shared memory (as k_transport_pool) ------------------------------
   Scene<real> s = sg;
   size_t table_bytes;
   {
