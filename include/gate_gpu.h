@@ -280,8 +280,8 @@ int gg_destroy(gg_ctx *ctx);
    ctx is NULL) into buf, always NUL-terminated. */
 int gg_last_error(const gg_ctx *ctx, char *buf, size_t len);
 
-/* The tables stay in each transport block's shared memory beside its two
-   per-history voxel lists: sizeof(real) * (n_comp * n_e + n_e + n_mat) +
+/* The tables stay in each transport block's shared memory beside its photons
+   (room for 256 threads' two voxel lists is kept for them): sizeof(real) * (n_comp * n_e + n_e + n_mat) +
    4 * n_mat bytes (16-byte aligned) plus 2 * 8 * 256 * (4 + sizeof(real))
    must not exceed 200 KiB (GG_ERR_ARG otherwise). */
 int gg_upload_tables(gg_ctx *ctx, const gg_tables_desc *tables);

@@ -79,7 +79,11 @@ struct gg_ctx {
   int precision = GG_PREC_F32;
   int block = 256;
   int blocks_per_sm = 0;
-  int chunk = 256;
+  // histories claimed per warp and fetch: large claims leave the last gangs and warps uneven
+  // work (ms at 32 / 64 / 128 / 256: dose grid 5e6 histories 2.06 / 2.06 / 2.06 / 2.13, FP64 1e6
+  // 4.16 / 4.09 / 4.17 / 4.24, head stage of 3e7 decays 2.48 / 2.53 / 2.59 / 2.81, split pass
+  // phantom stage 4.69 / 4.72 / 4.77 / 4.97; CT 1e8 30.9 / 30.7 / 30.7 / 30.7, at 16 38.1)
+  int chunk = 64;
   // histories per batch: large batches keep the persistent grids and the SPECT
   // stage passes busy (2^24 made the 60-position Tc-99m acquisition ~20 % slower)
   int64_t batch = 1 << 26;
@@ -845,7 +849,7 @@ int gg_upload_tables(gg_ctx *c, const gg_tables_desc *t) {
   char msg[160];
   if (gg::check_tables(t, msg, sizeof(msg))) return c->fail(GG_ERR_ARG, "gg_upload_tables: %s", msg);
   size_t nce = (size_t)t->n_comp * t->n_e;
-  // tables plus the transport block's two per-history voxel lists
+  // tables plus the least room kept for the transport block's photons (two voxel lists of 256 threads)
   size_t need = c->precision == GG_PREC_F64
                     ? gg::transport_smem_bytes<double>(t->n_comp, t->n_e, t->n_mat) + gg::hist_list_bytes<double>(2)
                     : gg::transport_smem_bytes<float>(t->n_comp, t->n_e, t->n_mat) + gg::hist_list_bytes<float>(2);

@@ -183,8 +183,8 @@ __host__ __device__ inline size_t transport_smem_bytes(int n_comp, int n_e, int 
   return (b + 15) & ~(size_t)15;
 }
 
-// Shared memory of `lists` per-history voxel lists of a block of `threads`
-// (one column per thread; the track-length estimator's kernel).
+// Shared memory of `lists` per-history voxel lists of `threads` histories: the
+// room that the largest tables leave to a pooled kernel's photons.
 template <typename real>
 __host__ __device__ constexpr size_t hist_list_bytes(int lists, int threads = kBlock) {
   return (size_t)lists * kHistList * (size_t)threads * (sizeof(uint32_t) + sizeof(real));

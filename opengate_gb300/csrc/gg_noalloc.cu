@@ -294,7 +294,7 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
     a.acc_e2 = d_edep2 ? (unsigned long long *)(b + L.acc_e2) : nullptr;
     a.counters = (unsigned long long *)(b + L.counters);
     a.status = (unsigned int *)(b + L.status);
-    a.chunk = gg::pool_chunk(plan, 256, most);
+    a.chunk = gg::pool_chunk(plan, 64, most);
     a.slot_scratch = b + L.slots;
     a.records = b + L.records;
     a.rec_cap = (size_t)GG_NOALLOC_BATCH;
