@@ -195,31 +195,31 @@ struct PoolPlan {
   int gang_threads;               // (the last gang may have fewer)
   size_t smem, scratch;           // dynamic shared memory; global scratch (KernelArgs::slot_scratch)
 };
-// Threads of a block (one block per SM), warps of a gang, entries of an event
-// queue's ring (more than a gang's slots).  Measured on the 256 x 256 x 160 CT,
+// Threads of a block (one block per SM), warps of a full block's gang, most gangs
+// of a block, entries of an event queue's ring (more than a gang's slots).  Measured on the 256 x 256 x 160 CT,
 // 1e8 histories (transport ms): gangs of 2 / 3 / 4 / 6 / 12 warps of 24: 37.9 /
 // - / 33.5 / 32.5 / 34.6 (small gangs fetch more instructions, large ones wait
 // at their barrier); 16 / 18 / 20 / 24 warps in gangs of 4 / 3 / 4 / 4: 32.4 /
-// 30.4 / 30.4 / 33.5 (more warps leave fewer slots each).  FP64, 128 x 128 x 80
+// 30.4 / 30.4 / 33.5 (more warps leave fewer slots each); 20 warps in gangs of
+// 4 / 5: 30.7 / 30.8, the phantom stage of 3e7 decays 13.0 / 12.5, the track-length
+// estimator 6.7 / 6.5 (24 in gangs of 4: 14.9, 7.2).  FP64, 128 x 128 x 80
 // CT, 1e6 histories: 8 / 9 / 12 / 16 warps in gangs of 4 / 3 / 4 / 8: 4.64 /
 // 4.22 / 4.86 / 5.16 ms (FP64 units bound it: full rounds count, not warps).
 template <typename real>
 struct PoolShape {
-  static constexpr int kBlock = 640, kGang = 4, kRing = 512;
+  static constexpr int kBlock = 640, kGang = 5, kGangs = 5, kRing = 512;
 };
 template <>
 struct PoolShape<double> {
-  static constexpr int kBlock = 288, kGang = 3, kRing = 512;
+  static constexpr int kBlock = 288, kGang = 3, kGangs = 3, kRing = 512;
 };
 // (a block has 16 named barriers: number 0 for the block, one for each gang)
-static_assert(PoolShape<float>::kBlock / (32 * PoolShape<float>::kGang) <= 15 &&
-                  PoolShape<double>::kBlock / (32 * PoolShape<double>::kGang) <= 15,
-              "more gangs than named barriers");
+static_assert(PoolShape<float>::kGangs <= 15 && PoolShape<double>::kGangs <= 15, "more gangs than named barriers");
 // static shared memory of a pooled kernel with as many event queues, at most
 template <typename real>
 __host__ __device__ constexpr int pool_static(int queues) {
   using P = PoolShape<real>;
-  return 1024 + 16 * P::kBlock + (P::kBlock / (32 * P::kGang)) * (2 * queues * P::kRing + (queues > 4 ? 112 : 64));
+  return 1024 + 16 * P::kBlock + P::kGangs * (2 * queues * P::kRing + (queues > 4 ? 112 : 64));
 }
 template <typename real>
 cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,

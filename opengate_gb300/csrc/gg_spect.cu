@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
-  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang);
+  constexpr int kGangs = Shape::kGangs;
   __shared__ __align__(16) unsigned push[kGangs][3 * kQueues];
   __shared__ __align__(16) uint32_t ahead[Shape::kBlock][4];  // EventRng's second block of each thread
   __shared__ uint16_t ring[kGangs][kQueues * Shape::kRing];

@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
   __shared__ BlockCounters bc;
   using Shape = PoolShape<real>;
   using Slot = std::conditional_t<TLE, TleSlot<real>, std::conditional_t<DG == 2, GridSlot<real>, DoseSlot<real>>>;
-  constexpr int kGangs = Shape::kBlock / (32 * Shape::kGang);
+  constexpr int kGangs = Shape::kGangs;
   constexpr int kNq = TLE ? kTleQueues : kQueues;
   using Queues = EventQueues<Shape::kRing, kNq>;
   __shared__ __align__(16) unsigned push[kGangs][3 * Queues::kSet];
@@ -678,11 +678,12 @@ cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uin
   const size_t slot = slot_bytes, fixed = pool_static<real>(queues) + table_bytes;
   const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
   while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
-  // a small run's block has as many gangs as a full one: a photon then waits for fewer others'
+  // a small run's block has as many gangs as may be: a photon then waits for fewer others'
   // events (2e4 / 4e4 / 6e4 histories, us, gangs of kGang: 64^3 water 94 / 100 / 109 -> 85 / 94 /
   // 96, 128 x 128 x 80 CT 219 / 233 / 244 -> 189 / 211 / 229; from a full block on the same)
-  constexpr int kGangs = Shape::kBlock / kGang;
-  const int gang = room < threads ? kGang : (threads + 32 * kGangs - 1) / (32 * kGangs) * 32;
+  const int gang = room < threads || threads == Shape::kBlock
+                       ? kGang
+                       : (threads + 32 * Shape::kGangs - 1) / (32 * Shape::kGangs) * 32;
   const int gangs = (threads + gang - 1) / gang;
   const int most = std::min(room / gangs, Shape::kRing - 32) / 8 * 8;
   if (most < 8) return cudaErrorInvalidValue;
