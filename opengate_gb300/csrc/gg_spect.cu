@@ -573,6 +573,9 @@ static __device__ __noinline__ unsigned score_returned(const Scene<real> &s, voi
 // there, and every Compton up to the maximum level and every Rayleigh
 // scattering asks for split copies (GateScatterSplittingFreeFlightOptrActor.cpp:
 // 291-360), made by the split kernel.
+// Bound by instruction issue and latency (46 % of issue slots, 21 active lanes):
+// Tc-99m in the CT phantom, 3e7 decays, 25.0 -> 12.5 ms against one photon per thread with
+// block-wide phases.
 template <typename real, bool SPLIT>
 __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1)
     k_spect_phantom(const __grid_constant__ Scene<real> sg, KernelArgs args, StageArgs q, int n_slots,

@@ -300,9 +300,9 @@ __device__ __forceinline__ int tle_walk(const Scene<real> &s, TleSlot<real> *slo
 // The order of operations inside each history, hence its result, does not
 // depend on which lane or round executes them.
 // Bound by instruction issue and by the gangs' barrier: 256 x 256 x 160 CT, 1e8
-// histories to 6 MeV, 47.9 -> 30.4 ms against one photon per thread with block-wide phases
+// histories to 6 MeV, 47.9 -> 30.8 ms against one photon per thread with block-wide phases
 // (203 warp instructions per history at 21.5 active lanes; 379 at 8.6); 24
-// batched simulations 22.8 -> 14.1 ms, FP64 9.2 -> 4.2 ms per 1e6.
+// batched simulations 22.8 -> 14.3 ms, FP64 9.2 -> 4.1 ms per 1e6.
 // MULTI: batched simulations; DG: dose tally on a grid of its own (1: edep,
 // 2: edep and dose), Scene::dgrid; TLE: track-length estimator
 // (GateTLEDoseActor::ScoreTLEDepositStep,
@@ -311,7 +311,7 @@ __device__ __forceinline__ int tle_walk(const Scene<real> &s, TleSlot<real> *slo
 // voxel its flights cross, and its interactions deposit nothing
 // (GateTLEDoseActor.cpp:236-243).  Such a flight is two kinds of event: its path
 // is drawn, then walked kTleSteps boundaries a round.  64^3 voxels of 2 mm,
-// 3e6 photons of 1 MeV in a pencil beam (81 voxels each): 13.5 -> 6.9 ms
+// 3e6 photons of 1 MeV in a pencil beam (81 voxels each): 13.5 -> 6.5 ms
 // against one photon per thread with each path walked at once (2088 warp
 // instructions per history at 7.4 lanes; now 880 at 25).  Two things count
 // together: without the sums of equal voxels (lists_flush_same) the atomics of
