@@ -506,4 +506,108 @@ __device__ __forceinline__ void lists_flush_same(const List &S, int n, const Tal
   }
 }
 
+// Boundaries a walk of the track-length estimator crosses in one round: their
+// label loads are in flight together, but a path's last round leaves lanes idle
+// (2 / 3 / 4 / 5 / 6 / 8 boundaries: 9.5 / 7.8 / 6.9 / 7.1 / 7.0 / 7.5 ms, the
+// workload of k_transport_pool).
+constexpr int kTleSteps = 4;
+static_assert(kTleSteps <= kHistList, "the list holds what is left of a round after a flush");
+
+template <typename real>
+__device__ __forceinline__ void tle_store(VoxelWalkList<real> &X, const VoxelWalk<real> &w, real sd) {
+  X.tn = Real4<real>{w.tn[0], w.tn[1], w.tn[2], w.tc};
+  X.td = Real4<real>{w.td[0], w.td[1], w.td[2], sd};
+  X.it = make_int4(w.i[0], w.i[1], w.i[2], w.k);
+}
+
+// One round of the estimator's walks (slot k of each lane, -1: none); the
+// slot's next event.  The warp calls it together; a lane without a slot reads
+// slot 0, which may never have held a photon, so nothing of it becomes an address.
+template <typename real>
+__device__ __forceinline__ int tle_walk(const Scene<real> &s, TleSlot<real> *slots, int k, unsigned lane,
+                                        const Tally<real> &t, unsigned int &n_dep, unsigned int &n_ent,
+                                        unsigned int &n_over) {
+  TleSlot<real> &S = slots[max(k, 0)];
+  const uint4 e = S.e;
+  const Real4<real> b = S.b, tn = S.x.tn, td = S.x.td;
+  const int4 it = S.x.it;
+  VoxelWalk<real> w{{tn.x, tn.y, tn.z}, {td.x, td.y, td.z}, tn.w, {it.x, it.y, it.z}, it.w};
+  const real d[3] = {b.x, b.y, b.z}, len = td.w < S.a.w ? td.w : S.a.w;
+  EIdx<real> ei;
+  ei.fe = S.c.z;
+  ei.ie = k >= 0 ? (int)(real_bits(S.c.w) & 0xffffu) : 0;
+  // the crossings, then their labels with all loads in flight, then the energies
+  uint32_t v[kTleSteps];
+  real ed[kTleSteps];
+  bool more = k >= 0;
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    v[j] = 0u;
+    ed[j] = R<real>(0);
+    if (more) more = w.step(s, d, len, v[j], ed[j]);
+  }
+  int m[kTleSteps];
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) m[j] = (int)__ldg(s.labels + v[j]);
+  int last = -1;
+  real mu_e = R<real>(0);
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    if (m[j] != last) {
+      last = m[j];
+      real mu = interp_row(s.muen + (size_t)s.mat_comp[last] * s.n_e, ei);
+      mu = s.mat_rho[last] * mu;
+      mu_e = b.w * mu;
+    }
+    ed[j] = ed[j] > R<real>(0) ? mu_e * ed[j] : R<real>(0);
+  }
+  // into the list: a walk never comes back to a voxel, so only the entries from
+  // before this round can be a crossing's voxel, and none once the list is flushed
+  int n = (int)((e.z >> kSlList) & 15u), n_old = n;
+  const uint4 ua = *reinterpret_cast<const uint4 *>(S.x.vox), ub = *reinterpret_cast<const uint4 *>(S.x.vox + 4);
+  const uint32_t u[kHistList] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+  bool full = false;
+#pragma unroll
+  for (int j = 0; j < kTleSteps; ++j) {
+    if (ed[j] > R<real>(0) && !full) {
+      int at = n;
+#pragma unroll
+      for (int q = 0; q < kHistList; ++q)
+        if (q < n_old && u[q] == v[j]) at = q;
+      if (at == kHistList) {
+        full = true;
+      } else {
+        const bool add = at == n;
+        S.x.vox[at] = v[j];
+        S.x.acc[at] = add ? ed[j] : S.x.acc[at] + ed[j];
+        n += add ? 1 : 0;
+        ++n_dep;
+        ed[j] = R<real>(0);
+      }
+    }
+  }
+  __syncwarp();
+  if (__any_sync(0xffffffffu, full)) {
+    lists_flush_same(S.x, full ? n : 0, t, lane);
+    if (full) {
+      ++n_over;
+      n_ent += kHistList;
+      n = 0;
+#pragma unroll
+      for (int j = 0; j < kTleSteps; ++j)
+        if (ed[j] > R<real>(0)) {
+          S.x.vox[n] = v[j];
+          S.x.acc[n] = ed[j];
+          ++n;
+          ++n_dep;
+        }
+    }
+  }
+  if (k < 0) return kQNone;
+  S.x.tn = Real4<real>{w.tn[0], w.tn[1], w.tn[2], w.tc};
+  S.x.it = make_int4(w.i[0], w.i[1], w.i[2], w.k);
+  S.e.z = (e.z & ~(15u << kSlList)) | ((uint32_t)n << kSlList);
+  return more ? kQWalk : kQFly;
+}
+
 }  // namespace gg
