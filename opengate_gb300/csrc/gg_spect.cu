@@ -29,6 +29,7 @@
 #include "gg_pool.cuh"
 #include "gg_queue.cuh"
 #include "gg_spect.cuh"
+#include "gg_split.h"
 
 namespace gg {
 
@@ -218,14 +219,13 @@ struct TrialFilter {
 
 // What a warp of the split kernel keeps in shared memory.
 constexpr int kSplitBatch = 32;  // requests at a time
-constexpr int kSplitPend = 64;
 struct SplitWarp {
   TrialFilter f[kSplitBatch];  // the requests' constants, and their streams
   uint32_t h0[kSplitBatch], h1[kSplitBatch], stream[kSplitBatch];
   // copies rejected so far, waiting for their next trial: copy of the batch | trial << 20
-  uint32_t retry[kSplitPend], word3[kSplitPend];  // (word 3 of its stream)
+  uint32_t retry[kSplitRetry], word3[kSplitRetry];  // (word 3 of its stream)
   // copies of the batch whose trial the filter leaves open: copy | trial << 20
-  uint32_t open[kSplitPend];
+  uint32_t open[kSplitOpen];
 };
 static_assert(GG_MAX_SPLITTING * kSplitBatch < (1 << 20) && kLoopCap < (1 << 12), "a retry packs copy and trial");
 
@@ -356,10 +356,9 @@ __global__ void __launch_bounds__(256) k_spect_split(Scene<real> s, KernelArgs a
     uint32_t fr = lane / per, fc = lane - fr * per;  // request and copy of copy next + lane
     int nr = 0, no = 0;                              // copies waiting in P.retry, P.open (the same in every lane)
     for (;;) {
-      const bool last = next >= total;
-      if (no >= 32 || (last && nr == 0)) {
-        // ---- a round of exact trials
-        if (no == 0) break;
+      const SplitRound round = split_round(nr, no, next >= total);
+      if (round == kSplitDone) break;
+      if (round == kSplitExactTrials) {
         const int n = min(no, 32);
         no -= n;
         bool live = false, again = false;
@@ -415,10 +414,10 @@ __global__ void __launch_bounds__(256) k_spect_split(Scene<real> s, KernelArgs a
         __syncwarp();
         continue;
       }
-      // ---- a round of filtered trials: of rejected copies when 32 wait (or no other is left), else first ones
+      // ---- a round of filtered trials: of rejected copies, or first ones
       bool on;
       uint32_t r = 0, c = 0, t = 0, w3 = 0;
-      if (nr >= 32 || last) {
+      if (round == kSplitRetries) {
         const int n = min(nr, 32);
         nr -= n;
         on = (int)lane < n;
