@@ -259,8 +259,10 @@ typedef struct gg_ctx gg_ctx;
 typedef struct {
   int32_t device;     /* CUDA device ordinal */
   int32_t precision;  /* GG_PREC_F32 or GG_PREC_F64 */
-  int32_t block_size; /* 0 = default */
-  int32_t blocks_per_sm; /* 0 = default */
+  int32_t block_size; /* threads per block of the SPECT head stage and of the walks to it, a multiple of 32
+                         up to 256, 0 = default (256); the pooled kernels' blocks are their own */
+  int32_t blocks_per_sm; /* register budget of the SPECT head stage for as many blocks of 256 threads per SM, 2
+                            (also for 1) to 4; the pooled kernels' block has at most as many threads; 0 = default */
   int32_t chunk;      /* histories a warp claims per queue fetch, 0 = default */
   int64_t batch;      /* histories per tally batch, 0 = default (2^26; buffers sized to min(batch, run)) */
   int32_t refill_min;   /* 1..32: lanes waiting for a photon that trigger a refill phase of the SPECT head

@@ -1389,12 +1389,11 @@ static int run_impl(gg_ctx *c, uint64_t n, uint64_t seed, uint64_t first, bool c
     const bool f64 = c->precision == GG_PREC_F64, sp = c->have_spect;
     const bool two = c->dgrid_on && c->ddose && !c->have_batch && !sp;
     const int queues = tle_run ? 5 : 4;  // (the estimator's walks are events of their own)
-    const int pool_threads = c->block == gg::kBlock ? 0 : c->block;  // (the default: the kernel's own block size)
     cudaError_t e =
-        f64 ? gg::pool_plan<double>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
+        f64 ? gg::pool_plan<double>(c->device, smem, c->blocks_per_sm, cap,
                                     sp ? gg::phantom_slot_bytes<double>() : gg::dose_slot_bytes<double>(tle_run, two),
                                     gg::slot_scratch_bytes<double>(), queues, &plan)
-            : gg::pool_plan<float>(c->device, smem, pool_threads, c->blocks_per_sm, cap,
+            : gg::pool_plan<float>(c->device, smem, c->blocks_per_sm, cap,
                                    sp ? gg::phantom_slot_bytes<float>() : gg::dose_slot_bytes<float>(tle_run, two),
                                    gg::slot_scratch_bytes<float>(), queues, &plan);
     if (e != cudaSuccess) return c->cuda(e, "transport launch shape");

@@ -3,6 +3,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 
@@ -221,8 +222,48 @@ __host__ __device__ constexpr int pool_static(int queues) {
   using P = PoolShape<real>;
   return 1024 + 16 * P::kBlock + P::kGangs * (2 * queues * P::kRing + (queues > 4 ? 112 : 64));
 }
+// Launch shape of a pooled run: one block per SM.  More slots per thread keep
+// the rounds full, so they take all shared memory beside the tables, but no
+// more than the run has histories for.  blocks: of the options, resident blocks
+// per SM of 256 threads each, 0 for the kernel's register budget; as with the
+// register budgets of the kernels that have several, 1 stands for 2 (1e7
+// histories, 128 x 128 x 80 CT, 256 / 512 / 640 threads: 6.16 / 4.16 / 3.95 ms).
+// The options' block_size means nothing here: 32 / 64 / 128 / 224 threads per SM
+// take 36.6 / 19.3 / 10.3 / 6.8 ms.  slot_bytes, scratch_bytes: of one slot, shared
+// and global.  False: the tables leave no room.
 template <typename real>
-cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
+inline bool pool_shape(int n_sm, size_t optin, size_t table_bytes, int blocks, uint64_t n_hist, size_t slot_bytes,
+                       size_t scratch_bytes, int queues, PoolPlan *p) {
+  using Shape = PoolShape<real>;
+  constexpr int kGang = 32 * Shape::kGang;
+  const uint64_t per_sm = (n_hist + n_sm - 1) / n_sm;
+  int threads = Shape::kBlock;
+  if (blocks > 0) threads = std::min(threads, 256 * std::max(std::min(blocks, 4), 2));
+  threads = (int)std::min<uint64_t>(threads, (per_sm + 31) / 32 * 32);
+  const size_t fixed = pool_static<real>(queues) + table_bytes;
+  const int room = optin > fixed ? (int)((optin - fixed) / slot_bytes) : 0;
+  while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
+  // a small run's block has as many gangs as may be: a photon then waits for fewer others'
+  // events (2e4 / 4e4 / 6e4 histories, us, gangs of kGang: 64^3 water 94 / 100 / 109 -> 85 / 94 /
+  // 96, 128 x 128 x 80 CT 219 / 233 / 244 -> 189 / 211 / 229; from a full block on the same)
+  const int gang = room < threads || threads == Shape::kBlock
+                       ? kGang
+                       : (threads + 32 * Shape::kGangs - 1) / (32 * Shape::kGangs) * 32;
+  const int gangs = (threads + gang - 1) / gang;
+  const int most = std::min(room / gangs, Shape::kRing - 32) / 8 * 8;
+  if (most < 8) return false;
+  const uint64_t share = std::max<uint64_t>((per_sm + gangs - 1) / gangs, 32);
+  p->grid = n_sm;
+  p->block = threads;
+  p->gangs = gangs;
+  p->gang_threads = gang;
+  p->slots = (int)std::min<uint64_t>(most, (share + 7) / 8 * 8);
+  p->smem = slot_bytes * p->slots * gangs + table_bytes;
+  p->scratch = (size_t)p->grid * gangs * p->slots * scratch_bytes;
+  return true;
+}
+template <typename real>
+cudaError_t pool_plan(int device, size_t table_bytes, int blocks, uint64_t n_hist, size_t slot_bytes,
                       size_t scratch_bytes, int queues, PoolPlan *p);
 int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist);
 // Shared memory of a dose slot (tle: with the track-length estimator; two: a

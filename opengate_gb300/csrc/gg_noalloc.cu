@@ -280,7 +280,7 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
     size_t smem = gg::transport_smem_bytes<float>(t->n_comp, t->n_e, t->n_mat);
     const uint64_t most = n_histories < (uint64_t)GG_NOALLOC_BATCH ? n_histories : (uint64_t)GG_NOALLOC_BATCH;
     gg::PoolPlan plan{};
-    if ((e = gg::pool_plan<float>(device, smem, 0, 0, most, gg::dose_slot_bytes<float>(false, false),
+    if ((e = gg::pool_plan<float>(device, smem, 0, most, gg::dose_slot_bytes<float>(false, false),
                                    gg::slot_scratch_bytes<float>(), 4, &plan)) != cudaSuccess) {
       rc = fail(err, err_len, GG_ERR_CUDA, "launch shape: %s", cudaGetErrorString(e));
       break;

@@ -553,46 +553,16 @@ cudaError_t launch_flush(unsigned long long *acc_e, unsigned long long *acc_e2, 
   return cudaGetLastError();
 }
 
-// Launch shape of a pooled run: one block per SM.  More slots per thread keep
-// the rounds full, so they take all shared memory beside the tables, but no
-// more than the run has histories for.  block, blocks: most threads per block
-// and resident blocks per SM (of 256 threads) of the options, 0 for the
-// kernel's register budget; slot_bytes, scratch_bytes: of one slot, shared and global.
 template <typename real>
-cudaError_t pool_plan(int device, size_t table_bytes, int block, int blocks, uint64_t n_hist, size_t slot_bytes,
+cudaError_t pool_plan(int device, size_t table_bytes, int blocks, uint64_t n_hist, size_t slot_bytes,
                       size_t scratch_bytes, int queues, PoolPlan *p) {
   int n_sm = 0, optin = 0;
   cudaError_t e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   if (e != cudaSuccess) return e;
-  using Shape = PoolShape<real>;
-  constexpr int kGang = 32 * Shape::kGang;
-  const uint64_t per_sm = (n_hist + n_sm - 1) / n_sm;
-  int threads = Shape::kBlock;
-  if (blocks > 0) threads = std::min(threads, 256 * blocks);
-  if (block > 0) threads = std::min(threads, block);
-  threads = (int)std::min<uint64_t>(threads, (per_sm + 31) / 32 * 32);
-  const size_t slot = slot_bytes, fixed = pool_static<real>(queues) + table_bytes;
-  const int room = (size_t)optin > fixed ? (int)(((size_t)optin - fixed) / slot) : 0;
-  while (threads > kGang && room < threads) threads -= kGang;  // (large tables: fewer gangs)
-  // a small run's block has as many gangs as may be: a photon then waits for fewer others'
-  // events (2e4 / 4e4 / 6e4 histories, us, gangs of kGang: 64^3 water 94 / 100 / 109 -> 85 / 94 /
-  // 96, 128 x 128 x 80 CT 219 / 233 / 244 -> 189 / 211 / 229; from a full block on the same)
-  const int gang = room < threads || threads == Shape::kBlock
-                       ? kGang
-                       : (threads + 32 * Shape::kGangs - 1) / (32 * Shape::kGangs) * 32;
-  const int gangs = (threads + gang - 1) / gang;
-  const int most = std::min(room / gangs, Shape::kRing - 32) / 8 * 8;
-  if (most < 8) return cudaErrorInvalidValue;
-  const uint64_t share = std::max<uint64_t>((per_sm + gangs - 1) / gangs, 32);
-  p->grid = n_sm;
-  p->block = threads;
-  p->gangs = gangs;
-  p->gang_threads = gang;
-  p->slots = (int)std::min<uint64_t>(most, (share + 7) / 8 * 8);
-  p->smem = slot * p->slots * gangs + table_bytes;
-  p->scratch = (size_t)p->grid * gangs * p->slots * scratch_bytes;
-  return cudaSuccess;
+  return pool_shape<real>(n_sm, (size_t)optin, table_bytes, blocks, n_hist, slot_bytes, scratch_bytes, queues, p)
+             ? cudaSuccess
+             : cudaErrorInvalidValue;
 }
 
 template <typename real>
@@ -619,8 +589,8 @@ template cudaError_t launch_generate<double>(const Scene<double> &, const Kernel
 template cudaError_t launch_transport<float>(const Scene<float> &, const KernelArgs &, const PoolPlan &, cudaStream_t);
 template cudaError_t launch_transport<double>(const Scene<double> &, const KernelArgs &, const PoolPlan &,
                                               cudaStream_t);
-template cudaError_t pool_plan<float>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
-template cudaError_t pool_plan<double>(int, size_t, int, int, uint64_t, size_t, size_t, int, PoolPlan *);
+template cudaError_t pool_plan<float>(int, size_t, int, uint64_t, size_t, size_t, int, PoolPlan *);
+template cudaError_t pool_plan<double>(int, size_t, int, uint64_t, size_t, size_t, int, PoolPlan *);
 template size_t dose_slot_bytes<float>(bool, bool);
 template size_t dose_slot_bytes<double>(bool, bool);
 template size_t slot_scratch_bytes<float>();

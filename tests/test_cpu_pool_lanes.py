@@ -25,3 +25,8 @@ def _run(name, tmp_path, headers):
 def test_walk_of_a_lane_without_a_slot_reads_no_table_out_of_range(tmp_path, cuda_headers):
     r = _run("walk_idle_lane", tmp_path, cuda_headers)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
+
+
+def test_launch_shapes(tmp_path, cuda_headers):
+    r = _run("pool_shape", tmp_path, cuda_headers)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
