@@ -598,11 +598,11 @@ int gg_get_arf_projection(gg_ctx *ctx, double *counts, double *squared, size_t n
    accumulate: call gg_reset_tally between replays to repeat a step).
    gg_batch_autotune searches the launch configuration of the one persistent
    transport launch that takes the histories of all simulations from one
-   device work counter: first blocks per SM (of 256 threads; at most the pooled
-   kernel's block) x refill / interaction thresholds (which that kernel
-   ignores), then, at the best of those, the per-warp claim chunk x the batch length
-   (histories per generate / transport / flush sequence).  Every point is
-   timed as the median of three gg_batch_run calls; the fastest stays in the
+   device work counter: every launch shape of the pooled kernel (blocks per SM
+   of 256 threads, as far as they differ) x the per-warp claim chunk x the batch
+   length (histories per generate / transport / flush sequence).  Every point is
+   timed as the median of three gg_batch_run calls; the fastest, the context's own
+   when none is faster, stays in the
    context (*best, may be NULL) and gg_batch_autotune_result reports the
    search (points timed, the winner's median / min / max); images are reset
    afterwards.

@@ -21,6 +21,7 @@
 #include "../../include/gate_gpu.h"
 #include "gg_device.cuh"
 #include "gg_internal.h"
+#include "gg_tune.h"
 #include "gg_validate.h"
 #include "gg_mlp.cuh"
 
@@ -2246,9 +2247,15 @@ int gg_batch_autotune(gg_ctx *c, gg_device_opts *best) {
   cudaSetDevice(c->device);
   if (!c->have_batch || !c->have_tally) return c->fail(GG_ERR_STATE, "gg_batch_autotune: call gg_batch_setup first");
   constexpr int kRep = 3;
-  int st = GG_OK;
-  // median / min / max of kRep device timings of the current configuration
-  auto time_point = [&](double stats[3]) -> int {
+  const gg::TunePoint before{c->blocks_per_sm, c->chunk, c->batch};
+  auto use = [&](const gg::TunePoint &p) {
+    c->blocks_per_sm = p.blocks;
+    c->chunk = p.chunk;
+    c->batch = p.batch;
+  };
+  // median / min / max of kRep device timings of a configuration
+  auto time_point = [&](const gg::TunePoint &p, double stats[3]) -> int {
+    use(p);
     double t[kRep];
     for (int r = 0; r < kRep; ++r) {
       int s2;
@@ -2259,68 +2266,21 @@ int gg_batch_autotune(gg_ctx *c, gg_device_opts *best) {
     stats[0] = t[kRep / 2];
     stats[1] = t[0];
     stats[2] = t[kRep - 1];
-    ++c->tune.points;
     return GG_OK;
   };
+  const int block = c->precision == GG_PREC_F64 ? gg::PoolShape<double>::kBlock : gg::PoolShape<float>::kBlock;
+  gg::TuneSearch found;
   c->tune = gg_autotune_result{};
-  c->tune.repeats = kRep;
-  double cur[3];
-  if ((st = time_point(cur))) return st;
-  c->tune.default_median_ms = cur[0];
-  double bst[3] = {cur[0], cur[1], cur[2]};
-  // the starting configuration as run_impl resolves it (0 blocks per SM = its default)
-  int bm = c->blocks_per_sm > 0 ? std::min(c->blocks_per_sm, 4) : (c->precision == GG_PREC_F64 || c->have_batch ? 2 : 4);
-  int br = c->refill_min, bi = c->interact_min, bc = c->chunk;
-  int64_t bb = c->batch;
-  // stage 1: resident blocks per SM x phase thresholds
-  const int minbs[3] = {2, 3, 4};
-  const int thresholds[3][2] = {{8, 16}, {4, 8}, {12, 24}};
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) {
-      c->blocks_per_sm = minbs[a];
-      c->refill_min = thresholds[b][0];
-      c->interact_min = thresholds[b][1];
-      double t[3];
-      if ((st = time_point(t))) return st;
-      if (t[0] < bst[0]) {
-        std::copy(t, t + 3, bst);
-        bm = minbs[a];
-        br = thresholds[b][0];
-        bi = thresholds[b][1];
-      }
-    }
-  c->blocks_per_sm = bm;
-  c->refill_min = br;
-  c->interact_min = bi;
-  // stage 2: per-warp claim chunk x batch length (all histories in one
-  // generate / transport / flush sequence, or in 2 or 4)
-  const int chunks[3] = {64, 256, 1024};
-  const uint64_t tot = c->batch_total;
-  const int64_t batches[3] = {(int64_t)tot, (int64_t)((tot + 1) / 2), (int64_t)((tot + 3) / 4)};
-  const int64_t batch0 = c->batch;
-  const int chunk0 = c->chunk;
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) {
-      c->chunk = chunks[a];
-      c->batch = std::max<int64_t>(1, batches[b]);
-      double t[3];
-      if ((st = time_point(t))) return st;
-      if (t[0] < bst[0]) {
-        std::copy(t, t + 3, bst);
-        bc = chunks[a];
-        bb = c->batch;
-      }
-    }
-  if (bst[0] >= c->tune.default_median_ms) {  // nothing beat the starting point
-    bc = chunk0;
-    bb = batch0;
-  }
-  c->chunk = bc;
-  c->batch = bb;
-  c->tune.median_ms = bst[0];
-  c->tune.min_ms = bst[1];
-  c->tune.max_ms = bst[2];
+  int st = gg::tune_search(before, block, c->batch_total, time_point, found);
+  use(st ? before : found.best);
   drop_graph(c);
+  if (st) return st;
+  c->tune.points = found.points;
+  c->tune.repeats = kRep;
+  c->tune.default_median_ms = found.start_ms;
+  c->tune.median_ms = found.best_ms[0];
+  c->tune.min_ms = found.best_ms[1];
+  c->tune.max_ms = found.best_ms[2];
   if ((st = gg_reset_tally(c))) return st;
   if (best) {
     best->device = c->device;
