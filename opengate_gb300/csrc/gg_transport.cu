@@ -574,14 +574,6 @@ size_t slot_scratch_bytes() {
   return 6 * sizeof(real);
 }
 
-// Histories a gang claims at a time: an even share of a small run, else the
-// per-warp chunk of the options for each of its warps.
-int pool_chunk(const PoolPlan &p, int chunk, uint64_t n_hist) {
-  const uint64_t gangs = (uint64_t)p.grid * p.gangs, share = (n_hist + gangs - 1) / gangs;
-  const uint64_t warps = (uint64_t)std::max(p.block / 32 / p.gangs, 1);
-  return (int)std::max<uint64_t>(32, std::min<uint64_t>(share, warps * std::min(chunk, 1 << 20)));
-}
-
 template size_t record_bytes<float>(size_t);
 template size_t record_bytes<double>(size_t);
 template cudaError_t launch_generate<float>(const Scene<float> &, const KernelArgs &, cudaStream_t);

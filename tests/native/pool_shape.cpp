@@ -32,6 +32,14 @@ static int check(size_t slot, int queues) {
           REQUIRE(p.smem + gg::pool_static<real>(queues) <= kOptin);
           REQUIRE(p.smem == slot * p.slots * p.gangs + table);
           REQUIRE(p.scratch == (size_t)24 * p.slots * p.gangs * n_sm);
+          // claims: an even share of a small run, so no gang is left out; the option's otherwise
+          const uint64_t gangs = (uint64_t)p.grid * p.gangs;
+          for (int chunk : {1, 64, 4096, INT_MAX}) {
+            const uint64_t got = (uint64_t)gg::pool_chunk(p, chunk, n);
+            const uint64_t warps = (uint64_t)std::max(p.block / 32 / p.gangs, 1);
+            REQUIRE(got >= 1 && got <= (n + gangs - 1) / gangs);
+            REQUIRE(got == (n + gangs - 1) / gangs || got >= std::max<uint64_t>(32, warps * std::min(chunk, 1 << 20)));
+          }
           // one block of 256 threads per SM is taken as two, more than four as four
           const int same = blocks > 4 ? 4 : (blocks == 1 ? 2 : (blocks < 0 ? 0 : blocks));
           REQUIRE(gg::pool_shape<real>(n_sm, kOptin, table, same, n, slot, 24, queues, &q));
