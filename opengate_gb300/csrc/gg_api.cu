@@ -764,18 +764,28 @@ static int tally_alloc(gg_ctx *c) {
 }
 
 // A projection tally of n pixels as FP64 into the caller's buffer, through a
-// device buffer that the context keeps.
+// device buffer that the context keeps: 128 MB at most, so that a fetch asks
+// little of a device whose memory is taken.
+constexpr size_t kFetchPixels = (size_t)1 << 24;
+
 static int fetch_projection(gg_ctx *c, int kind, const unsigned long long *src, double *out, size_t n) {
   int st;
-  if (n > c->fetch_cap) {
+  const size_t cap = std::min(n, kFetchPixels);
+  if (cap > c->fetch_cap) {
     dfree(c->d_fetch);
     c->fetch_cap = 0;
-    if ((st = c->cuda(cudaMalloc(&c->d_fetch, n * sizeof(double)), "cudaMalloc projection"))) return st;
-    c->fetch_cap = n;
+    if ((st = c->cuda(cudaMalloc(&c->d_fetch, cap * sizeof(double)), "cudaMalloc projection"))) return st;
+    c->fetch_cap = cap;
   }
-  if ((st = c->cuda(gg::launch_projection_f64(kind, src, c->d_fetch, n, c->n_sm, c->stream), "projection to FP64")))
-    return st;
-  return c->d2h(out, c->d_fetch, n * sizeof(double), "download projection");
+  const size_t words = kind == gg::kProjSquares ? 2 : 1;
+  for (size_t at = 0; at < n; at += cap) {
+    const size_t m = std::min(cap, n - at);
+    if ((st = c->cuda(gg::launch_projection_f64(kind, src + words * at, c->d_fetch, m, c->n_sm, c->stream),
+                      "projection to FP64")))
+      return st;
+    if ((st = c->d2h(out + at, c->d_fetch, m * sizeof(double), "download projection"))) return st;
+  }
+  return GG_OK;
 }
 
 extern "C" {
