@@ -252,8 +252,10 @@ static_assert(GG_MAX_SPLITTING * kSplitBatch < (1 << 20) && kLoopCap < (1 << 12)
 // 4.1 ms against one thread per copy from request to end; of that, constants per
 // request and full rounds 6.6, the approximate trial with the azimuth 4.3, the
 // generator in line 4.1.
+// Three resident blocks (80 registers) in FP32: with 84 registers only two fit, 6.17
+// -> 6.50 ms for the copies and walks of 1e7 decays' scatter pass at 140 keV.
 template <typename real>
-__global__ void __launch_bounds__(256) k_spect_split(Scene<real> s, KernelArgs args, StageArgs q) {
+__global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) k_spect_split(Scene<real> s, KernelArgs args, StageArgs q) {
   __shared__ BlockCounters bc;
   __shared__ SplitWarp warps[kBlock / 32];
   if (threadIdx.x == 0) bc = BlockCounters{0, 0, 0, 0, 0, 0, 0, 0};
