@@ -262,6 +262,12 @@ inline bool pool_shape(int n_sm, size_t optin, size_t table_bytes, int blocks, u
   p->scratch = (size_t)p->grid * gangs * p->slots * scratch_bytes;
   return true;
 }
+// Photon slots of a pooled run of n histories, at most: one for each, an SM's histories
+// rounded up to warps (a gang has 32 slots at least) or its gangs' shares to 8.
+template <typename real>
+constexpr size_t pool_slots_most(uint64_t n, int n_sm) {
+  return (size_t)n + (size_t)n_sm * (1 + std::max(31, 8 * PoolShape<real>::kGangs));
+}
 template <typename real>
 cudaError_t pool_plan(int device, size_t table_bytes, int blocks, uint64_t n_hist, size_t slot_bytes,
                       size_t scratch_bytes, int queues, PoolPlan *p);

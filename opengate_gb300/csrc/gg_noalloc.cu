@@ -40,9 +40,9 @@ namespace {
 
 constexpr size_t kScratchBytes = (size_t)GG_NOALLOC_SCRATCH_BYTES;
 constexpr int kMaxDevices = 64;
-// scratch of the transport's photon slots (24 bytes each): a slot for every
-// history of a batch on 152 SMs x 3 blocks, rounded up to 32 per block
-constexpr size_t kSlotBytes = (size_t)24 * 32 * 2500;
+// scratch of the transport's photon slots (24 bytes each): those of a batch on 352 SMs
+// (with more the grid is cut to what fits)
+constexpr size_t kSlotBytes = (size_t)24 * gg::pool_slots_most<float>(GG_NOALLOC_BATCH, 352);
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 

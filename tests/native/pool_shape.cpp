@@ -22,7 +22,7 @@ static int check(size_t slot, int queues) {
   for (int n_sm : {1, 132, 152})
     for (size_t table : {(size_t)4096, (size_t)57344, (size_t)110000, most_table / 16 * 16})
       for (int blocks : {0, 1, 2, 3, 4, 5, INT_MAX, -1})
-        for (uint64_t n : {1ull, 31ull, 4864ull, 4865ull, 20000ull, 97280ull, 150000ull, 1ull << 26, 0xffffffffull}) {
+        for (uint64_t n : {1ull, 31ull, 33ull, 1000ull, 4864ull, 4865ull, 20000ull, 65536ull, 97280ull, 150000ull, 1ull << 26, 0xffffffffull}) {
           gg::PoolPlan p{}, q{};
           REQUIRE(gg::pool_shape<real>(n_sm, kOptin, table, blocks, n, slot, 24, queues, &p));
           REQUIRE(p.grid == n_sm && p.block >= 32 && p.block <= Shape::kBlock && p.block % 32 == 0);
@@ -32,6 +32,7 @@ static int check(size_t slot, int queues) {
           REQUIRE(p.smem + gg::pool_static<real>(queues) <= kOptin);
           REQUIRE(p.smem == slot * p.slots * p.gangs + table);
           REQUIRE(p.scratch == (size_t)24 * p.slots * p.gangs * n_sm);
+          REQUIRE((size_t)p.slots * p.gangs * n_sm <= gg::pool_slots_most<real>(n, n_sm));
           // claims: an even share of a small run, so no gang is left out; the option's otherwise
           const uint64_t gangs = (uint64_t)p.grid * p.gangs;
           for (int chunk : {1, 64, 4096, INT_MAX}) {
