@@ -111,11 +111,8 @@ __global__ void __launch_bounds__(256, kArfBlocks<real>) k_arf_sample(Scene<real
       sec.stride = blockDim.x;
       sec.tid = threadIdx.x;
       sec.has = 0;
-      HistList<real> l{nullptr, nullptr, 0, 0};  // never scored here
-      Tally<real> t{nullptr, nullptr};
       Event<real> ev;
       ev.clear();
-      unsigned int n_dep = 0;
       for (;;) {  // flights to the next interaction, which the warp's photons then have together
         int mat;
         bool hit = false;
@@ -128,7 +125,7 @@ __global__ void __launch_bounds__(256, kArfBlocks<real>) k_arf_sample(Scene<real
           hit = head_flight(s, ph, g, mat) != 0;
         }
         if (!hit) break;
-        do_interaction<real, true>(s, ph, g, &bc, mat, 0u, ph.hreg == s.hreg_cr ? 2 : 3, l, t, sec, n_dep, ev);
+        head_interaction(s, ph, g, &bc, mat, ph.hreg == s.hreg_cr ? 2 : 3, sec, ev);
       }
       int label = 0;
       real ed = ev.esum[0];

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_spect_arf(Scene<real> s, ArfS
     n_net = 0;
     n_fb = 0;
   }
-  const bool ready = tc_net_prepare(sm, a.params, a.wbf + kTcBf);
+  const bool ready = tc_net_prepare(sm, a.params, a.wbf);
 
   const PQueue<real> in = PQueue<real>::carve(a.in_q, a.q_cap);
   const PQueue<real> out = PQueue<real>::carve(a.out_q, a.q_cap);

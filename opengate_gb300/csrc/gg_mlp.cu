@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     k_mlp_predict(MlpTrainArgs a, float *out, uint64_t n, unsigned int *status) {
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   TcNetSmem &sm = *reinterpret_cast<TcNetSmem *>(tc_smem_raw);
-  const bool ready = tc_net_prepare(sm, a.params, a.wbf + kTcBf);
+  const bool ready = tc_net_prepare(sm, a.params, a.wbf);
   const int g = threadIdx.x >> 7, r = threadIdx.x & 127;
   uint32_t phase = 0;
   const uint64_t n_tiles = (n + kTcRows - 1) / kTcRows;

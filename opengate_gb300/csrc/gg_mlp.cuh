@@ -43,20 +43,17 @@ __host__ __device__ constexpr int param_of_partial(int q) {
   return off + o * kHid + i;
 }
 
-// BF16 weight copies used by the tensor cores: W2, W3, W4 back to back,
-// row-major [out][in] (the training kernel's ldmatrix operands), then the same
-// three matrices again as 5th-generation tensor-core operands (K-major core
-// matrices, gg_tc.cuh) starting at element kTcBf, so that one bulk copy per
-// matrix stages them in shared memory
+// BF16 weight copies used by the tensor cores: W2, W3, W4 back to back as
+// 5th-generation tensor-core operands (K-major core matrices, gg_tc.cuh), so
+// that one bulk copy per matrix stages them in shared memory
 constexpr int kBfW2 = 0;
 constexpr int kBfW3 = kHid * kHid;
 constexpr int kBfW4 = 2 * kHid * kHid;
 constexpr int kNBf = 2 * kHid * kHid + kOutPad * kHid;
-constexpr int kTcBf = kNBf;
 // ... and transposed, W^T[in][out] (K = out; W4^T is 128 x 16), the B operands
 // of the backward pass dH = dZ W, starting at element kTcTBf
-constexpr int kTcTBf = 2 * kNBf;
-constexpr int kNBfAll = 3 * kNBf;
+constexpr int kTcTBf = kNBf;
+constexpr int kNBfAll = 2 * kNBf;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -70,17 +67,16 @@ __host__ __device__ constexpr int tc_elem(int n, int k) { return tc_elem_k(n, k,
 // Stores parameter p (a weight of W2, W3 or W4, value w) as BF16 in both copies.
 __device__ __forceinline__ void bf16_store_weight(__nv_bfloat16 *wbf, int p, float w) {
   const __nv_bfloat16 b = __float2bfloat16_rn(w);
-  int base, tc, q;
-  if (p >= kOffW2 && p < kOffB2) base = kBfW2, tc = kTcBf + kBfW2, q = p - kOffW2;
-  else if (p >= kOffW3 && p < kOffB3) base = kBfW3, tc = kTcBf + kBfW3, q = p - kOffW3;
-  else if (p >= kOffW4 && p < kOffB4) base = kBfW4, tc = kTcBf + kBfW4, q = p - kOffW4;
+  int base, q;
+  if (p >= kOffW2 && p < kOffB2) base = kBfW2, q = p - kOffW2;
+  else if (p >= kOffW3 && p < kOffB3) base = kBfW3, q = p - kOffW3;
+  else if (p >= kOffW4 && p < kOffB4) base = kBfW4, q = p - kOffW4;
   else return;
   const int o = q / kHid, i = q % kHid;
-  wbf[base + q] = b;
-  wbf[tc + tc_elem(o, i)] = b;
+  wbf[base + tc_elem(o, i)] = b;
   // transposed: W^T[i][o], K = out units (128, or 16 for W4)
   const int kk = base == kBfW4 ? kOutPad : kHid;
-  wbf[tc - kTcBf + kTcTBf + tc_elem_k(i, o, kk)] = b;
+  wbf[kTcTBf + base + tc_elem_k(i, o, kk)] = b;
 }
 
 }  // namespace gg

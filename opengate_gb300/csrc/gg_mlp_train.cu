@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(MlpTrainArgs a) {
   }
   __syncthreads();
   cudaGridDependencySynchronize();  // the previous step's parameters
-  const __nv_bfloat16 *wtc = a.wbf + kTcBf, *wtt = a.wbf + kTcTBf;
+  const __nv_bfloat16 *wtc = a.wbf, *wtt = a.wbf + kTcTBf;
   if (threadIdx.x == 0) {
     mbar_expect_tx(&sm.mbar_load, (uint32_t)(2 * kTcBytesHid + kTcBytesOut));
     bulk_load(sm.w2, wtc + kBfW2, (uint32_t)kTcBytesHid, &sm.mbar_load);

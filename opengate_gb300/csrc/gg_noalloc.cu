@@ -298,8 +298,6 @@ extern "C" int gg_dose_run_noalloc(int32_t device, void *stream, const gg_tables
     a.slot_scratch = b + L.slots;
     a.records = b + L.records;
     a.rec_cap = (size_t)GG_NOALLOC_BATCH;
-    a.refill_min = 8;
-    a.interact_min = 16;
     for (uint64_t h0 = first_history; h0 < first_history + n_histories && e == cudaSuccess;
          h0 += (uint64_t)GG_NOALLOC_BATCH) {
       a.h_begin = h0;

@@ -17,8 +17,7 @@ namespace gg {
 
 // One history's voxel list: entry k at vox[k * stride], acc[k * stride] in
 // shared memory (a column per thread of the block), so the list takes no
-// registers across the transport loop.  Kernels that never score pass null
-// arrays with n = 0.
+// registers across the transport loop.
 template <typename real>
 struct HistList {
   uint32_t *vox;
@@ -1214,25 +1213,18 @@ __device__ __forceinline__ void event_add(const Scene<real> &s, Event<real> &ev,
   }
 }
 
-template <typename real, bool SPECT>
-__device__ __forceinline__ int do_interaction(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc,
-                                              int pmat, uint32_t pv, int pscored, HistList<real> &l,
-                                              const Tally<real> &t, Secondary<real> &sec, unsigned int &n_dep,
-                                              Event<real> &ev, int *kind = nullptr) {
-  real ed = interact(s, ph, pmat, g, bc, sec, kind);
-  if (pscored == 1) {
-    if constexpr (!SPECT) {
-      deposit(l, t, bc, pv, ed, n_dep);
-    }
-    if (ph.alive && ph.in_image) ph.t_exit = exit_distance(ph.pos, ph.dir, s.bmin, s.bmax);
-  } else if (pscored == 0) {
+// An interaction in the world (pscored 0), a crystal (2: a hit of the event) or
+// another part of a head (3).
+template <typename real>
+__device__ __forceinline__ int head_interaction(const Scene<real> &s, Photon<real> &ph, Rng &g, BlockCounters *bc,
+                                                int pmat, int pscored, Secondary<real> &sec, Event<real> &ev) {
+  const real ed = interact(s, ph, pmat, g, bc, sec);
+  if (pscored == 0) {
     ph.can_enter = 1;
     ph.exclude = -1;
-  } else if constexpr (SPECT) {
-    if (pscored == 2 && ed > R<real>(0)) {
-      if (ph.head == 0) event_add<real, 0>(s, ev, ph, ed);
-      else event_add<real, 1>(s, ev, ph, ed);
-    }
+  } else if (pscored == 2 && ed > R<real>(0)) {
+    if (ph.head == 0) event_add<real, 0>(s, ev, ph, ed);
+    else event_add<real, 1>(s, ev, ph, ed);
   }
   return ph.alive ? kFly : kRefill;
 }

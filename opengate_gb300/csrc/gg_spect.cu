@@ -933,16 +933,13 @@ __global__ void __launch_bounds__(256, MINB) k_spect_head(Scene<real> sg, Kernel
   sec.stride = blockDim.x;
   sec.tid = threadIdx.x;
   sec.has = 0;
-  HistList<real> l{nullptr, nullptr, 0, 0};  // never scored here
-  Tally<real> t{nullptr, nullptr};
   Event<real> ev;
   ev.clear();
   Rng g;
   int state = kRefill;
   bool in_hist = false;
   int pmat = 0, pscored = 0;
-  uint32_t pv = 0;
-  unsigned int n_dep = 0, n_world = 0, n_head = 0, n_singles = 0;
+  unsigned int n_world = 0, n_head = 0, n_singles = 0;
 
   for (;;) {
     // phase chosen per block: all warps run the same code region at the same
@@ -986,7 +983,7 @@ __global__ void __launch_bounds__(256, MINB) k_spect_head(Scene<real> sg, Kernel
       }
     } else if (phase == kInteract) {
       if (state == kInteract) {
-        state = do_interaction<real, true>(s, ph, g, &bc, pmat, pv, pscored, l, t, sec, n_dep, ev);
+        state = head_interaction(s, ph, g, &bc, pmat, pscored, sec, ev);
         if (state == kRefill && sec.has) {
           pop_secondary(s, ph, sec);
           state = kFly;

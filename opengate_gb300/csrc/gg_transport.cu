@@ -335,9 +335,7 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           if ((f & 3u) == kRecInImage) {
             aim = true;
             dest = kQFly;
-          } else if ((f & 3u) == kRecWorld) {
-            dest = kQWorld;
-          } else {
+          } else {  // (the source stage takes the first flight of a photon in the world)
             pmat = s.world_mat;
             dest = kQInteract;
           }

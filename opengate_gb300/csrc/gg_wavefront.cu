@@ -195,7 +195,7 @@ __device__ __forceinline__ int wf_process(int code, int slot, uint64_t h, const 
     return nc;
   }
   if (code == kWCompton || code == kWOther) {
-    // ---- the pending interaction (do_interaction of the dose path) -----------
+    // ---- the pending interaction ------------------------------------------
     Photon<real> ph;
     load_photon(S, slot, ph);
     Rng g;
