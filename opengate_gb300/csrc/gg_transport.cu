@@ -332,13 +332,11 @@ __global__ void __launch_bounds__(PoolShape<real>::kBlock, 1) k_transport_pool(S
           ph.steps = (int)((f >> 2) & 1u);
           ph.can_enter = 1;
           ph.t_exit = R<real>(0);
-          if ((f & 3u) == kRecInImage) {
-            aim = true;
-            dest = kQFly;
-          } else {  // (the source stage takes the first flight of a photon in the world)
-            pmat = s.world_mat;
-            dest = kQInteract;
-          }
+          // in the image, or at the collision in the world that ended the source stage's flight
+          // (without a branch: 24 batched simulations 12.5 -> 12.2 ms, CT 30.4 -> 30.1)
+          aim = (f & 3u) == kRecInImage;
+          dest = aim ? kQFly : kQInteract;
+          pmat = s.world_mat;
         }
       } else {
         slot_load(S, e, ph, cw, idx);
