@@ -44,6 +44,15 @@ void prefault(void *out, size_t bytes) noexcept {
     const uintptr_t lo = ((uintptr_t)out + page - 1) / page * page, hi = ((uintptr_t)out + bytes) / page * page;
     if (hi <= lo) return;
     const size_t n = (hi - lo) / page;
+    // (a kept buffer, page-locked or used before: three pages instead of the whole table, 16 us
+    // for 84 MB)
+    bool there = true;
+    for (size_t i : {(size_t)0, n / 2, n - 1}) {
+      unsigned char p = 0;
+      if (mincore((void *)(lo + i * page), page, &p) != 0) return;
+      there = there && (p & 1u);
+    }
+    if (there) return;
     std::vector<unsigned char> present(n);
     if (mincore((void *)lo, hi - lo, present.data()) != 0) return;
     size_t missing = 0;
