@@ -197,9 +197,9 @@ __device__ __forceinline__ Tally<real> tally_at(const KernelArgs &a, size_t off,
 // The order of operations inside each history, hence its result, does not
 // depend on which lane or round executes them.
 // Bound by instruction issue and by the gangs' barrier: 256 x 256 x 160 CT, 1e8
-// histories to 6 MeV, 47.9 -> 30.8 ms against one photon per thread with block-wide phases
-// (203 warp instructions per history at 21.5 active lanes; 379 at 8.6); 24
-// batched simulations 22.8 -> 14.3 ms, FP64 9.2 -> 4.1 ms per 1e6.
+// histories to 6 MeV, 47.1 -> 29.9 ms against one photon per thread with block-wide phases
+// (204 warp instructions per history at 21 active lanes; 379 at 8.6); 24
+// batched simulations 21.0 -> 12.2 ms, FP64 8.9 -> 4.1 ms per 1e6.
 // MULTI: batched simulations; DG: dose tally on a grid of its own (1: edep,
 // 2: edep and dose), Scene::dgrid; TLE: track-length estimator
 // (GateTLEDoseActor::ScoreTLEDepositStep,
